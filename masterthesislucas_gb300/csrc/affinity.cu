@@ -103,132 +103,247 @@ __device__ inline double aff_log(double x)
 }
 
 // ------------------------------------------------------------------ kNN
-// A block takes kQ query rows and walks every candidate tile of kQ points:
-// each thread accumulates a 4 x 4 block of squared distances over the
-// dimensions in order (one fmaf per dimension, as the definition), the tile's
-// distances go to shared memory, and each warp folds its rows' candidates into
-// their sorted top-k lists (kept in shared memory, ordered by (d, j)).
-constexpr int kQ = 64;        // query rows and candidates per tile
-constexpr int kDC = 32;       // dimensions per staged chunk
+// Every pair costs two FP32 operations a dimension (a difference and a fused
+// multiply-add, in the definition's order), so the FP32 pipe bounds the kernel
+// (15.6 ms at 20,000 x 784) and the rest is kept off it:
+// * A thread accumulates a 4 x 8 block of distances, two candidates to a
+//   packed FP32x2 operand: 32 packed instructions a dimension against 3
+//   16-byte shared loads.
+// * kKC dimensions of the tile's rows are staged transposed in shared memory,
+//   the next kKC fetched into registers meanwhile.
+// * The (query block, candidate tile) units are dealt to the blocks in equal
+//   contiguous runs: a block may start and end inside a query block's row of
+//   tiles, and then leaves a partial neighbour list.  k_knn_merge joins the
+//   partial lists of every query row.  One block per 64 queries instead left
+//   a third of the SMs idle in the second wave.
+// A list entry is the 64-bit key (distance bits, index): distances are never
+// negative, so integer order is (distance, index) order, and NaNs sort last.
+// 20,000 x 784, k = 90: 70.0 ms before (4 x 4 blocks of scalar operations, a
+// block per 64 queries), 22.8 ms now.  8 x 8 blocks need fewer shared loads
+// but leave 8 or 12 warps an SM instead of 16: 23.9 and 25.4 ms.
+constexpr int kQ = 64;        // query rows per block
+constexpr int kC = 128;       // candidates per tile
+constexpr int kKC = 16;       // dimensions per staged chunk
 constexpr int kKnnT = 256;    // threads
 constexpr int kMaxK = 128;    // longest neighbour list
+constexpr int kTilePad = 4;   // floats between the rows of a distance tile
+constexpr int kStageFloats = 2 * kKC * (kQ + kC);
+constexpr int kTileFloats = kQ * (kC + kTilePad);
+// the distance tile takes the staging buffers' place once its last chunk is used
+constexpr size_t kKnnStatic = 4 * (size_t)(kStageFloats > kTileFloats ? kStageFloats : kTileFloats);
+typedef unsigned long long u64;
 
-__device__ __forceinline__ bool before(float da, int ja, float db, int jb)
+// packed FP32 operations that keep subnormals, as fmaf does
+__device__ __forceinline__ u64 x2_sub(u64 a, u64 b)
 {
-    return da < db || (da == db && ja < jb);
+    u64 d;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ u64 x2_fma(u64 a, u64 b, u64 c)
+{
+    u64 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ u64 x2_pack(float a, float b)
+{
+    u64 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ void x2_unpack(u64 v, float& a, float& b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
 }
 
-__global__ void __launch_bounds__(kKnnT) k_knn(const float* __restrict__ x, int64_t n, int dim, int k,
-                                               float* __restrict__ out_d, int32_t* __restrict__ out_i)
+// unit u of `units` belongs to run owner(u): run b holds [b units / runs, (b + 1) units / runs)
+__host__ __device__ inline int64_t knn_owner(int64_t u, int64_t units, int64_t runs)
 {
-    __shared__ float sq[kDC][kQ + 1];
-    __shared__ float sc[kDC][kQ + 1];
-    __shared__ float tile[kQ][kQ + 1];
-    extern __shared__ uint8_t dyn[];
-    float* ld = reinterpret_cast<float*>(dyn);                   // [kQ][k] distances
-    int32_t* li = reinterpret_cast<int32_t*>(ld + kQ * k);      // [kQ][k] indices
-    __shared__ int lcount[kQ];
+    return ((u + 1) * runs - 1) / units;
+}
+
+// one key into a row's sorted list (k keys, unused ones all-ones), by a warp
+__device__ __forceinline__ void knn_insert(u64* __restrict__ list, int k, u64 key, int lane)
+{
+    u64 own[kMaxK / 32], prev[kMaxK / 32];
+    int pos = 0;
+#pragma unroll
+    for (int u = 0; u < kMaxK / 32; u++) {
+        const int e = lane + 32 * u;
+        own[u] = e < k ? list[e] : ~0ull;
+        prev[u] = e > 0 && e < k ? list[e - 1] : 0ull;
+        pos += __popc(__ballot_sync(0xffffffffu, own[u] < key));
+    }
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < kMaxK / 32; u++) {
+        const int e = lane + 32 * u;
+        if (e < k && e >= pos) list[e] = e == pos ? key : prev[u];
+    }
+    __syncwarp();
+}
+
+template <bool kVec>
+__global__ void __launch_bounds__(kKnnT, 2)
+    k_knn(const float* __restrict__ x, int64_t n, int dim, int k, int64_t ctiles, int64_t units, u64* __restrict__ part)
+{
+    extern __shared__ __align__(16) uint8_t dyn[];
+    float* stage = reinterpret_cast<float*>(dyn);          // [2][kKC][kQ + kC]
+    float* tile = stage;                                   // [kQ][kC + kTilePad]
+    u64* lists = reinterpret_cast<u64*>(dyn + kKnnStatic); // [kQ][k]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int64_t q0 = (int64_t)blockIdx.x * kQ;
-    const int tr = (tid / 16) * 4, tc = (tid % 16) * 4;  // this thread's 4 x 4 block
-    if (tid < kQ) lcount[tid] = 0;
-    for (int64_t c0 = 0; c0 < n; c0 += kQ) {
-        float acc[4][4];
+    const int ty = tid >> 4, tx = tid & 15;  // queries 4 ty + a; candidates 4 tx + b and 64 + 4 tx + b
+    constexpr int kRows = kQ + kC;
+    constexpr int kLoads = kRows * (kKC / 4) / kKnnT;  // 16-byte pieces a thread fetches per chunk
+    const int64_t runs = gridDim.x, run = blockIdx.x;
+    const int64_t u0 = run * units / runs, u1 = (run + 1) * units / runs;
+    const int chunks = (dim + kKC - 1) / kKC;
+    float4 pre[kLoads];
+    // piece i of a chunk: row (i mod kRows) of the tile, dimensions 4 (i / kRows) on; a warp's pieces are 32
+    // different rows, so their transposed stores hit 32 banks
+    auto fetch = [&](int64_t q0, int64_t c0, int t0) {
+#pragma unroll
+        for (int j = 0; j < kLoads; j++) {
+            const int i = tid + j * kKnnT, r = i % kRows, t = t0 + 4 * (i / kRows);
+            const int64_t row = r < kQ ? q0 + r : c0 + (r - kQ);
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);  // rows and dimensions past the end add (0 - 0)^2
+            if (row < n) {
+                const float* src = x + row * dim + t;
+                if (kVec) {
+                    if (t < dim) v = *reinterpret_cast<const float4*>(src);
+                } else {
+                    if (t < dim) v.x = src[0];
+                    if (t + 1 < dim) v.y = src[1];
+                    if (t + 2 < dim) v.z = src[2];
+                    if (t + 3 < dim) v.w = src[3];
+                }
+            }
+            pre[j] = v;
+        }
+    };
+    auto store = [&](float* s) {
+#pragma unroll
+        for (int j = 0; j < kLoads; j++) {
+            const int i = tid + j * kKnnT, r = i % kRows, t = 4 * (i / kRows);
+            s[t * kRows + r] = pre[j].x;
+            s[(t + 1) * kRows + r] = pre[j].y;
+            s[(t + 2) * kRows + r] = pre[j].z;
+            s[(t + 3) * kRows + r] = pre[j].w;
+        }
+    };
+    if (u0 < u1) fetch(u0 / ctiles * kQ, u0 % ctiles * kC, 0);
+    for (int64_t u = u0; u < u1; u++) {
+        const int64_t qb = u / ctiles, q0 = qb * kQ, c0 = u % ctiles * kC;
+        if (u == u0 || u % ctiles == 0)
+            for (int e = tid; e < kQ * k; e += kKnnT) lists[e] = ~0ull;
+        u64 acc[4][4];
 #pragma unroll
         for (int a = 0; a < 4; a++)
 #pragma unroll
-            for (int b = 0; b < 4; b++) acc[a][b] = 0.f;
-        for (int t0 = 0; t0 < dim; t0 += kDC) {
+            for (int b = 0; b < 4; b++) acc[a][b] = 0ull;
+        for (int c = 0; c < chunks; c++) {
+            float* s = stage + (c & 1) * kKC * kRows;
+            store(s);
             __syncthreads();
-            for (int e = tid; e < kQ * kDC; e += kKnnT) {
-                const int r = e / kDC, t = e % kDC;
-                const int64_t qi = q0 + r, ci = c0 + r;
-                sq[t][r] = (qi < n && t0 + t < dim) ? x[qi * dim + t0 + t] : 0.f;
-                sc[t][r] = (ci < n && t0 + t < dim) ? x[ci * dim + t0 + t] : 0.f;
-            }
-            __syncthreads();
-            const int tn = dim - t0 < kDC ? dim - t0 : kDC;
-            for (int t = 0; t < tn; t++) {
-                float qv[4], cv[4];
+            if (c + 1 < chunks)
+                fetch(q0, c0, (c + 1) * kKC);
+            else if (u + 1 < u1)
+                fetch((u + 1) / ctiles * kQ, (u + 1) % ctiles * kC, 0);
 #pragma unroll
-                for (int a = 0; a < 4; a++) qv[a] = sq[t][tr + a];
-#pragma unroll
-                for (int b = 0; b < 4; b++) cv[b] = sc[t][tc + b];
+            for (int t = 0; t < kKC; t++) {
+                const float4 q = *reinterpret_cast<const float4*>(s + t * kRows + 4 * ty);
+                const ulonglong2 ca = *reinterpret_cast<const ulonglong2*>(s + t * kRows + kQ + 4 * tx);
+                const ulonglong2 cb = *reinterpret_cast<const ulonglong2*>(s + t * kRows + kQ + 64 + 4 * tx);
+                const u64 q2[4] = {x2_pack(q.x, q.x), x2_pack(q.y, q.y), x2_pack(q.z, q.z), x2_pack(q.w, q.w)};
+                const u64 c2[4] = {ca.x, ca.y, cb.x, cb.y};
 #pragma unroll
                 for (int a = 0; a < 4; a++)
 #pragma unroll
                     for (int b = 0; b < 4; b++) {
-                        const float df = qv[a] - cv[b];
-                        acc[a][b] = fmaf(df, df, acc[a][b]);
+                        const u64 df = x2_sub(q2[a], c2[b]);
+                        acc[a][b] = x2_fma(df, df, acc[a][b]);
                     }
             }
         }
+        __syncthreads();  // the last chunk is read: the tile may overwrite the staging buffers
 #pragma unroll
         for (int a = 0; a < 4; a++)
 #pragma unroll
-            for (int b = 0; b < 4; b++) tile[tr + a][tc + b] = acc[a][b];
+            for (int b = 0; b < 4; b += 2) {
+                float4 v;
+                x2_unpack(acc[a][b], v.x, v.y);
+                x2_unpack(acc[a][b + 1], v.z, v.w);
+                *reinterpret_cast<float4*>(tile + (4 * ty + a) * (kC + kTilePad) + 32 * b + 4 * tx) = v;
+            }
         __syncthreads();
         // fold the tile into the lists: warp w owns rows w, w + 8, ...
         for (int r = warp; r < kQ; r += kKnnT / 32) {
             const int64_t qi = q0 + r;
             if (qi >= n) break;
-            float* rd = ld + r * k;
-            int32_t* ri = li + r * k;
+            u64* list = lists + r * k;
 #pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int cc = lane + 32 * h;
-                const int64_t cj = c0 + cc;
-                const float d = tile[r][cc];
-                int cnt = lcount[r];
-                bool want = cj < n && cj != qi && (cnt < k || before(d, (int)cj, rd[k - 1], ri[k - 1]));
-                uint32_t m = __ballot_sync(0xffffffffu, want);
+            for (int h = 0; h < kC / 32; h++) {
+                const int64_t cj = c0 + 32 * h + lane;
+                const u64 key = (u64)__float_as_uint(tile[r * (kC + kTilePad) + 32 * h + lane]) << 32 | (uint32_t)cj;
+                uint32_t m = __ballot_sync(0xffffffffu, cj < n && cj != qi && key < list[k - 1]);
                 while (m) {
                     const int src = __ffs(m) - 1;
                     m &= m - 1u;
-                    const float dv = __shfl_sync(0xffffffffu, d, src);
-                    const int jv = (int)(c0 + src + 32 * h);
-                    cnt = lcount[r];
-                    if (cnt == k && !before(dv, jv, rd[k - 1], ri[k - 1])) continue;
-                    // position: entries before (dv, jv)
-                    int pos = 0;
-                    for (int e = lane; e < cnt; e += 32) pos += before(rd[e], ri[e], dv, jv) ? 1 : 0;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) pos += __shfl_xor_sync(0xffffffffu, pos, o);
-                    const int last = cnt < k ? cnt : k - 1;  // shift [pos, last) up by one
-                    float sd[kMaxK / 32];
-                    int si[kMaxK / 32];
-#pragma unroll
-                    for (int u = 0; u < kMaxK / 32; u++) {
-                        const int e = lane + 32 * u;
-                        sd[u] = (e > pos && e <= last) ? rd[e - 1] : 0.f;
-                        si[u] = (e > pos && e <= last) ? ri[e - 1] : 0;
-                    }
-                    __syncwarp();
-#pragma unroll
-                    for (int u = 0; u < kMaxK / 32; u++) {
-                        const int e = lane + 32 * u;
-                        if (e > pos && e <= last) {
-                            rd[e] = sd[u];
-                            ri[e] = si[u];
-                        }
-                    }
-                    if (lane == 0) {
-                        rd[pos] = dv;
-                        ri[pos] = jv;
-                        if (cnt < k) lcount[r] = cnt + 1;
-                    }
-                    __syncwarp();
+                    const u64 kv = __shfl_sync(0xffffffffu, key, src);
+                    if (kv < list[k - 1]) knn_insert(list, k, kv, lane);
                 }
             }
         }
         __syncthreads();
+        if (u + 1 == u1 || (u + 1) % ctiles == 0) {
+            // runs and query blocks both grow along the units: run + query block numbers the partial lists
+            u64* dst = part + (run + qb) * (int64_t)(kQ * k);
+            for (int e = tid; e < kQ * k; e += kKnnT) dst[e] = lists[e];
+            __syncthreads();
+        }
     }
-    for (int e = tid; e < kQ * k; e += kKnnT) {
-        const int r = e / k, c = e % k;
-        const int64_t qi = q0 + r;
-        if (qi < n) {
-            out_d[qi * k + c] = ld[e];
-            out_i[qi * k + c] = li[e];
+}
+
+// A warp per query row joins the row's partial lists (of the runs that hold
+// its query block's units): an entry's place is its own index plus, for every
+// other list, the number of that list's smaller entries.
+constexpr int kMergeWarps = 4;
+__global__ void __launch_bounds__(32 * kMergeWarps)
+    k_knn_merge(const u64* __restrict__ part, int64_t n, int k, int64_t ctiles, int64_t units, int64_t runs,
+                int maxseg, float* __restrict__ out_d, int32_t* __restrict__ out_i)
+{
+    extern __shared__ __align__(16) uint8_t dyn[];
+    const int lane = threadIdx.x & 31;
+    u64* sl = reinterpret_cast<u64*>(dyn) + (size_t)(threadIdx.x >> 5) * maxseg * k;
+    const int64_t row = blockIdx.x * (int64_t)kMergeWarps + (threadIdx.x >> 5);
+    if (row >= n) return;
+    const int64_t qb = row / kQ;
+    const int64_t b0 = knn_owner(qb * ctiles, units, runs), b1 = knn_owner((qb + 1) * ctiles - 1, units, runs);
+    const int nseg = (int)(b1 - b0 + 1) < maxseg ? (int)(b1 - b0 + 1) : maxseg;
+    for (int sg = 0; sg < nseg; sg++) {
+        const u64* src = part + (b0 + sg + qb) * (int64_t)(kQ * k) + (row % kQ) * k;
+        for (int e = lane; e < k; e += 32) sl[sg * k + e] = src[e];
+    }
+    __syncwarp();
+    for (int e = lane; e < nseg * k; e += 32) {
+        const u64 key = sl[e];
+        if (key == ~0ull) continue;
+        const int sg = e / k;
+        int place = e - sg * k;
+        for (int o = 0; o < nseg && place < k; o++) {
+            if (o == sg) continue;
+            int lo = 0, hi = k;  // the first entry of list o not below key
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (sl[o * k + mid] < key) lo = mid + 1;
+                else hi = mid;
+            }
+            place += lo;
+        }
+        if (place < k) {
+            out_d[row * k + place] = __uint_as_float((uint32_t)(key >> 32));
+            out_i[row * k + place] = (int32_t)(uint32_t)key;
         }
     }
 }
@@ -340,10 +455,26 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
         tc_set_error("tc_knn_device: invalid arguments (need 1 <= k <= %d, k < n)", kMaxK);
         return TC_ERR_INVALID;
     }
-    const size_t dyn = (size_t)kQ * k * 8;
-    TC_CUDA_TRY(cudaFuncSetAttribute(k_knn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    k_knn<<<(unsigned)((n + kQ - 1) / kQ), kKnnT, dyn, (cudaStream_t)stream>>>(d_x, n, dim, k, d_dist, d_idx);
-    TC_CUDA_TRY(cudaGetLastError());
+    cudaStream_t s = (cudaStream_t)stream;
+    const int64_t qblocks = (n + kQ - 1) / kQ, ctiles = (n + kC - 1) / kC, units = qblocks * ctiles;
+    // two resident blocks per SM (registers and shared memory), each one run of units
+    const int64_t runs = units < 2 * (int64_t)sm_count() ? units : 2 * (int64_t)sm_count();
+    // runs that share a query block: each holds at least units / runs of its ctiles units
+    const int64_t maxseg = runs / qblocks + 2 < ctiles ? runs / qblocks + 2 : ctiles;
+    const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
+    // 16-byte loads: every row starts on a 16-byte boundary
+    const bool vec = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0;
+    auto kernel = vec ? k_knn<true> : k_knn<false>;
+    TC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+    TC_CUDA_TRY(cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mdyn));
+    void* part = nullptr;
+    TC_CUDA_TRY(cudaMallocAsync(&part, (size_t)(runs + qblocks) * kQ * k * 8, s));
+    kernel<<<(unsigned)runs, kKnnT, dyn, s>>>(d_x, n, dim, k, ctiles, units, static_cast<u64*>(part));
+    k_knn_merge<<<(unsigned)((n + kMergeWarps - 1) / kMergeWarps), 32 * kMergeWarps, mdyn, s>>>(
+        static_cast<const u64*>(part), n, k, ctiles, units, runs, (int)maxseg, d_dist, d_idx);
+    const cudaError_t e = cudaGetLastError(), ef = cudaFreeAsync(part, s);
+    if (e != cudaSuccess) return tc_cuda_fail(e, "tc_knn_device");
+    TC_CUDA_TRY(ef);
     return TC_OK;
 }
 
