@@ -22,6 +22,15 @@ namespace tc {
 int sm_count();
 // leaves above this many particles take a warp (leaf moments, P2M) in the order-p path
 constexpr uint32_t kLeafSmall = 32;
+// P2M: leaves above this many particles take a block each, between the two a
+// warp each.  A warp alone on a leaf of 6,600 particles (200,001 particles of
+// two disks, 4,096 leaves) took 104 us at order 8, a block of four 35 us.
+constexpr uint32_t kLeafBlock = 512;
+// the two lists of large leaves: [0] the number above kLeafSmall, [1] above
+// kLeafBlock, then the first kind's leaves from kBigLeaves on, the second
+// kind's (which the first includes) huge_leaves(n) words on
+constexpr int kBigLeaves = 2;
+__host__ __device__ inline int64_t huge_leaves(int64_t n) { return kBigLeaves + n / (kLeafSmall + 1) + 1; }
 
 __host__ __device__ inline uint32_t spread16(uint32_t x)
 {

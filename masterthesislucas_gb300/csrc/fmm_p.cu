@@ -29,7 +29,8 @@ namespace {
 // ------------------------------------------------------------------ P2M
 // mu_a = sum (r/h)^a / a! about the COM.  Leaves of up to kLeafSmall
 // particles take one thread each (monomials built degree by degree, two rows
-// live); the larger leaves, listed by the leaf build, one warp each.
+// live); the larger leaves, listed by the leaf build, a warp or (above
+// kLeafBlock) a block each.
 
 template <int P>
 __global__ void __launch_bounds__(128) k_p2m_small(int dep, float h, const uint32_t* __restrict__ count,
@@ -79,33 +80,56 @@ template <int P>
 __global__ void __launch_bounds__(128) k_p2m(int dep, float h, const uint32_t* __restrict__ count,
                                              const uint32_t* __restrict__ first, const float* __restrict__ comrel,
                                              const float* __restrict__ prel, const uint32_t* __restrict__ big,
-                                             float* __restrict__ mu)
+                                             int64_t huge, float* __restrict__ mu)
 {
-    constexpr int K = ncoef(P);
-    const int lane = threadIdx.x & 31;
+    constexpr int K = ncoef(P), W = 4;  // warps of a block
+    __shared__ float part[W][K];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t li = level_index(dep);
-    const int64_t nbig = big[0];
+    const uint32_t nbig = big[0];
     const float ih = 1.0f / h;
-    const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < nbig; w += wstride) {
-        const int64_t node = li + big[1 + w];
-        const uint32_t c = count[node];
+    // particles [f + q0, f + c) in steps of `step`, this lane's share
+    auto sum = [&](int64_t node, uint32_t c, uint32_t q0, uint32_t step, float (&acc)[K]) {
         const uint32_t f = first[node];
         const float cx = comrel[2 * node], cy = comrel[2 * node + 1];
-        float acc[K];
 #pragma unroll
         for (int k = 0; k < K; k++) acc[k] = 0.f;
-        for (uint32_t q = lane; q < c; q += 32) {
+        for (uint32_t q = q0; q < c; q += step) {
             float w[K];
             monomials<P>((prel[2 * (f + q)] - cx) * ih, (prel[2 * (f + q) + 1] - cy) * ih, w);
 #pragma unroll
             for (int k = 0; k < K; k++) acc[k] += w[k];
         }
+    };
+    float acc[K];
+    for (uint32_t b = blockIdx.x * W + wid; b < nbig; b += gridDim.x * W) {
+        const int64_t node = li + big[kBigLeaves + b];
+        const uint32_t c = count[node];
+        if (c > kLeafBlock) continue;
+        sum(node, c, lane, 32, acc);
 #pragma unroll
         for (int k = 0; k < K; k++) {
             const float v = warp_sum(acc[k]);
             if (lane == 0) mu[node * kstride(P) + k] = v;
         }
+    }
+    const uint32_t nhuge = big[1];
+    for (uint32_t b = blockIdx.x; b < nhuge; b += gridDim.x) {
+        const int64_t node = li + big[huge + b];
+        sum(node, count[node], threadIdx.x, 32 * W, acc);
+#pragma unroll
+        for (int k = 0; k < K; k++) {
+            const float v = warp_sum(acc[k]);
+            if (lane == 0) part[wid][k] = v;
+        }
+        __syncthreads();
+        for (int k = threadIdx.x; k < K; k += 32 * W) {
+            float v = part[0][k];
+#pragma unroll
+            for (int i = 1; i < W; i++) v += part[i][k];
+            mu[node * kstride(P) + k] = v;
+        }
+        __syncthreads();
     }
 }
 
@@ -746,9 +770,19 @@ constexpr int kNearWarps = 4;
 // sinks per block item: leaves of more than 32 particles are split into
 // items of this many sinks, a block (a warp per 32 sinks) each
 constexpr uint32_t kBlockSinks = 32u * kNearWarps;
+// A leaf of more than kSplitLeaf particles lies in a dense region, where its
+// near list is tens of thousands of particles long: items of 128 sinks are
+// then fewer than the resident blocks and up to three times their mean, and
+// the last of them run alone on their SMs.  Its items hold 32 sinks and the
+// block's warps split the sources instead (near_split_item).  200,001
+// particles of two disks in 4,096 leaves (largest 6,600, 3.2e9 pairs):
+// 1,630 us with items of 128 sinks, 1,273 us now.  Leaves below the line
+// keep the wider items, which stage every source once for 128 sinks.
+constexpr uint32_t kSplitLeaf = 512u;
+__device__ __forceinline__ uint32_t block_item_sinks(uint32_t c) { return c > kSplitLeaf ? 32u : kBlockSinks; }
 
 // per leaf: warp items (a leaf of 1..32 particles) and block items (a larger
-// leaf, one per kBlockSinks of its particles)
+// leaf, one per block_item_sinks of its particles)
 __global__ void k_chunks(int dep, const uint32_t* __restrict__ count, uint32_t* __restrict__ nwarp,
                          uint32_t* __restrict__ nblock)
 {
@@ -757,7 +791,7 @@ __global__ void k_chunks(int dep, const uint32_t* __restrict__ count, uint32_t* 
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nl; i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t c = count[li + i];
         nwarp[i] = c >= 1u && c <= 32u ? 1u : 0u;
-        nblock[i] = c > 32u ? (c + kBlockSinks - 1u) / kBlockSinks : 0u;
+        nblock[i] = c > 32u ? (c + block_item_sinks(c) - 1u) / block_item_sinks(c) : 0u;
     }
 }
 
@@ -785,45 +819,17 @@ __global__ void k_chunk_leaf(int dep, const uint32_t* __restrict__ wptr, const u
 #define TC_NEAR_BUF 512
 #endif
 constexpr int kNearBuf = TC_NEAR_BUF;
-// Padding source: far enough that its force factor underflows to zero and its
-// pair term (~1e-18 gravity, ~1e-36 t-SNE) is absorbed by any real sum.
-constexpr float kFarAway = 1.0e18f;
 
-// One sink (px, py) against its share of the staged sources: g lanes share a
-// sink, lane r of the group takes 16-byte slots r, r + g, r + 2g, ... (two
-// sources each, stored (x0, x1, y0, y1) so that each pair of coordinates is
-// one packed FP32x2 operand; consecutive lanes read consecutive slots, so the
-// group's loads are conflict-free and the groups' identical loads
-// broadcast).  Both sources of a slot go through each instruction together
-// (fma/add/sub/mul.f32x2), halving the instructions per pair; the two
-// partial sums per accumulator are added at the end.  n4 is a multiple of 4g,
-// so every lane runs the same number of trips.
+// p2p_slots over n4 staged slots, added to the sink's sums
 template <typename KN>
 __device__ __forceinline__ void p2p_staged(const KN& ker, const float4* __restrict__ s4, uint32_t n4, uint32_t r,
                                            uint32_t g, float px, float py, float& gx, float& gy, float& zs)
 {
-    const unsigned long long px2 = f2_pack(px, px), py2 = f2_pack(py, py);
     unsigned long long ax = 0ull, ay = 0ull, az = 0ull;  // packed +0.0f, +0.0f
-    for (uint32_t j = r; j < n4; j += 4 * g) {
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const float4 t4 = s4[j + u * g];
-            const unsigned long long Rx = f2_sub(px2, f2_pack(t4.x, t4.y));
-            const unsigned long long Ry = f2_sub(py2, f2_pack(t4.z, t4.w));
-            unsigned long long a, tt;
-            ker.near_xy2(Rx, Ry, a, tt);
-            ax = f2_fma(a, Rx, ax);
-            ay = f2_fma(a, Ry, ay);
-            az = f2_add(az, tt);
-        }
-    }
-    float a0, a1;
-    f2_unpack(ax, a0, a1);
-    gx += KN::kSign * (a0 + a1);
-    f2_unpack(ay, a0, a1);
-    gy += KN::kSign * (a0 + a1);
-    f2_unpack(az, a0, a1);
-    zs += KN::kSign * (a0 + a1);
+    p2p_slots(ker, s4, n4, r, g, px, py, ax, ay, az);
+    gx += KN::kSign * f2_total(ax);
+    gy += KN::kSign * f2_total(ay);
+    zs += KN::kSign * f2_total(az);
 }
 
 // Direct P2P of a leaf S's sinks with every particle of near(S); each sink's
@@ -971,6 +977,142 @@ __device__ __forceinline__ float near_item(const KN& ker, int dep, float h, cons
     return warp_sum(act ? zs : 0.0f);
 }
 
+// An item of a leaf above kSplitLeaf: the block's warps hold the same m <= 32
+// sinks and take every kNearWarps-th run of kFill sources of the near list,
+// each staging its own run kNearBuf sources at a time.  After each round of
+// runs the runs' sums are added in list order, so a sink's force is the one
+// near_item computes from the same list (whose staging buffer holds kFill
+// sources), bit for bit.  Returns the item's pair sum (all warps the same).  A
+// call, so that its registers are not the other items' (inlined: 4M two-disk
+// particles, which never reach it, 0.6 % slower).
+template <typename KN>
+__device__ __noinline__ float near_split_item(const KN& ker, int dep, float h, const uint32_t* __restrict__ count,
+                                                 const uint32_t* __restrict__ first,
+                                                 const uint32_t* __restrict__ near_ptr,
+                                                 const uint32_t* __restrict__ near_idx,
+                                                 const float2* __restrict__ prel2, uint32_t n,
+                                                 float2* __restrict__ nearf, int64_t si, uint32_t c0, uint32_t m,
+                                                 float* src, uint32_t* pairs)
+{
+    constexpr uint32_t kFill = kNearWarps * kNearBuf;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float* buf = src + w * 2 * kNearBuf;
+    const float4* buf4 = reinterpret_cast<const float4*>(buf);
+    auto stage = [&](uint32_t q, float x, float y) {
+        buf[(q >> 1) * 4 + (q & 1)] = x;
+        buf[(q >> 1) * 4 + 2 + (q & 1)] = y;
+    };
+    const uint32_t li = level_index(dep);
+    const uint32_t fS = first[li + si];
+    const uint32_t lg = 5u - (32u - __clz(m - 1u));  // log2 g, g * m <= 32
+    const uint32_t g = 1u << lg, r = lane & (g - 1u), sk = lane >> lg;
+    const bool act = sk < m;
+    const uint32_t s = fS + c0 + (act ? sk : 0u);
+    const int isx = (int)compact16((uint32_t)si), isy = (int)compact16((uint32_t)si >> 1);
+    const float2 p2 = act ? prel2[s] : make_float2(0.f, 0.f);
+    const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
+    // the list's length in particles, and whether it holds the leaf itself
+    uint32_t total = 0;
+    bool has_self = false;
+    for (uint32_t e = e0 + lane; e < e1; e += 32) {
+        const uint32_t ti = near_idx[e];
+        total += count[li + ti];
+        has_self |= ti == (uint32_t)si;
+    }
+    total = __reduce_add_sync(0xffffffffu, total);
+    has_self = __any_sync(0xffffffffu, has_self);
+    // the current batch of 32 entries, one per lane, holding positions [pos0, pos0 + tot)
+    uint32_t eb = e0, nt = 0, mf = 0, ex = 0, pos0 = 0, tot = 0;
+    float mox = 0.f, moy = 0.f;
+    float gx = 0.f, gy = 0.f, zs = 0.f;
+    for (uint32_t f0 = 0; f0 < total; f0 += kNearWarps * kFill) {
+        const uint32_t lo = f0 + w * kFill, hi = min(lo + kFill, total);
+        unsigned long long ax = 0ull, ay = 0ull, az = 0ull;
+        uint32_t fill = 0;
+        for (uint32_t q0 = lo; q0 < hi;) {
+            while (q0 >= pos0 + tot && eb < e1) {  // the batch holding q0
+                pos0 += tot;
+                nt = min(32u, e1 - eb);
+                uint32_t mc = 0;
+                if (lane < nt) {
+                    const uint32_t ti = near_idx[eb + lane];
+                    mf = first[li + ti];
+                    mc = count[li + ti];
+                    mox = (float)((int)compact16(ti) - isx) * h;
+                    moy = (float)((int)compact16(ti >> 1) - isy) * h;
+                }
+                uint32_t inc = mc;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t v = __shfl_up_sync(0xffffffffu, inc, o);
+                    if (lane >= (uint32_t)o) inc += v;
+                }
+                ex = inc - mc;
+                tot = __shfl_sync(0xffffffffu, inc, 31);
+                eb += nt;
+            }
+            if (q0 >= pos0 + tot) break;  // q0 < total: only in a list whose length overflowed 32 bits
+            const uint32_t b0 = q0 - pos0;  // within the batch
+            const uint32_t take = min(min(tot - b0, (uint32_t)kNearBuf - fill), hi - q0);
+            for (uint32_t k = 0; k < take; k += 32) {
+                // the entry of position q, as in near_item: the entries starting at or before it, minus one
+                const uint32_t base = b0 + k, q = base + lane;
+                const uint32_t before = __popc(__ballot_sync(0xffffffffu, lane < nt && ex < base));
+                const uint32_t d = ex - base;
+                const uint32_t bits = __reduce_or_sync(0xffffffffu, (lane < nt && d < 32u) ? 1u << d : 0u);
+                const uint32_t t = before + __popc(bits & (0xffffffffu >> (31u - lane))) - 1u;
+                const uint32_t fT = __shfl_sync(0xffffffffu, mf, t), eT = __shfl_sync(0xffffffffu, ex, t);
+                const float ox = __shfl_sync(0xffffffffu, mox, t), oy = __shfl_sync(0xffffffffu, moy, t);
+                if (k + lane < take) {
+                    const uint32_t sp = fT + (q - eT);
+                    const float2 t2 = sp < n ? prel2[sp] : make_float2(kFarAway, kFarAway);
+                    stage(fill + k + lane, t2.x + ox, t2.y + oy);
+                }
+            }
+            fill += take;
+            q0 += take;
+            if (fill == kNearBuf || q0 == hi) {
+                const uint32_t n8 = (fill + 8u * g - 1u) / (8u * g) * (8u * g);
+                if (fill + lane < n8) stage(fill + lane, kFarAway, kFarAway);
+                for (uint32_t q = fill + 32u + lane; q < n8; q += 32u) stage(q, kFarAway, kFarAway);
+                __syncwarp();
+                if (act) p2p_slots(ker, buf4, n8 / 2, r, g, p2.x, p2.y, ax, ay, az);
+                __syncwarp();
+                fill = 0;
+            }
+        }
+        // (the warp's buffer is free between its runs)
+        buf[lane] = KN::kSign * f2_total(ax);
+        buf[32 + lane] = KN::kSign * f2_total(ay);
+        buf[64 + lane] = KN::kSign * f2_total(az);
+        __syncthreads();
+        for (uint32_t k = 0; k < kNearWarps && f0 + k * kFill < total; k++) {
+            const float* part = src + k * 2 * kNearBuf;
+            gx += part[lane];
+            gy += part[32 + lane];
+            zs += part[64 + lane];
+        }
+        __syncthreads();
+    }
+    for (uint32_t o = g >> 1; o > 0; o >>= 1) {
+        gx += __shfl_xor_sync(0xffffffffu, gx, o);
+        gy += __shfl_xor_sync(0xffffffffu, gy, o);
+    }
+    if (act && r == 0) {
+        if (w == 0) {
+            *pairs += total - (has_self ? 1u : 0u);
+            nearf[s] = make_float2(gx, gy);
+        }
+        if (has_self) {
+            // the sink's own pair term, as in near_item
+            float D1, t0;
+            ker.near_xy(0.0f, 0.0f, D1, t0);
+            zs -= t0;
+        }
+    }
+    return warp_sum(act ? zs : 0.0f);
+}
+
 // Block items first (each block takes whole items), then warp items (each
 // warp its own); per item one FP64 pair-sum word in zwork: warp items at
 // [0, nw), block items after them.
@@ -999,6 +1141,15 @@ __global__ void __launch_bounds__(32 * kNearWarps, TC_NEAR_MIN_WARPS / kNearWarp
     for (uint32_t bi = blockIdx.x; bi < nb; bi += gridDim.x) {
         const int64_t si = bitem[bi];
         const uint32_t cS = count[li + si];
+        if (cS > kSplitLeaf) {
+            const uint32_t c0 = (bi - bptr[si]) * 32u;
+            uint32_t pairs = 0;
+            const float z = near_split_item(ker, dep, h, count, first, near_ptr, near_idx, prel2, n, nearf, si, c0,
+                                            min(32u, cS - c0), s_src, &pairs);
+            n_pp += pairs;
+            if (threadIdx.x == 0 && nw + bi < cap) zwork[nw + bi] = (double)z;
+            continue;
+        }
         const uint32_t c0 = (bi - bptr[si]) * kBlockSinks + 32u * w;
         const uint32_t m = cS > c0 ? min(32u, cS - c0) : 0u;
         const float z = near_item<true>(ker, dep, h, count, first, near_ptr, near_idx, prel2, n, nearf, si, c0, m,
@@ -1232,7 +1383,8 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
     const uint32_t* witem = P<uint32_t>(h.chunk_leaf);
     const uint32_t* bitem = witem + wmax;
     {
-        const int64_t wblk = (wmax + kNearWarps - 1) / kNearWarps;
+        // a block per block item as far as the split leaves go (at most n / 32 items), four warp items a block
+        const int64_t wb = (wmax + kNearWarps - 1) / kNearWarps, wblk = wb > h.n / 32 ? wb : h.n / 32;
         const uint32_t* ptr_n = P<uint32_t>(h.ptr_pool);
         const uint32_t* idx_n = P<uint32_t>(h.idx_pool);
         k_near_p<KN><<<(unsigned)(wblk < sm_count() * 256 ? wblk : sm_count() * 256), 32 * kNearWarps, 0, sn>>>(
@@ -1414,7 +1566,8 @@ int multipoles_p(Handle& h)
     k_p2m_small<ORD><<<grid_for(nleaf, 128), 128, 0, s>>>(dep, hl(dep), count, P<uint32_t>(h.first), comrel,
                                                          P<float>(h.prel), mu, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
     k_p2m<ORD><<<grid_for((h.n / (kLeafSmall + 1) + 1) * 32, 128), 128, 0, s>>>(
-        dep, hl(dep), count, P<uint32_t>(h.first), comrel, P<float>(h.prel), P<uint32_t>(h.bigleaf), mu);
+        dep, hl(dep), count, P<uint32_t>(h.first), comrel, P<float>(h.prel), P<uint32_t>(h.bigleaf),
+        huge_leaves(h.n), mu);
     for (int l = dep - 1; l >= 0; l--) {
         const int64_t nl = (int64_t)1 << (2 * l);
         if (nl <= kM2mQuadLevelNodes)

@@ -153,5 +153,46 @@ struct KGrav {
     }
 };
 
+// Padding source: far enough that its force factor underflows to zero and its
+// pair term (~1e-18 gravity, ~1e-36 t-SNE) is absorbed by any real sum.
+constexpr float kFarAway = 1.0e18f;
+
+// One sink (px, py) against its share of the staged sources: g lanes share a
+// sink, lane r of the group takes 16-byte slots r, r + g, r + 2g, ... (two
+// sources each, stored (x0, x1, y0, y1) so that each pair of coordinates is
+// one packed FP32x2 operand; consecutive lanes read consecutive slots, so the
+// group's loads are conflict-free and the groups' identical loads
+// broadcast).  Both sources of a slot go through each instruction together
+// (fma/add/sub/mul.f32x2), halving the instructions per pair; the two
+// partial sums per accumulator are added at the end.  n4 is a multiple of 4g,
+// so every lane runs the same number of trips.
+template <typename KN>
+__device__ __forceinline__ void p2p_slots(const KN& ker, const float4* __restrict__ s4, uint32_t n4, uint32_t r,
+                                          uint32_t g, float px, float py, unsigned long long& ax,
+                                          unsigned long long& ay, unsigned long long& az)
+{
+    const unsigned long long px2 = f2_pack(px, px), py2 = f2_pack(py, py);
+    for (uint32_t j = r; j < n4; j += 4 * g) {
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const float4 t4 = s4[j + u * g];
+            const unsigned long long Rx = f2_sub(px2, f2_pack(t4.x, t4.y));
+            const unsigned long long Ry = f2_sub(py2, f2_pack(t4.z, t4.w));
+            unsigned long long a, tt;
+            ker.near_xy2(Rx, Ry, a, tt);
+            ax = f2_fma(a, Rx, ax);
+            ay = f2_fma(a, Ry, ay);
+            az = f2_add(az, tt);
+        }
+    }
+}
+
+// the two halves of a packed accumulator, added
+__device__ __forceinline__ float f2_total(unsigned long long v)
+{
+    float a0, a1;
+    f2_unpack(v, a0, a1);
+    return a0 + a1;
+}
 
 }  // namespace tc

@@ -66,7 +66,7 @@ __global__ void k_leaf_small_p(int depth, double minx, double miny, double h, ui
                                double2* __restrict__ com64, double* __restrict__ m0, double* __restrict__ m2,
                                double2* __restrict__ bbc, double* __restrict__ bblen, float* __restrict__ comrel,
                                float* __restrict__ m0r, float* __restrict__ m2t, uint32_t* __restrict__ big,
-                               float* __restrict__ bmax, int box)
+                               int64_t huge, float* __restrict__ bmax, int box)
 {
     const uint32_t li = level_index(depth);
     const int64_t nl = (int64_t)1 << (2 * depth);
@@ -78,7 +78,8 @@ __global__ void k_leaf_small_p(int depth, double minx, double miny, double h, ui
         const uint32_t c = e - f;
         count[node] = c;
         if (c > kLeafSmall) {
-            big[1 + atomicAdd(big, 1u)] = (uint32_t)i;
+            big[kBigLeaves + atomicAdd(big, 1u)] = (uint32_t)i;
+            if (c > kLeafBlock) big[huge + atomicAdd(big + 1, 1u)] = (uint32_t)i;
             continue;
         }
         float sx = 0.f, sy = 0.f;
@@ -117,7 +118,7 @@ __global__ void k_leaf_big_p(int depth, double minx, double miny, double h, cons
     const int64_t nbig = big[0];
     const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t w = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); w < nbig; w += wstride) {
-        const int64_t i = big[1 + w];
+        const int64_t i = big[kBigLeaves + w];
         const int64_t node = li + i;
         const uint32_t c = count[node], f = first[node];
         float sx = 0.f, sy = 0.f;
@@ -266,12 +267,13 @@ int build_records_p(Handle& h, double hleaf)
     const int64_t maxbig = h.n / (kLeafSmall + 1) + 1;
     const int box = h.centre == TC_CENTRE_BOX;
     int rc;
-    if ((rc = ensure(h.bigleaf, (maxbig + 1) * 4)) || (rc = ensure(h.bmax, h.nnodes * 4))) return rc;
-    TC_CUDA_TRY(cudaMemsetAsync(h.bigleaf.p, 0, 4, s));
+    const int64_t huge = huge_leaves(h.n);
+    if ((rc = ensure(h.bigleaf, (huge + h.n / (kLeafBlock + 1) + 1) * 4)) || (rc = ensure(h.bmax, h.nnodes * 4))) return rc;
+    TC_CUDA_TRY(cudaMemsetAsync(h.bigleaf.p, 0, 4 * kBigLeaves, s));
     k_leaf_small_p<<<grid_for(nleaf, 128), 128, 0, s>>>(
         depth, h.minx, h.miny, hleaf, P<uint32_t>(h.count), P<uint32_t>(h.first), P<float2>(h.prel),
         P<double2>(h.com64), P<double>(h.m0), P<double>(h.m2), P<double2>(h.bbc), P<double>(h.bblen),
-        P<float>(h.comrel), P<float>(h.m0r), P<float>(h.m2t), P<uint32_t>(h.bigleaf), P<float>(h.bmax), box);
+        P<float>(h.comrel), P<float>(h.m0r), P<float>(h.m2t), P<uint32_t>(h.bigleaf), huge, P<float>(h.bmax), box);
     k_leaf_big_p<<<grid_for(maxbig * 32, 128), 128, 0, s>>>(
         depth, h.minx, h.miny, hleaf, P<uint32_t>(h.count), P<uint32_t>(h.first), P<float2>(h.prel),
         P<double2>(h.com64), P<double>(h.m0), P<double>(h.m2), P<double2>(h.bbc), P<double>(h.bblen),

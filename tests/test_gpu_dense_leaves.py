@@ -1,0 +1,46 @@
+"""Leaves of many particles beside small ones, where the leaf passes change the way they split the work: order p,
+leaves around the split line of the near field (512 particles) and around whole runs of its staged sources (2,048),
+and around the line above which a leaf's P2M takes a block.
+"""
+import numpy as np
+import pytest
+
+import oracle
+from masterthesislucas_gb300 import NBodySolverFMM_SYM_MORTON, Points
+
+pytestmark = pytest.mark.gpu
+
+EPS = 1e-3
+
+
+def cells(sizes, depth, seed=0):
+    """sizes[i] random points in cell i (row-major) of the 2^depth grid over [0, 1)^2, and the box."""
+    rng = np.random.default_rng(seed)
+    w = 1 << depth
+    pts = [(np.array([i % w, i // w]) + 0.01 + 0.98 * rng.random((c, 2))) / w for i, c in enumerate(sizes) if c]
+    return np.concatenate(pts), np.zeros(2), np.ones(2)
+
+
+@pytest.mark.parametrize("kernel", ["tsne", "gravity"])
+@pytest.mark.parametrize("sizes", [(512, 0, 0, 1), (513, 7, 0, 33), (1023, 1, 512, 514), (2047, 0, 0, 0),
+                                   (2048, 1, 0, 0), (4097, 513, 0, 2), (5000, 600, 545, 40)])
+def test_order_p_near_field_of_dense_leaves(kernel, sizes):
+    pos, mn, mx = cells(sizes, 1)
+    pos *= 10.0
+    s = NBodySolverFMM_SYM_MORTON(kernel, tree_depth=1, order=8, theta=0.1, softening=EPS)  # all pairs direct
+    pts = Points.from_positions(pos)
+    s.updateTree(pts, mn, 10.0 * mx)
+    total = s.solveNbody(0.0, pts)
+    k = oracle.KERNEL_TSNE if kernel == "tsne" else oracle.KERNEL_GRAVITY
+    ref, ref_total = oracle.naive(pts.position, kernel=k, eps=EPS)
+    # An FP32 sum of m terms is off by at most (longest chain) 2^-24 sum |f|: chains of 1,024 terms a run and one
+    # term a run, and some 64 roundings of coordinates and of the kernel a term (cancellation in R included: cells
+    # of 5, separations above 5e-6 of them enter with their full weight, so bound the term's error by its largest
+    # derivative times 2^-22 of the cell as well)
+    d = pts.position[:, None, :] - pts.position[None, :, :]
+    r2 = (d * d).sum(-1)
+    w = 1.0 / (1.0 + r2) ** 2 if kernel == "tsne" else (r2 + EPS * EPS) ** -1.5
+    chain = (1024 + len(pos) / 2048 + 64) * 2.0 ** -24 * (w * np.sqrt(r2)).sum(1)
+    shift = 5.0 * 2.0 ** -22 * 3.0 * w.sum(1)
+    assert np.all(np.linalg.norm(pts.derivative - ref, axis=1) <= chain + shift)
+    assert total == pytest.approx(ref_total, rel=1e-4 if kernel == "tsne" else 1e-3)
