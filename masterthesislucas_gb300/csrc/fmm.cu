@@ -9,7 +9,7 @@
 //   k_m2l     one warp per node A: C(A) += M2L(B -> A) for B in nn(A)
 //             (kernelNN, :622-723; the MA0 factor that applyForces later
 //             divides out (:488-492) is never applied)
-//   k_leaf    one warp per non-empty leaf S:
+//   k_leaf_local, k_leaf_near  one block per non-empty leaf S, per 32 sinks of S:
 //             C_S = own C(S) + every ancestor's C shifted to com_S
 //                   (applyForces' L2L chain, :482-519, composed per leaf)
 //                 + P2L from points t of partners T < S with pass(t, S)
@@ -162,11 +162,65 @@ __device__ inline bool pn_pass(double2 x, double2 com, double len, double inv_th
     return dist > thr * thr;
 }
 
+// The point-node MAC from the FP32 offset R = x - com_B (threshold thr =
+// L_B / theta, the same for every non-empty leaf), decided in FP64 by exact()
+// only where the FP32 squared distance is too close to the threshold: at the
+// threshold R is off by at most a few 2^-24 (thr + 3 h), which moves |R|^2 by
+// less than an eighth of the band.  FP64 runs at 1/64 of the FP32 rate, and
+// the test is made for every particle and partner leaf.
+template <typename real, typename F>
+__device__ __forceinline__ bool pn_pass_fast(real Rx, real Ry, real thr, real h, F&& exact)
+{
+    if (sizeof(real) == 4) {
+        const real diff = (Rx * Rx + Ry * Ry) - thr * thr;
+        if (fabs(diff) > real(3.2e-6) * thr * (thr + real(3) * h)) return diff > real(0);
+    }
+    return exact();
+}
+
 constexpr int kLeafWarps = 4;
 
-// phase A, one warp per non-empty leaf S: the final local expansion of S at
-// com_S (own M2L + shifted ancestors + P2L from the passing points of
-// partners T < S), and the number of 32-sink chunks of S
+// 32 entries of a near list, one per lane: leaf, first particle, count and the
+// offset (cell of S - cell of the entry) h
+template <typename real>
+struct NearBatch {
+    uint32_t ti, f, c;
+    real ox, oy;
+    __device__ __forceinline__ void load(const uint32_t* __restrict__ near_idx, const uint32_t* __restrict__ first,
+                                         const uint32_t* __restrict__ count, uint32_t li, uint32_t e, uint32_t e1,
+                                         int isx, int isy, real h)
+    {
+        ti = f = c = 0;
+        ox = oy = real(0);
+        if (e >= e1) return;
+        ti = near_idx[e];
+        f = first[li + ti];
+        c = count[li + ti];
+        ox = real(isx - (int)compact16(ti)) * h;
+        oy = real(isy - (int)compact16(ti >> 1)) * h;
+    }
+    __device__ __forceinline__ NearBatch at(int k) const
+    {
+        NearBatch b;
+        b.ti = __shfl_sync(0xffffffffu, ti, k);
+        b.f = __shfl_sync(0xffffffffu, f, k);
+        b.c = __shfl_sync(0xffffffffu, c, k);
+        b.ox = __shfl_sync(0xffffffffu, ox, k);
+        b.oy = __shfl_sync(0xffffffffu, oy, k);
+        return b;
+    }
+};
+
+// phase A, per non-empty leaf S: the final local expansion of S at com_S (own
+// M2L + shifted ancestors + P2L from the passing points of partners T < S),
+// and the number of 32-sink chunks of S.  A block takes kLeafWarps leaves, a
+// warp each; a leaf of more than kLeafLocalBlock particles, which lies in a
+// dense region, takes a block of its own: a warp alone was a
+// serial chain of up to 10^5 points there (200,003 particles of two disks:
+// 947 us, 172 us now).  The points of 32 partners are one flat range
+// dealt 32 at a time, so that partners of a few points fill the lanes too.
+constexpr uint32_t kLeafLocalBlock = 64;
+
 template <typename real, typename K>
 __global__ void __launch_bounds__(32 * kLeafWarps)
     k_leaf_local(K ker, Geo geo, const uint32_t* __restrict__ count, const uint32_t* __restrict__ first,
@@ -176,33 +230,26 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
                  const real* __restrict__ prel, real* __restrict__ locfin, double* __restrict__ zloc,
                  uint32_t* __restrict__ nchunk, unsigned long long* __restrict__ counters)
 {
+    __shared__ real s_part[kLeafWarps][L_NCOEF];
+    __shared__ double s_z[kLeafWarps];
     uint32_t n_p2l = 0;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int dep = geo.depth;
     const uint32_t li = level_index(dep);
     const int64_t nl = (int64_t)1 << (2 * dep);
-    const real h = (real)geo.h_leaf;
+    const real h = (real)geo.h_leaf, thr = (real)(geo.h_leaf * geo.inv_theta);
     const double inv_theta = geo.inv_theta;
-    const int64_t wstride = (int64_t)gridDim.x * kLeafWarps;
-    for (int64_t si = blockIdx.x * (int64_t)kLeafWarps + w; si < nl; si += wstride) {
+    // leaf si by nv warps, this one taking runs v, v + nv, ... of its partners' points; C and z are the warp's sums
+    auto leaf = [&](int64_t si, int v, int nv, real (&C)[L_NCOEF], double& z) {
         const int64_t S = li + si;
-        const uint32_t cS = count[S];
-        if (lane == 0) nchunk[si] = (cS + 31u) / 32u;
-        if (cS == 0) {
-            if (lane == 0) zloc[si] = 0.0;
-            continue;
-        }
         const int isx = (int)compact16((uint32_t)si), isy = (int)compact16((uint32_t)si >> 1);
-        const double2 comS64 = com64[S];
-        const double lenS = bblen[S];
         const real csx = comrel[2 * S], csy = comrel[2 * S + 1];
         const real mS = m0r[S];
         const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
-        real C[L_NCOEF];
 #pragma unroll
         for (int c = 0; c < L_NCOEF; c++) C[c] = real(0);
         real zA = real(0);
-        if (lane <= dep) {
+        if (v == 0 && lane <= dep) {
             // lane k shifts the expansion of the ancestor at level k (k == dep is S)
             const int k = lane;
             const uint32_t ai = (uint32_t)((uint64_t)si >> (2 * (dep - k)));
@@ -217,18 +264,35 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
             const real dy = h * (((real)isy + real(0.5)) - (iay + real(0.5)) * scale) + (csy - comrel[2 * A + 1]);
             add_shifted(CA, dx, dy, C);
         }
-        for (uint32_t e = e0; e < e1 && !geo.variant; e++) {  // the non-symmetric solver has no P2L here
-            const uint32_t ti = near_idx[e];
-            if (ti >= (uint32_t)si) continue;
-            const int64_t T = li + ti;
-            const uint32_t fT = first[T], cT = count[T];
-            const real ox = real(isx - (int)compact16(ti)) * h, oy = real(isy - (int)compact16(ti >> 1)) * h;
-            for (uint32_t q = lane; q < cT; q += 32) {
-                const uint32_t t = fT + q;
-                if (!pn_pass(pos64[t], comS64, lenS, inv_theta)) continue;
+        // partners T < S: lists are in ascending order, so they come first (the non-symmetric solver has no P2L here)
+        for (uint32_t eb = e0; eb < e1 && !geo.variant; eb += 32) {
+            NearBatch<real> batch;
+            batch.load(near_idx, first, count, li, eb + lane, e1, isx, isy, h);
+            const uint32_t nt = __popc(__ballot_sync(0xffffffffu, eb + lane < e1 && batch.ti < (uint32_t)si));
+            const uint32_t mc = (uint32_t)lane < nt ? batch.c : 0u;
+            uint32_t inc = mc;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t u = __shfl_up_sync(0xffffffffu, inc, o);
+                if (lane >= o) inc += u;
+            }
+            const uint32_t ex = inc - mc, tot = __shfl_sync(0xffffffffu, inc, 31);
+            for (uint32_t base = 32u * (uint32_t)v; base < tot; base += 32u * (uint32_t)nv) {
+                // position q belongs to the last entry that starts at or before it (every entry is a non-empty leaf)
+                const uint32_t q = base + lane;
+                const uint32_t before = __popc(__ballot_sync(0xffffffffu, (uint32_t)lane < nt && ex < base));
+                const uint32_t d = ex - base;
+                const uint32_t bits = __reduce_or_sync(0xffffffffu, ((uint32_t)lane < nt && d < 32u) ? 1u << d : 0u);
+                const int k = (int)(before + __popc(bits & (0xffffffffu >> (31 - lane)))) - 1;
+                const NearBatch<real> T = batch.at(k);
+                const uint32_t exT = __shfl_sync(0xffffffffu, ex, k);
+                if (q >= tot) continue;
+                const uint32_t t = T.f + (q - exT);
                 // R' = com_S - x_t
-                const real Rx = ox + (csx - prel[2 * t]);
-                const real Ry = oy + (csy - prel[2 * t + 1]);
+                const real Rx = T.ox + (csx - prel[2 * t]);
+                const real Ry = T.oy + (csy - prel[2 * t + 1]);
+                if (!pn_pass_fast(Rx, Ry, thr, h, [&] { return pn_pass(pos64[t], com64[S], bblen[S], inv_theta); }))
+                    continue;
                 real D1, D2, D3, tt;
                 ker.far(Rx * Rx + Ry * Ry, D1, D2, D3, tt);
                 C[L_C1X] += Rx * D1;
@@ -237,21 +301,122 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
                 zA += mS * tt;
                 n_p2l++;
             }
+            if (nt < 32u) break;
         }
 #pragma unroll
         for (int c = 0; c < L_NCOEF; c++) C[c] = warp_sum(C[c]);
-        const double z = (double)warp_sum(zA);
+        z = (double)warp_sum(zA);
+    };
+    for (int64_t s0 = blockIdx.x * (int64_t)kLeafWarps; s0 < nl; s0 += (int64_t)gridDim.x * kLeafWarps) {
+        real C[L_NCOEF];
+        double z;
+        const int64_t own = s0 + w;
+        const uint32_t cO = own < nl ? count[li + own] : 0u;
+        if (own < nl) {
+            if (lane == 0) nchunk[own] = (cO + 31u) / 32u;
+            if (cO == 0) {
+                if (lane == 0) zloc[own] = 0.0;
+            } else if (cO <= kLeafLocalBlock) {
+                leaf(own, 0, 1, C, z);
+                if (lane == 0) {
+#pragma unroll
+                    for (int c = 0; c < L_NCOEF; c++) locfin[own * L_NCOEF + c] = C[c];
+                    zloc[own] = z;
+                }
+            }
+        }
+    }
+    for (int64_t si = blockIdx.x; si < nl; si += gridDim.x) {
+        if (count[li + si] <= kLeafLocalBlock) continue;  // the same in the whole block
+        real C[L_NCOEF];
+        double z;
+        leaf(si, w, kLeafWarps, C, z);
         if (lane == 0) {
 #pragma unroll
-            for (int c = 0; c < L_NCOEF; c++) locfin[si * L_NCOEF + c] = C[c];
-            zloc[si] = z;
+            for (int c = 0; c < L_NCOEF; c++) s_part[w][c] = C[c];
+            s_z[w] = z;
         }
+        __syncthreads();
+        if (threadIdx.x < L_NCOEF) {
+            real sum = s_part[0][threadIdx.x];
+#pragma unroll
+            for (int i = 1; i < kLeafWarps; i++) sum += s_part[i][threadIdx.x];
+            locfin[si * L_NCOEF + threadIdx.x] = sum;
+        }
+        if (threadIdx.x == 0) {
+            double sum = s_z[0];
+#pragma unroll
+            for (int i = 1; i < kLeafWarps; i++) sum += s_z[i];
+            zloc[si] = sum;
+        }
+        __syncthreads();
     }
     const unsigned long long c = warp_sum((unsigned long long)n_p2l);
     if (lane == 0 && c) atomicAdd(counters + 2, c);
 }
 
-// phase B, one warp per work item (leaf S, chunk of up to 32 sinks of S)
+// sources a warp of phase B stages before it evaluates them (a multiple of 8
+// per lane of a sink, for 1 to 32 lanes)
+constexpr int kLeafBuf = 256;
+
+// the staged sources of one warp in the sink leaf's frame: FP32 two per
+// 16-byte slot for the packed loop, FP64 one per slot
+template <typename K>
+__device__ __forceinline__ void leaf_stage(float* buf, uint32_t q, float x, float y)
+{
+    buf[(q >> 1) * 4 + (q & 1)] = x;
+    buf[(q >> 1) * 4 + 2 + (q & 1)] = y;
+}
+template <typename K>
+__device__ __forceinline__ void leaf_stage(double* buf, uint32_t q, double x, double y)
+{
+    buf[2 * q] = x;
+    buf[2 * q + 1] = y;
+}
+__device__ __forceinline__ float2 leaf_staged(const float* buf, uint32_t q)
+{
+    return make_float2(buf[(q >> 1) * 4 + (q & 1)], buf[(q >> 1) * 4 + 2 + (q & 1)]);
+}
+__device__ __forceinline__ double2 leaf_staged(const double* buf, uint32_t q)
+{
+    return make_double2(buf[2 * q], buf[2 * q + 1]);
+}
+
+// the sink (px, py) against its lane's share of n staged sources (g lanes a sink, this one the r-th)
+template <typename K>
+__device__ __forceinline__ void leaf_eval(const K& ker, const float* buf, uint32_t n8, uint32_t r, uint32_t g,
+                                          float px, float py, float& gx, float& gy, float& zs)
+{
+    unsigned long long ax = 0ull, ay = 0ull, az = 0ull;
+    p2p_slots(ker, reinterpret_cast<const float4*>(buf), n8 / 2, r, g, px, py, ax, ay, az);
+    gx += K::kSign * f2_total(ax);
+    gy += K::kSign * f2_total(ay);
+    zs += K::kSign * f2_total(az);
+}
+template <typename K>
+__device__ __forceinline__ void leaf_eval(const K& ker, const double* buf, uint32_t n, uint32_t r, uint32_t g,
+                                          double px, double py, double& gx, double& gy, double& zs)
+{
+    for (uint32_t j = r; j < n; j += g) {
+        const double2 s = leaf_staged(buf, j);
+        const double Rx = px - s.x, Ry = py - s.y;
+        double D1, t;
+        ker.near(Rx * Rx + Ry * Ry, D1, t);
+        gx += D1 * Rx;
+        gy += D1 * Ry;
+        zs += t;
+    }
+}
+
+// phase B, one block per work item (leaf S, chunk of up to 32 sinks of S).
+// The P2P pairs bound it.  The block's warps take the 32-point runs of each
+// partner in turn, every warp with all of the item's sinks (a sink of an item
+// of m sinks gets g = 2^floor(log2(32/m)) of a warp's lanes, which split the
+// sources), and stage the points that interact directly, shifted into S's
+// frame, until kLeafBuf of them can be evaluated at once; runs that only some
+// of the sinks see are evaluated by themselves.  The warps' sums are added in
+// warp order.  200,003 particles of two disks, 4,096 leaves, theta 0.5: 2,805 us
+// with a warp per item and one source at a time, 1,547 us now.
 template <typename real, typename K>
 __global__ void __launch_bounds__(32 * kLeafWarps)
     k_leaf_near(K ker, Geo geo, const uint32_t* __restrict__ count, const uint32_t* __restrict__ first,
@@ -262,203 +427,175 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
                 const real* __restrict__ prel, const uint32_t* __restrict__ perm, double* __restrict__ grad,
                 int accumulate, int scatter, double* __restrict__ zwork, unsigned long long* __restrict__ counters)
 {
-    __shared__ real s_src[kLeafWarps][32][2];
+    __shared__ __align__(16) real s_src[kLeafWarps][2 * kLeafBuf];
+    __shared__ real s_part[kLeafWarps][3][32];
     uint32_t n_pp = 0, n_m2p = 0;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    real* buf = s_src[w];
     const int dep = geo.depth;
     const uint32_t li = level_index(dep);
     const int64_t nl = (int64_t)1 << (2 * dep);
-    const real h = (real)geo.h_leaf;
+    const real h = (real)geo.h_leaf, thr = (real)(geo.h_leaf * geo.inv_theta);
     const double inv_theta = geo.inv_theta;
     const uint32_t nwork = chunk_ptr[nl];
-    const int64_t wstride = (int64_t)gridDim.x * kLeafWarps;
-    for (int64_t wi = blockIdx.x * (int64_t)kLeafWarps + w; wi < nwork; wi += wstride) {
+    for (uint32_t wi = blockIdx.x; wi < nwork; wi += gridDim.x) {
         // leaf of this work item: last si with chunk_ptr[si] <= wi
         int64_t lo = 0, hi = nl;
         while (hi - lo > 1) {
             const int64_t mid = (lo + hi) >> 1;
-            if (chunk_ptr[mid] <= (uint32_t)wi) lo = mid; else hi = mid;
+            if (chunk_ptr[mid] <= wi) lo = mid; else hi = mid;
         }
         const int64_t si = lo;
         const int64_t S = li + si;
-        const uint32_t cS = count[S];
         const uint32_t fS = first[S];
-        const uint32_t c0 = ((uint32_t)wi - chunk_ptr[si]) * 32u;
+        const uint32_t c0 = (wi - chunk_ptr[si]) * 32u;
+        const uint32_t m = min(32u, count[S] - c0);
         const int isx = (int)compact16((uint32_t)si), isy = (int)compact16((uint32_t)si >> 1);
-        const double2 comS64 = com64[S];
-        const double lenS = bblen[S];
         const real csx = comrel[2 * S], csy = comrel[2 * S + 1];
         const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
-        real C[L_NCOEF];
-#pragma unroll
-        for (int c = 0; c < L_NCOEF; c++) C[c] = locfin[si * L_NCOEF + c];
-
-        const uint32_t sl = c0 + lane;
-        const bool act = sl < cS;
-        const uint32_t s = fS + (act ? sl : 0);
+        const uint32_t lg = 5u - (32u - __clz(m - 1u));  // log2 g, g * m <= 32
+        const uint32_t g = 1u << lg, r = lane & (g - 1u), sk = lane >> lg;
+        const bool act = sk < m;
+        const uint32_t sl = c0 + (act ? sk : 0u);
+        const uint32_t s = fS + sl;
         const real px = prel[2 * s], py = prel[2 * s + 1];
-        const double2 x64 = pos64[s];
         real gx = real(0), gy = real(0), zs = real(0);
-        if (act) eval_c1(C, px - csx, py - csy, gx, gy);
-        for (uint32_t e = e0; e < e1; e++) {
-            const uint32_t ti = near_idx[e];
-            const int64_t T = li + ti;
-            const uint32_t fT = first[T], cT = count[T];
-            const real ox = real(isx - (int)compact16(ti)) * h, oy = real(isy - (int)compact16(ti >> 1)) * h;
-            // base = x_s - (cell centre of T); each source subtracts its prel
-            const real bx = ox + px, by = oy + py;
-            if (geo.variant) {
-                // non-symmetric: every sink tests every partner T (S itself
-                // included): M2P when L_T / |x - com_T| < theta, else P2P over
-                // T without the sink itself (traverseBHMP, :199-232)
-                const bool pass = act && pn_pass_m(x64, com64[T], bblen[T], geo.theta);
-                if (pass) {
-                    const real Rx = bx - comrel[2 * T], Ry = by - comrel[2 * T + 1];
-                    real D1, D2, D3, t;
-                    ker.far(Rx * Rx + Ry * Ry, D1, D2, D3, t);
-                    const real mT = m0r[T];
-                    real c1x, c1y;
-                    far_c1(Rx, Ry, mT, m2t[3 * T], m2t[3 * T + 1], m2t[3 * T + 2], D1, D2, D3, c1x, c1y);
-                    gx += c1x;
-                    gy += c1y;
-                    zs += mT * t;
-                    n_m2p++;
+        uint32_t fill = 0;
+        // evaluates the staged sources for the sinks of the lanes in `sees`
+        auto flush = [&](bool sees) {
+            if (fill == 0) return;
+            uint32_t n = fill;
+            if (sizeof(real) == 4) {
+                n = (fill + 8u * g - 1u) / (8u * g) * (8u * g);
+                for (uint32_t q = fill + lane; q < n; q += 32u) leaf_stage<K>(buf, q, (real)kFarAway, (real)kFarAway);
+            }
+            __syncwarp();
+            if (sees) {
+                leaf_eval(ker, buf, n, r, g, px, py, gx, gy, zs);
+                if (r == 0) n_pp += fill;
+            }
+            __syncwarp();
+            fill = 0;
+        };
+        // a run of up to 32 points of a partner: those with `take`, in the sink leaf's frame
+        auto append = [&](bool take, real x, real y) {
+            const uint32_t bal = __ballot_sync(0xffffffffu, take);
+            if (take) leaf_stage<K>(buf, fill + __popc(bal & ((1u << lane) - 1u)), x, y);
+            fill += __popc(bal);
+        };
+        for (uint32_t eb = e0; eb < e1; eb += 32) {
+            NearBatch<real> batch;
+            batch.load(near_idx, first, count, li, eb + lane, e1, isx, isy, h);
+            const int nt = (int)min(32u, e1 - eb);
+            for (int k = 0; k < nt; k++) {
+                const uint32_t q1 = 32u * ((w + (uint32_t)k) % kLeafWarps);  // this warp's first run
+                const NearBatch<real> T = batch.at(k);
+                if (q1 > 0 && q1 >= T.c) continue;
+                const int64_t nT = li + T.ti;
+                bool direct = act;
+                if (geo.variant || T.ti > (uint32_t)si) {
+                    // symmetric: S is the first node of the pair and each sink is tested against T; non-symmetric:
+                    // every sink tests every partner T, S itself included (traverseBHMP, :199-232)
+                    const real Rx = (T.ox + px) - comrel[2 * nT], Ry = (T.oy + py) - comrel[2 * nT + 1];
+                    const bool pass = act && pn_pass_fast(Rx, Ry, thr, h, [&] {
+                        return geo.variant ? pn_pass_m(pos64[s], com64[nT], bblen[nT], geo.theta)
+                                           : pn_pass(pos64[s], com64[nT], bblen[nT], inv_theta);
+                    });
+                    if (pass && q1 == 0 && r == 0) {
+                        real D1, D2, D3, t;
+                        ker.far(Rx * Rx + Ry * Ry, D1, D2, D3, t);
+                        const real mT = m0r[nT];
+                        real c1x, c1y;
+                        far_c1(Rx, Ry, mT, m2t[3 * nT], m2t[3 * nT + 1], m2t[3 * nT + 2], D1, D2, D3, c1x, c1y);
+                        gx += c1x;
+                        gy += c1y;
+                        zs += mT * t;
+                        n_m2p++;
+                    }
+                    direct = act && !pass;
                 }
-                const bool direct = act && !pass;
-                if (__any_sync(0xffffffffu, direct)) {
-                    for (uint32_t q0 = 0; q0 < cT; q0 += 32) {
-                        const uint32_t q = q0 + lane;
-                        if (q < cT) {
-                            s_src[w][lane][0] = prel[2 * (fT + q)];
-                            s_src[w][lane][1] = prel[2 * (fT + q) + 1];
-                        }
+                if (!__any_sync(0xffffffffu, direct)) continue;
+                const bool all = __all_sync(0xffffffffu, direct || !act);
+                const bool tested = !geo.variant && T.ti < (uint32_t)si;  // S is the second node of the pair
+                if (!all) flush(act);
+                for (uint32_t q0 = q1; q0 < T.c; q0 += 32u * kLeafWarps) {
+                    const uint32_t q = q0 + lane;
+                    real x = real(0), y = real(0);
+                    bool take = q < T.c;
+                    if (take) {
+                        const uint32_t t = T.f + q;
+                        const real tx = prel[2 * t], ty = prel[2 * t + 1];
+                        // only the points of T that fail the MAC against S interact with the sinks directly
+                        if (tested)
+                            take = !pn_pass_fast(T.ox + (csx - tx), T.oy + (csy - ty), thr, h, [&] {
+                                return pn_pass(pos64[t], com64[S], bblen[S], inv_theta);
+                            });
+                        x = tx - T.ox;
+                        y = ty - T.oy;
+                    }
+                    if (T.ti == (uint32_t)si && q0 == c0) {
+                        // the sinks themselves: each against the others, one at a time
+                        flush(all ? act : direct);
+                        append(take, x, y);
                         __syncwarp();
-                        const uint32_t m = min(32u, cT - q0);
                         if (direct) {
-                            const bool self = ti == (uint32_t)si && sl >= q0 && sl < q0 + m;
-                            n_pp += m - (self ? 1u : 0u);
-                            for (uint32_t j = 0; j < m; j++) {
-                                if (self && q0 + j == sl) continue;
-                                const real Rx = bx - s_src[w][j][0], Ry = by - s_src[w][j][1];
+                            for (uint32_t j = r; j < m; j += g) {
+                                if (j == sk) continue;
+                                const auto src = leaf_staged(buf, j);
+                                const real Rx = px - src.x, Ry = py - src.y;
                                 real D1, t;
                                 ker.near(Rx * Rx + Ry * Ry, D1, t);
                                 gx += D1 * Rx;
                                 gy += D1 * Ry;
                                 zs += t;
                             }
+                            if (r == 0) n_pp += m - 1u;
                         }
                         __syncwarp();
+                        fill = 0;
+                        continue;
                     }
+                    append(take, x, y);
+                    if (fill > kLeafBuf - 32) flush(all ? act : direct);
                 }
-            } else if (ti == (uint32_t)si) {
-                for (uint32_t q0 = 0; q0 < cT; q0 += 32) {
-                    const uint32_t q = q0 + lane;
-                    if (q < cT) {
-                        s_src[w][lane][0] = prel[2 * (fT + q)];
-                        s_src[w][lane][1] = prel[2 * (fT + q) + 1];
-                    }
-                    __syncwarp();
-                    const uint32_t m = min(32u, cT - q0);
-                    if (act) {
-                        n_pp += m - ((sl >= q0 && sl < q0 + m) ? 1u : 0u);
-                        for (uint32_t j = 0; j < m; j++) {
-                            if (q0 + j == sl) continue;
-                            const real Rx = bx - s_src[w][j][0], Ry = by - s_src[w][j][1];
-                            real D1, t;
-                            ker.near(Rx * Rx + Ry * Ry, D1, t);
-                            gx += D1 * Rx;
-                            gy += D1 * Ry;
-                            zs += t;
-                        }
-                    }
-                    __syncwarp();
-                }
-            } else if (ti > (uint32_t)si) {
-                // S is the first node of the pair: each sink is tested against T
-                const bool pass = act && pn_pass(x64, com64[T], bblen[T], inv_theta);
-                if (pass) {
-                    const real Rx = bx - comrel[2 * T], Ry = by - comrel[2 * T + 1];
-                    real D1, D2, D3, t;
-                    ker.far(Rx * Rx + Ry * Ry, D1, D2, D3, t);
-                    const real mT = m0r[T];
-                    real c1x, c1y;
-                    far_c1(Rx, Ry, mT, m2t[3 * T], m2t[3 * T + 1], m2t[3 * T + 2], D1, D2, D3, c1x, c1y);
-                    gx += c1x;
-                    gy += c1y;
-                    zs += mT * t;
-                    n_m2p++;
-                }
-                const bool direct = act && !pass;
-                if (__any_sync(0xffffffffu, direct)) {
-                    for (uint32_t q0 = 0; q0 < cT; q0 += 32) {
-                        const uint32_t q = q0 + lane;
-                        if (q < cT) {
-                            s_src[w][lane][0] = prel[2 * (fT + q)];
-                            s_src[w][lane][1] = prel[2 * (fT + q) + 1];
-                        }
-                        __syncwarp();
-                        const uint32_t m = min(32u, cT - q0);
-                        if (direct) {
-                            n_pp += m;
-                            for (uint32_t j = 0; j < m; j++) {
-                                const real Rx = bx - s_src[w][j][0], Ry = by - s_src[w][j][1];
-                                real D1, t;
-                                ker.near(Rx * Rx + Ry * Ry, D1, t);
-                                gx += D1 * Rx;
-                                gy += D1 * Ry;
-                                zs += t;
-                            }
-                        }
-                        __syncwarp();
-                    }
-                }
-            } else {
-                // S is the second node: the points of T that fail the MAC
-                // against S interact with every sink directly
-                for (uint32_t q0 = 0; q0 < cT; q0 += 32) {
-                    const uint32_t q = q0 + lane;
-                    bool fail = false;
-                    real tx = real(0), ty = real(0);
-                    if (q < cT) {
-                        fail = !pn_pass(pos64[fT + q], comS64, lenS, inv_theta);
-                        tx = prel[2 * (fT + q)];
-                        ty = prel[2 * (fT + q) + 1];
-                    }
-                    const uint32_t bal = __ballot_sync(0xffffffffu, fail);
-                    if (fail) {
-                        const int slot = __popc(bal & ((1u << lane) - 1u));
-                        s_src[w][slot][0] = tx;
-                        s_src[w][slot][1] = ty;
-                    }
-                    __syncwarp();
-                    const int m = __popc(bal);
-                    if (act) {
-                        n_pp += (uint32_t)m;
-                        for (int j = 0; j < m; j++) {
-                            const real Rx = bx - s_src[w][j][0], Ry = by - s_src[w][j][1];
-                            real D1, t;
-                            ker.near(Rx * Rx + Ry * Ry, D1, t);
-                            gx += D1 * Rx;
-                            gy += D1 * Ry;
-                            zs += t;
-                        }
-                    }
-                    __syncwarp();
-                }
+                if (!all) flush(direct);
             }
         }
-        if (act) {
-            const int64_t o = scatter ? (int64_t)perm[s] : (int64_t)s;
-            double ox2 = (double)gx, oy2 = (double)gy;
-            if (accumulate) {
-                ox2 += grad[2 * o];
-                oy2 += grad[2 * o + 1];
-            }
-            grad[2 * o] = ox2;
-            grad[2 * o + 1] = oy2;
+        flush(act);
+        for (uint32_t o = g >> 1; o > 0; o >>= 1) {
+            gx += __shfl_xor_sync(0xffffffffu, gx, o);
+            gy += __shfl_xor_sync(0xffffffffu, gy, o);
         }
-        const double z = warp_sum(act ? (double)zs : 0.0);
-        if (lane == 0) zwork[wi] = z;
+        s_part[w][0][lane] = gx;
+        s_part[w][1][lane] = gy;
+        s_part[w][2][lane] = act ? zs : real(0);
+        __syncthreads();
+        if (w == 0) {
+            real C[L_NCOEF];
+#pragma unroll
+            for (int c = 0; c < L_NCOEF; c++) C[c] = locfin[si * L_NCOEF + c];
+            eval_c1(C, px - csx, py - csy, gx, gy);
+            real z = real(0);
+#pragma unroll
+            for (int i = 0; i < kLeafWarps; i++) {
+                gx += s_part[i][0][lane];
+                gy += s_part[i][1][lane];
+                z += s_part[i][2][lane];
+            }
+            if (act && r == 0) {
+                const int64_t o = scatter ? (int64_t)perm[s] : (int64_t)s;
+                double ox2 = (double)gx, oy2 = (double)gy;
+                if (accumulate) {
+                    ox2 += grad[2 * o];
+                    oy2 += grad[2 * o + 1];
+                }
+                grad[2 * o] = ox2;
+                grad[2 * o + 1] = oy2;
+            }
+            const double zz = warp_sum((double)z);
+            if (lane == 0) zwork[wi] = zz;
+        }
+        __syncthreads();
     }
     const unsigned long long a = warp_sum((unsigned long long)n_pp);
     const unsigned long long b = warp_sum((unsigned long long)n_m2p);
@@ -571,16 +708,14 @@ int solve_t(Handle& h, K ker, double* d_grad, int accumulate, int scatter, doubl
         return rc;
     uint32_t* nchunk = P<uint32_t>(h.cnt_tmp);
     uint32_t* chunk_ptr = P<uint32_t>(h.chunk);
-    const int64_t nblk = (nleaf + kLeafWarps - 1) / kLeafWarps;
-    k_leaf_local<real, K><<<(unsigned)(nblk < sm_count() * 256 ? nblk : sm_count() * 256), 32 * kLeafWarps, 0, s>>>(
+    k_leaf_local<real, K><<<(unsigned)(nleaf < sm_count() * 256 ? nleaf : sm_count() * 256), 32 * kLeafWarps, 0, s>>>(
         ker, geo, P<uint32_t>(h.count), P<uint32_t>(h.first), P<double2>(h.com64), P<double>(h.bblen),
         P<real>(h.comrel), P<real>(h.m0r), loc, ptr + h.lists.near_ptr_off[dep], idx + h.lists.near_idx_off[dep],
         P<double2>(h.pos64), P<real>(h.prel), P<real>(h.locfin), P<double>(h.zloc), nchunk,
         P<unsigned long long>(h.counters));
     if ((rc = exclusive_scan_u32(nchunk, chunk_ptr, nleaf, P<uint32_t>(h.tmp), s))) return rc;
     if ((rc = record(h, 5))) return rc;
-    const int64_t wblk = (wmax + kLeafWarps - 1) / kLeafWarps;
-    k_leaf_near<real, K><<<(unsigned)(wblk < sm_count() * 256 ? wblk : sm_count() * 256), 32 * kLeafWarps, 0, s>>>(
+    k_leaf_near<real, K><<<(unsigned)(wmax < sm_count() * 256 ? wmax : sm_count() * 256), 32 * kLeafWarps, 0, s>>>(
         ker, geo, P<uint32_t>(h.count), P<uint32_t>(h.first), P<double2>(h.com64), P<double>(h.bblen),
         P<real>(h.comrel), P<real>(h.m0r), P<real>(h.m2t), P<real>(h.locfin), ptr + h.lists.near_ptr_off[dep],
         idx + h.lists.near_idx_off[dep], chunk_ptr, P<double2>(h.pos64), P<real>(h.prel), P<uint32_t>(h.perm),

@@ -254,10 +254,14 @@ __global__ void k_lists(int l, double inv_theta, double theta, int variant, real
 // non-empty node, the lanes taking the candidates (parent near entry e, child
 // j) in order 32 at a time; ballots count them and place each accepted /
 // opened entry at its rank, so the lists equal the one-thread form's entry for
-// entry.  FP32 order-p path without per-pair orders; l >= 1.
-__global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, double theta, int variant, float hl,
+// entry.  Without per-pair orders; l >= 1.  act == nullptr (the reference's
+// expansion order): all nodes of the level are visited and the counts of the
+// empty ones written here.  20,011 particles in 4,096 leaves at that order:
+// 319 us for the seven levels with a thread per node, 92 us now.
+template <typename real>
+__global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, double theta, int variant, real hl,
                                                     const uint32_t* __restrict__ count,
-                                                    const double2* __restrict__ com64, const float* __restrict__ comrel,
+                                                    const double2* __restrict__ com64, const real* __restrict__ comrel,
                                                     const double* __restrict__ bblen,
                                                     const uint32_t* __restrict__ pnear_ptr,
                                                     const uint32_t* __restrict__ pnear_idx, uint32_t pcap,
@@ -275,16 +279,23 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
     const int64_t nl = (int64_t)1 << (2 * l);
     const int lane = threadIdx.x & 31;
     const uint32_t lt = (1u << lane) - 1u;
-    const uint32_t k1 = act_pos[li + nl];
+    const uint32_t k0 = act ? act_pos[li] : 0u, k1 = act ? act_pos[li + nl] : (uint32_t)nl;
     const uint32_t wstride = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t k = act_pos[li] + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += wstride) {
-        const int64_t a = (int64_t)act[k] - li;
+    for (uint32_t k = k0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += wstride) {
+        const int64_t a = act ? (int64_t)act[k] - li : (int64_t)k;
+        if (!act && count[li + a] == 0) {
+            if (!fill && lane == 0) {
+                nn_cnt[a] = 0;
+                near_cnt[a] = 0;
+            }
+            continue;
+        }
         const double2 ca = com64[li + a];
         const double len = bblen[li + a];
-        const float thr = (float)((len + len) * inv_theta);
-        const float thr2 = thr * thr;
+        const real thr = (real)((len + len) * inv_theta);
+        const real thr2 = thr * thr;
         const int iax = (int)compact16((uint32_t)a), iay = (int)compact16((uint32_t)a >> 1);
-        const float cra[2] = {comrel[2 * (li + a)], comrel[2 * (li + a) + 1]};
+        const real cra[2] = {comrel[2 * (li + a)], comrel[2 * (li + a) + 1]};
         const float ba = bmax ? bmax[li + a] : 0.f;
         const uint32_t ca_n = p2p_cut ? count[li + a] : 0u;
         const uint32_t p = (uint32_t)(a >> 2);
@@ -302,13 +313,15 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
                 if (bp < np && count[li + b] != 0) {
                     valid = true;
                     if (bmax) {
-                        const float dx = (float)(iax - (int)compact16(b)) * hl + (cra[0] - comrel[2 * (li + b)]);
-                        const float dy = (float)(iay - (int)compact16(b >> 1)) * hl + (cra[1] - comrel[2 * (li + b) + 1]);
+                        const float dx = (float)(iax - (int)compact16(b)) * (float)hl +
+                                         (float)(cra[0] - comrel[2 * (li + b)]);
+                        const float dy = (float)(iay - (int)compact16(b >> 1)) * (float)hl +
+                                         (float)(cra[1] - comrel[2 * (li + b) + 1]);
                         const float rb = ba + bmax[li + b];
                         acc = theta2 * fmaf(dx, dx, dy * dy) > rb * rb;
                     } else {
-                        acc = mac_accept_fast<float>(iax - (int)compact16(b), iay - (int)compact16(b >> 1), hl, thr2,
-                                                     cra, comrel + 2 * (li + b), ca, com64[li + b], len, inv_theta,
+                        acc = mac_accept_fast<real>(iax - (int)compact16(b), iay - (int)compact16(b >> 1), hl, thr2,
+                                                    cra, comrel + 2 * (li + b), ca, com64[li + b], len, inv_theta,
                                                      theta, variant);
                     }
                     if (acc && p2p_cut && ca_n * count[li + b] <= p2p_cut) acc = false;
@@ -628,6 +641,11 @@ int build_lists(Handle& h)
                                                                     P<uint8_t>(h.dec), nnp, nni, ordp, nncap, nrp,
                                                                     nri, nrcap, ovf_flag, act, act_pos);
             }
+        } else if (h.cfg.precision == TC_PREC_FP64 && l > 0 && nl <= kListsWarpLevelNodes) {
+            k_lists_warp<double><<<grid_for(nl * 32, 128), 128, 0, s>>>(
+                l, inv_theta, h.cfg.theta, h.variant, hl, P<uint32_t>(h.count), P<double2>(h.com64),
+                P<double>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnc, nrc, nnp, nni, nncap, nrp, nri, nrcap,
+                ovf_flag, fill, nullptr, nullptr, nullptr, 0.f, 0u);
         } else if (h.cfg.precision == TC_PREC_FP64) {
             k_lists<double><<<grid_for(nl, 128), 128, 0, s>>>(l, inv_theta, h.cfg.theta, h.variant, hl,
                                                              P<uint32_t>(h.count),
@@ -642,12 +660,12 @@ int build_lists(Handle& h)
                 int rc2 = ensure(h.dec, (size_t)pcap * 4 + 64);
                 if (rc2) return rc2;
             }
-            if (act && !adapt && l > 0 && nl <= kListsWarpLevelNodes) {
-                k_lists_warp<<<grid_for(nl * 32, 128), 128, 0, s>>>(
+            if (!adapt && l > 0 && nl <= kListsWarpLevelNodes) {
+                k_lists_warp<float><<<grid_for(nl * 32, 128), 128, 0, s>>>(
                     l, inv_theta, h.cfg.theta, h.variant, (float)hl, P<uint32_t>(h.count), P<double2>(h.com64),
                     P<float>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnc, nrc, nnp, nni, nncap, nrp, nri, nrcap,
                     ovf_flag, fill, act, act_pos, bmax, (float)(h.cfg.theta * h.cfg.theta),
-                    l == depth ? h.p2p_cut : 0u);
+                    act && l == depth ? h.p2p_cut : 0u);
                 return 0;
             }
             k_lists<float><<<grid_for(nl, 128), 128, 0, s>>>(l, inv_theta, h.cfg.theta, h.variant, (float)hl,

@@ -1,12 +1,15 @@
-"""Leaves of many particles beside small ones, where the leaf passes change the way they split the work: order p,
-leaves around the split line of the near field (512 particles) and around whole runs of its staged sources (2,048),
-and around the line above which a leaf's P2M takes a block.
+"""Leaves of many particles beside small ones, where the leaf passes change the way they split the work.
+
+* order p: leaves around the split line of the near field (512 particles) and around whole runs of its staged
+  sources (2,048), and around the line above which a leaf's P2M takes a block;
+* the reference's expansion order: leaves around a lane's, a warp's and a block's share of the moments, the P2L and
+  the point stage.
 """
 import numpy as np
 import pytest
 
 import oracle
-from masterthesislucas_gb300 import NBodySolverFMM_SYM_MORTON, Points
+from masterthesislucas_gb300 import NBodySolverFMM_MORTON, NBodySolverFMM_SYM_MORTON, Points
 
 pytestmark = pytest.mark.gpu
 
@@ -19,6 +22,10 @@ def cells(sizes, depth, seed=0):
     w = 1 << depth
     pts = [(np.array([i % w, i // w]) + 0.01 + 0.98 * rng.random((c, 2))) / w for i, c in enumerate(sizes) if c]
     return np.concatenate(pts), np.zeros(2), np.ones(2)
+
+
+def rel_err(a, b):
+    return np.linalg.norm(a - b, axis=1) / np.maximum(np.linalg.norm(b, axis=1), 1e-300)
 
 
 @pytest.mark.parametrize("kernel", ["tsne", "gravity"])
@@ -44,3 +51,33 @@ def test_order_p_near_field_of_dense_leaves(kernel, sizes):
     shift = 5.0 * 2.0 ** -22 * 3.0 * w.sum(1)
     assert np.all(np.linalg.norm(pts.derivative - ref, axis=1) <= chain + shift)
     assert total == pytest.approx(ref_total, rel=1e-4 if kernel == "tsne" else 1e-3)
+
+
+REF_SIZES = [0, 1, 7, 8, 9, 31, 32, 33, 63, 64, 65, 129, 300, 0, 2, 700]
+
+
+@pytest.mark.parametrize("kernel", ["tsne", "gravity"])
+@pytest.mark.parametrize("theta", [0.3, 1.0])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_reference_order_dense_leaves(kernel, theta, precision, symmetric):
+    pos, mn, mx = cells(REF_SIZES, 2)
+    k = oracle.KERNEL_TSNE if kernel == "tsne" else oracle.KERNEL_GRAVITY
+    cls = NBodySolverFMM_SYM_MORTON if symmetric else NBodySolverFMM_MORTON
+    s = cls(kernel, tree_depth=2, theta=theta, softening=EPS, precision=precision)
+    pts = Points.from_positions(pos)
+    s.updateTree(pts, mn, mx)
+    total = s.solveNbody(0.0, pts)
+    ref = oracle.sym_fmm(pos, kernel=k, eps=EPS, depth=2, theta=theta, mn=mn, mx=mx, symmetric=symmetric)
+    np.testing.assert_array_equal(pts.ID, ref["ids"])
+    nodes = s.tree_dump()["nodes"]  # ..., count at 5, centre of mass at 6, M0 at 8, M2 at 9
+    np.testing.assert_array_equal(nodes[:, 5], ref["nodes"]["count"])
+    np.testing.assert_array_equal(nodes[:, 6:8], ref["nodes"]["com"])
+    np.testing.assert_array_equal(nodes[:, 9:13], ref["nodes"]["m2"])
+    err = rel_err(pts.derivative, ref["grad"])
+    if precision == "fp64":
+        assert err.max() < 1e-10
+        assert total == pytest.approx(ref["total"], rel=1e-10)
+    else:
+        assert np.median(err) <= 2e-6 and err.max() <= 1e-3
+        assert total == pytest.approx(ref["total"], rel=2e-6)
