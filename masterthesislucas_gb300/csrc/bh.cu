@@ -11,10 +11,22 @@
 // Masses and COMs (quadtree.h:137-172) are rebuilt bottom-up with the
 // reference's types: float totalMass, FP64 COM, and the child COM seen by the
 // parent through std::pair<float, glm::vec2>, i.e. rounded to float.
-// Traversal (nBodySolverBH.h:56-89): one thread per point, depth-first in the
+// Traversal (nBodySolverBH.h:56-89): per point, depth-first in the
 // children order with the MAC l/|x - com| < theta; a node with at most one
 // child is treated as a leaf (PP over all its occupants).  In FP64 the
 // result is the reference's, bit for bit (same operations, same order).
+//
+// Trees of up to kPathLevels levels (all but clusters of nearly coincident
+// points) are built by one sort instead: a point's quadrants level by level
+// are a key, the key order is the depth-first order, and a node is a run of
+// keys with a common prefix.  Nodes are numbered depth first, so the
+// traversal needs no stack: the next node is the following one, or the one
+// after the subtree.  It visits the nodes a warp at a time, the warp's 32
+// points being neighbours in key order.  65,536 points of a Gaussian mixture,
+// leaves of 16, theta 0.5: 190 launches and 10 host round trips before,
+// 32 and one now; traversal 3,546 us with a thread per point in input order and
+// the MAC in FP64, 206 us now.  Deeper trees take the level-synchronous
+// build and the per-point traversal, which know no depth limit.
 //
 // The multipole variant (NBodySolverBHMP + QuadTreeMultiPole,
 // src/nbodysolvers/cpu/nBodySolverBHMP.h:17-135,
@@ -24,6 +36,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.cuh"
@@ -339,12 +352,408 @@ __global__ void __launch_bounds__(128) k_bh_traverse(K ker, const double2* __res
     }
 }
 
+// ---------------------------------------------------------------- path keys
+constexpr int kPathLevels = 16;
+// largest maxChildren of the sorted build, whose leaves are ordered by counting (a point against its leaf's others)
+constexpr int kPathMaxLeaf = 256;
+
+// sorted-build node records, depth-first order
+struct PathNodes {
+    uint32_t* start;    // occupants [start, end) in tree order
+    uint32_t* end;
+    uint32_t* skip;     // the node after the subtree
+    uint32_t* parent;
+    uint32_t* nchild;
+    uint32_t* arrived;  // children done (bottom-up pass)
+    double* len;        // box length
+    float* mass;        // monopole variant: the reference's float mass and the COM its parent sees
+    float2* comf;
+    double2* com;
+    double* m64;        // multipole variant
+    Quad* quad;
+    float4* rec;        // [2 i]: COM relative to the root corner, high and low parts (x, y, x, y);
+                        // [2 i + 1]: l / theta, mass, leaf flag, unused
+    float4* mom;        // multipole variant, FP32: quadrupole / mass
+};
+
+__device__ __forceinline__ void root_box(const double* keys, double2& lo, double& hix)
+{
+    const unsigned long long* k = reinterpret_cast<const unsigned long long*>(keys);
+    const double lx = bbox_unkey(k[0]), ly = bbox_unkey(k[1]);
+    const double ax = bbox_unkey(k[2]) - lx, ay = bbox_unkey(k[3]) - ly;
+    const double ld = (ax < ay) ? ay : ax;  // std::max(a, b)
+    lo = make_double2(lx, ly);
+    hix = lx + ld + 0.0001;
+}
+
+// one level down: the box of quadrant qd (quadtree.h:104-134; the upper y edge is never read)
+__device__ __forceinline__ void child_box(int qd, double2& lo, double& hix)
+{
+    const double l = (hix - lo.x) / 2.0;
+    const double mx = lo.x + l, my = lo.y + l;
+    if (qd < 2) lo.x = mx; else hix = mx;
+    if ((qd & 1) == 0) lo.y = my;
+}
+
+__global__ void k_path_keys(const double2* __restrict__ pos, uint32_t n, const double* __restrict__ bbox,
+                            uint32_t* __restrict__ keys)
+{
+    double2 rlo;
+    double rhi;
+    root_box(bbox, rlo, rhi);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double2 p = pos[i];
+        double2 lo = rlo;
+        double hix = rhi;
+        uint32_t key = 0;
+        for (int l = 0; l < kPathLevels; l++) {
+            const int qd = quadrant(p.x, p.y, lo, make_double2(hix, 0.0));
+            child_box(qd, lo, hix);
+            key = key << 2 | (uint32_t)qd;
+        }
+        keys[i] = key;
+    }
+}
+
+// leading quadrants two keys share
+__device__ __forceinline__ int common_levels(uint32_t a, uint32_t b)
+{
+    return a == b ? kPathLevels : __clz((int)(a ^ b)) >> 1;
+}
+
+// first index in [a, b) whose key's leading l quadrants are not below those of key (above: beyond those of key)
+__device__ __forceinline__ uint32_t path_bound(const uint32_t* __restrict__ keys, uint32_t a, uint32_t b, uint32_t key,
+                                               int l, bool above)
+{
+    const int sh = 2 * (kPathLevels - l);
+    const uint64_t v = ((uint64_t)key >> sh) + (above ? 1u : 0u);
+    while (a < b) {
+        const uint32_t mid = (a + b) >> 1;
+        if (((uint64_t)keys[mid] >> sh) < v) a = mid + 1;
+        else b = mid;
+    }
+    return a;
+}
+
+// per sorted point: the level of its leaf (the first with at most maxc occupants), the nodes that begin at it, and its
+// place in the leaf (the reference keeps a node's occupants in input order).  A leaf of more than maxc points at
+// level kPathLevels sets *deep.
+__global__ void k_path_leaves(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ perm, uint32_t n,
+                              uint32_t maxc, const double2* __restrict__ pos, const double* __restrict__ bbox,
+                              uint8_t* __restrict__ depth, uint32_t* __restrict__ nbegin,
+                              uint32_t* __restrict__ order, double2* __restrict__ psort, float4* __restrict__ prel,
+                              uint32_t* __restrict__ deep)
+{
+    double2 rlo;
+    double rhi;
+    root_box(bbox, rlo, rhi);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t key = keys[i];
+        uint32_t a = 0, b = n;
+        int l = 0;
+        while (b - a > maxc && l < kPathLevels) {
+            l++;
+            a = path_bound(keys, a, i, key, l, false);
+            b = path_bound(keys, i, b, key, l, true);
+        }
+        if (b - a > maxc) {
+            atomicOr(deep, 1u);
+            b = a;  // no place in the leaf is needed: the build is given up
+        }
+        const int shared = i ? common_levels(keys[i - 1], key) : -1;
+        depth[i] = (uint8_t)l;
+        nbegin[i] = l > shared ? (uint32_t)(l - shared) : 0u;
+        const uint32_t o = perm[i];
+        uint32_t r = a;
+        for (uint32_t j = a; j < b; j++) r += perm[j] < o;
+        if (a == b) r = i;
+        const double2 p = pos[o];
+        order[r] = o;
+        psort[r] = p;
+        const double rx = p.x - rlo.x, ry = p.y - rlo.y;
+        const float hx = (float)rx, hy = (float)ry;
+        prel[r] = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
+    }
+}
+
+// the nodes that begin at each sorted point, numbered from base[i] on by level
+__global__ void k_path_nodes(const uint32_t* __restrict__ keys, const uint8_t* __restrict__ depth,
+                             const uint32_t* __restrict__ base, uint32_t n, const double* __restrict__ bbox,
+                             PathNodes t)
+{
+    double2 rlo;
+    double rhi;
+    root_box(bbox, rlo, rhi);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t key = keys[i], b0 = base[i];
+        const int nl = (int)(base[i + 1] - b0);
+        if (nl == 0) continue;
+        const int l1 = depth[i], l0 = l1 - nl + 1;
+        // ends from the leaf up: a node's subtree holds its first child's
+        uint32_t e = i + 1;
+        for (int l = l1; l >= l0; l--) {
+            const uint32_t nd = b0 + (uint32_t)(l - l0);
+            e = path_bound(keys, e, n, key, l, true);
+            t.start[nd] = i;
+            t.end[nd] = e;
+            t.skip[nd] = base[e];
+            uint32_t par = nd - 1;
+            if (l == l0 && l > 0) {
+                // the level l - 1 node that holds i begins earlier
+                const uint32_t p0 = path_bound(keys, 0, i, key, l - 1, false);
+                par = base[p0] + (base[p0 + 1] - base[p0]) - 1u - (uint32_t)(depth[p0] - (l - 1));
+            }
+            t.parent[nd] = par;
+            if (l > 0) atomicAdd(&t.nchild[par], 1u);
+        }
+        double2 lo = rlo;
+        double hix = rhi;
+        for (int l = 0;; l++) {
+            if (l >= l0) t.len[b0 + (uint32_t)(l - l0)] = hix - lo.x;
+            if (l == l1) break;
+            child_box((int)(key >> (2 * (kPathLevels - 1 - l)) & 3u), lo, hix);
+        }
+    }
+}
+
+// masses, COMs and quadrupoles bottom up with the reference's types and orders (k_bh_mass, k_bhmp_moments): a thread
+// per leaf, and the last child to arrive goes on with the parent
+template <bool MP>
+__global__ void k_path_moments(uint32_t total, PathNodes t, const double2* __restrict__ psort,
+                               const double* __restrict__ bbox, double theta)
+{
+    double2 rlo;
+    double rhi;
+    root_box(bbox, rlo, rhi);
+    for (uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x; leaf < total; leaf += gridDim.x * blockDim.x) {
+        if (t.nchild[leaf] != 0) continue;
+        uint32_t nd = leaf;
+        while (true) {
+            double cx = 0.0, cy = 0.0, m = 0.0;
+            const uint32_t nch = t.nchild[nd], e = t.skip[nd];
+            if constexpr (MP) {
+                Quad q = {0.0, 0.0, 0.0, 0.0};
+                if (nch == 0) {
+                    for (uint32_t i = t.start[nd]; i < t.end[nd]; i++) {
+                        const double2 p = psort[i];
+                        m += 1.0;
+                        cx += 1.0 * p.x;
+                        cy += 1.0 * p.y;
+                    }
+                    cx /= m;
+                    cy /= m;
+                    for (uint32_t i = t.start[nd]; i < t.end[nd]; i++) {
+                        const double2 p = psort[i];
+                        const double rx = p.x - cx, ry = p.y - cy;
+                        q.x += rx * rx;
+                        q.y += rx * ry;
+                        q.z += ry * rx;
+                        q.w += ry * ry;
+                    }
+                } else {
+                    for (uint32_t c = nd + 1; c != e; c = t.skip[c]) {
+                        const double mc = __ldcg(t.m64 + c);
+                        const double2 cc = __ldcg(t.com + c);
+                        m += mc;
+                        cx += mc * cc.x;
+                        cy += mc * cc.y;
+                    }
+                    cx /= m;
+                    cy /= m;
+                    for (uint32_t c = nd + 1; c != e; c = t.skip[c]) {
+                        const double mc = __ldcg(t.m64 + c);
+                        const double2 cc = __ldcg(t.com + c);
+                        const double rx = cc.x - cx, ry = cc.y - cy;
+                        const double* qc = reinterpret_cast<const double*>(t.quad + c);
+                        q.x += mc * (rx * rx);
+                        q.y += mc * (rx * ry);
+                        q.z += mc * (ry * rx);
+                        q.w += mc * (ry * ry);
+                        q.x += __ldcg(qc);
+                        q.y += __ldcg(qc + 1);
+                        q.z += __ldcg(qc + 2);
+                        q.w += __ldcg(qc + 3);
+                    }
+                }
+                t.m64[nd] = m;
+                t.com[nd] = make_double2(cx, cy);
+                t.quad[nd] = q;
+                const double inv = 1.0 / (double)(float)m;
+                t.mom[nd] = make_float4((float)(inv * q.x), (float)(inv * q.y), (float)(inv * q.z), (float)(inv * q.w));
+            } else {
+                float tm = 0.0f;
+                if (nch == 0) {
+                    for (uint32_t i = t.start[nd]; i < t.end[nd]; i++) {
+                        tm = (float)((double)tm + 1.0);
+                        const double2 p = psort[i];
+                        cx += 1.0 * p.x;
+                        cy += 1.0 * p.y;
+                    }
+                } else {
+                    for (uint32_t c = nd + 1; c != e; c = t.skip[c]) {
+                        const double mc = (double)__ldcg(t.mass + c);
+                        tm = (float)((double)tm + mc);
+                        const float2 cc = __ldcg(t.comf + c);
+                        cx += mc * (double)cc.x;
+                        cy += mc * (double)cc.y;
+                    }
+                }
+                cx /= (double)tm;
+                cy /= (double)tm;
+                t.mass[nd] = tm;
+                t.com[nd] = make_double2(cx, cy);
+                t.comf[nd] = make_float2((float)cx, (float)cy);
+                m = (double)tm;
+            }
+            const double rx = cx - rlo.x, ry = cy - rlo.y;
+            const float hx = (float)rx, hy = (float)ry;
+            t.rec[2 * (size_t)nd] = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
+            t.rec[2 * (size_t)nd + 1] = make_float4((float)(t.len[nd] / theta), (float)m, nch <= 1 ? 1.0f : 0.0f, 0.0f);
+            if (nd == 0) break;
+            const uint32_t par = t.parent[nd];
+            __threadfence();
+            if (atomicAdd(&t.arrived[par], 1u) + 1u < t.nchild[par]) break;
+            __threadfence();
+            nd = par;
+        }
+    }
+}
+
+// a - b of two (high, low) pairs of coordinates relative to the root corner, to FP32 accuracy whatever they cancel
+__device__ __forceinline__ float2 split_sub(float4 a, float4 b)
+{
+    return make_float2((a.x - b.x) + (a.z - b.z), (a.y - b.y) + (a.w - b.w));
+}
+
+constexpr int kPathThreads = 64;  // few points leave few warps: small blocks spread them evenly
+
+// traverseBH, a warp per 32 points neighbouring in tree order: the warp walks the nodes depth first, going into a
+// node while any of its points opens it; a point that has accepted a node sits out the subtree.  Each point meets
+// its nodes in the order it would alone.  The MAC is decided in FP32 and, within 1e-5 of its threshold (the FP32
+// square is good to 3e-7), as the reference decides it.
+template <typename real, typename K, bool MP>
+__global__ void __launch_bounds__(kPathThreads) k_path_traverse(K ker, uint32_t n, uint32_t total, PathNodes t,
+                                                       const double2* __restrict__ psort,
+                                                       const float4* __restrict__ prel,
+                                                       const uint32_t* __restrict__ order, double theta,
+                                                       double* __restrict__ grad, double* __restrict__ zrow)
+{
+    constexpr bool kF32 = sizeof(real) == 4;
+    for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < n; p0 += gridDim.x * blockDim.x) {
+        const uint32_t i = p0 + (threadIdx.x & 31);
+        const bool valid = i < n;
+        const float4 xs = valid ? prel[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const double2 x = valid ? psort[i] : make_double2(0.0, 0.0);
+        real gx = 0, gy = 0, z = 0;
+        uint32_t resume = valid ? 0u : total;  // nodes before this one are not this point's
+        for (uint32_t nd = 0; nd < total;) {
+            const float4 c = t.rec[2 * (size_t)nd], r = t.rec[2 * (size_t)nd + 1];
+            const uint32_t skip = t.skip[nd];
+            const bool on = nd >= resume;
+            const float2 d = split_sub(xs, c);
+            const float d2 = d.x * d.x + d.y * d.y, thr2 = r.x * r.x;
+            bool pass = d2 > thr2;
+            if (on && !(fabsf(d2 - thr2) > 1e-5f * thr2 && thr2 > 1e-30f)) {
+                const double2 com = t.com[nd];
+                const double ex = x.x - com.x, ey = x.y - com.y;
+                pass = t.len[nd] / sqrt(ex * ex + ey * ey) < theta;
+            }
+            if (on && pass) {
+                resume = skip;
+                if constexpr (kF32) {
+                    if constexpr (MP) {
+                        const float4 q = t.mom[nd];
+                        real D1, D2, D3, tt;
+                        ker.far(d2, D1, D2, D3, tt);
+                        const real S2 = (d.x * d.x * q.x) + (d.x * d.y * q.y) + (d.y * d.x * q.z) + (d.y * d.y * q.w);
+                        const real base = D1 + real(0.5) * (q.x + q.w) * D2 + real(0.5) * S2 * D3;
+                        z += r.y * tt;
+                        gx += r.y * (d.x * base + (d.x * q.x + d.y * q.y) * D2);
+                        gy += r.y * (d.y * base + (d.x * q.z + d.y * q.w) * D2);
+                    } else {
+                        real D1, tt;
+                        ker.near(d2, D1, tt);
+                        z += r.y * tt;
+                        gx += r.y * D1 * d.x;
+                        gy += r.y * D1 * d.y;
+                    }
+                } else {
+                    const double2 com = t.com[nd];
+                    const double dx = x.x - com.x, dy = x.y - com.y;
+                    if constexpr (MP) {
+                        const real tm = (real)t.m64[nd];
+                        real D1, D2, D3, tt;
+                        ker.far((real)(dx * dx + dy * dy), D1, D2, D3, tt);
+                        real cx1, cy1;
+                        bh_far_c1<real>((real)dx, (real)dy, tm, t.quad[nd], D1, D2, D3, cx1, cy1);
+                        z += tm * tt;
+                        gx += cx1;
+                        gy += cy1;
+                    } else {
+                        const real tm = (real)t.mass[nd];
+                        real D1, tt;
+                        ker.near((real)(dx * dx + dy * dy), D1, tt);
+                        z += tm * tt;
+                        gx += tm * D1 * (real)dx;
+                        gy += tm * D1 * (real)dy;
+                    }
+                }
+            }
+            const bool open = on && !pass;
+            const bool any = __any_sync(0xffffffffu, open);
+            if (any && r.z == 0.0f) {
+                nd++;
+                continue;
+            }
+            if (any) {
+                const uint32_t e = t.end[nd];
+                if constexpr (kF32) {
+                    // summed by themselves first: fewer roundings against the running sums
+                    real lx = 0, ly = 0, lz = 0;
+#pragma unroll 4
+                    for (uint32_t j = t.start[nd]; j < e; j++) {
+                        const float2 f = split_sub(xs, prel[j]);
+                        real D1, tt;
+                        ker.near(f.x * f.x + f.y * f.y, D1, tt);
+                        const bool use = open && j != i;
+                        lz += use ? tt : real(0);
+                        lx += use ? D1 * f.x : real(0);
+                        ly += use ? D1 * f.y : real(0);
+                    }
+                    gx += lx;
+                    gy += ly;
+                    z += lz;
+                } else if (open) {
+                    for (uint32_t j = t.start[nd]; j < e; j++) {
+                        if (j == i) continue;
+                        const double2 q = psort[j];
+                        const double ex = x.x - q.x, ey = x.y - q.y;
+                        real D1, tt;
+                        ker.near((real)(ex * ex + ey * ey), D1, tt);
+                        z += tt;
+                        gx += D1 * (real)ex;
+                        gy += D1 * (real)ey;
+                    }
+                }
+            }
+            nd = skip;
+        }
+        if (valid) {
+            const uint32_t o = order[i];
+            grad[2 * (size_t)o] = (double)gx;
+            grad[2 * (size_t)o + 1] = (double)gy;
+            zrow[o] = (double)z;
+        }
+    }
+}
+
 // Scratch of one call, carved from a per-device workspace that persists
 // between calls and only grows (calls on one device are serialised by its
 // mutex), so that repeated solves allocate nothing after the first.
 struct BHWork {
     std::mutex mu;
-    Buf slot[32];
+    Buf slot[64];
+    cudaStream_t stream = nullptr;  // of the host entry points
     cudaEvent_t done = nullptr;  // recorded after each call's last use of the workspace
     bool recorded = false;
 };
@@ -384,7 +793,7 @@ thread_local int g_slot = 0;
 template <typename T>
 int dalloc(DevBuf& b, size_t count)
 {
-    if (!g_work || g_slot >= 32) {
+    if (!g_work || g_slot >= 64) {
         tc_set_error("bh: workspace slots exhausted");
         return TC_ERR_STATE;
     }
@@ -406,31 +815,100 @@ using namespace tc;
 namespace tc {
 namespace {
 
-int bh_solve_impl(int kernel, double softening, int max_children, double theta, int precision,
-                  const double* d_pos_xy, int64_t n64, double* d_grad_xy, double* d_total, void* stream, bool mp)
+// launches the traversal of either tree; F(ker, real(), mp) does the launch
+template <typename F>
+void bh_dispatch(int kernel, double softening, int precision, bool mp, F&& f)
 {
-    if (!d_pos_xy || !d_grad_xy || n64 <= 0 || n64 > (1 << 30) || max_children <= 0 || !(theta > 0.0) ||
-        (kernel != TC_KERNEL_TSNE && kernel != TC_KERNEL_GRAVITY)) {
-        tc_set_error("tc_bh_solve_device: invalid arguments");
+    const double e2 = softening * softening;
+    auto with_mp = [&](auto ker, auto zero) {
+        if (mp) f(ker, zero, std::true_type());
+        else f(ker, zero, std::false_type());
+    };
+    if (precision == TC_PREC_FP64) {
+        if (kernel == TC_KERNEL_GRAVITY) with_mp(KGrav<double>{e2}, 0.0);
+        else with_mp(KTsne<double>{}, 0.0);
+    } else {
+        if (kernel == TC_KERNEL_GRAVITY) with_mp(KGrav<float>{(float)e2}, 0.0f);
+        else with_mp(KTsne<float>{}, 0.0f);
+    }
+}
+
+// Builds the tree by sorting path keys and walks it.  1: the tree is not one for it (deeper than kPathLevels, or more
+// nodes than the level-synchronous build would accept, which then refuses it); nothing has been written that the
+// caller sees.
+int bh_path_solve(int kernel, double softening, int max_children, double theta, int precision, const double2* pos,
+                  uint32_t n, double* d_grad_xy, double* zrow, cudaStream_t s, bool mp, const double* bbox,
+                  uint32_t* err, size_t cap)
+{
+    int rc;
+    DevBuf b_keys, b_perm, b_akeys, b_avals, b_tmp, b_depth, b_nbegin, b_base, b_order, b_psort, b_prel;
+    const int64_t tw = radix_tmp_words(n) > scan_tmp_words(n) ? radix_tmp_words(n) : scan_tmp_words(n);
+    if ((rc = dalloc<uint32_t>(b_keys, n)) || (rc = dalloc<uint32_t>(b_perm, n)) ||
+        (rc = dalloc<uint32_t>(b_akeys, n)) || (rc = dalloc<uint32_t>(b_avals, n)) ||
+        (rc = dalloc<uint32_t>(b_tmp, (size_t)tw)) || (rc = dalloc<uint8_t>(b_depth, n)) ||
+        (rc = dalloc<uint32_t>(b_nbegin, n)) || (rc = dalloc<uint32_t>(b_base, (size_t)n + 1)) ||
+        (rc = dalloc<uint32_t>(b_order, n)) || (rc = dalloc<double2>(b_psort, n)) || (rc = dalloc<float4>(b_prel, n)))
+        return rc;
+    uint32_t *keys = (uint32_t*)b_keys.p, *perm = (uint32_t*)b_perm.p, *base = (uint32_t*)b_base.p;
+    uint32_t* order = (uint32_t*)b_order.p;
+    double2* psort = (double2*)b_psort.p;
+    float4* prel = (float4*)b_prel.p;
+    k_path_keys<<<grid_for(n, 128), 128, 0, s>>>(pos, n, bbox, keys);
+    if ((rc = radix_sort_u32(keys, perm, (uint32_t*)b_akeys.p, (uint32_t*)b_avals.p, n, (uint32_t*)b_tmp.p, s, nullptr,
+                             0)))
+        return rc;
+    k_path_leaves<<<grid_for(n, 128), 128, 0, s>>>(keys, perm, n, (uint32_t)max_children, pos, bbox,
+                                                   (uint8_t*)b_depth.p, (uint32_t*)b_nbegin.p, order, psort, prel,
+                                                   err + 1);
+    if ((rc = exclusive_scan_u32((uint32_t*)b_nbegin.p, base, n, (uint32_t*)b_tmp.p, s))) return rc;
+    uint32_t total = 0, flags[2] = {0, 0};
+    TC_CUDA_TRY(cudaMemcpyAsync(&total, base + n, 4, cudaMemcpyDeviceToHost, s));
+    TC_CUDA_TRY(cudaMemcpyAsync(flags, err, 8, cudaMemcpyDeviceToHost, s));
+    TC_CUDA_TRY(cudaStreamSynchronize(s));
+    if (flags[0]) {
+        tc_set_error("tc_bh_solve_device: positions contain NaN or infinity");
         return TC_ERR_INVALID;
     }
-    const uint32_t n = (uint32_t)n64;
-    cudaStream_t s = (cudaStream_t)stream;
-    int rc = TC_OK;
-    int dev = 0;
-    TC_CUDA_TRY(cudaGetDevice(&dev));
-    BHWork& work = bh_work(dev);
-    std::lock_guard<std::mutex> work_lock(work.mu);
-    if (!work.done) TC_CUDA_TRY(cudaEventCreateWithFlags(&work.done, cudaEventDisableTiming));
-    // the previous call's kernels (possibly on another stream) finish first
-    if (work.recorded) TC_CUDA_TRY(cudaStreamWaitEvent(s, work.done, 0));
-    WorkRelease release_on_exit{work, s};
-    g_work = &work;
-    g_slot = 0;
-    // node capacity (splits past it are refused, not written)
-    const size_t cap = (size_t)4 * n + 64;
+    if (flags[1] || total > cap) return 1;
+    // sized by the points, so that the workspace does not grow with every tree
+    const size_t nn = total > n ? total : n;
+    DevBuf b_start, b_end, b_skip, b_parent, b_cnt, b_len, b_mass, b_comf, b_com, b_m64, b_quad, b_rec, b_mom;
+    if ((rc = dalloc<uint32_t>(b_start, nn)) || (rc = dalloc<uint32_t>(b_end, nn)) ||
+        (rc = dalloc<uint32_t>(b_skip, nn)) || (rc = dalloc<uint32_t>(b_parent, nn)) ||
+        (rc = dalloc<uint32_t>(b_cnt, 2 * nn)) || (rc = dalloc<double>(b_len, nn)) ||
+        (rc = dalloc<double2>(b_com, nn)) || (rc = dalloc<float4>(b_rec, 2 * nn)))
+        return rc;
+    if (mp && ((rc = dalloc<double>(b_m64, nn)) || (rc = dalloc<Quad>(b_quad, nn)) ||
+               (rc = dalloc<float4>(b_mom, nn))))
+        return rc;
+    if (!mp && ((rc = dalloc<float>(b_mass, nn)) || (rc = dalloc<float2>(b_comf, nn)))) return rc;
+    uint32_t* cnt = (uint32_t*)b_cnt.p;
+    PathNodes t{(uint32_t*)b_start.p, (uint32_t*)b_end.p, (uint32_t*)b_skip.p, (uint32_t*)b_parent.p, cnt, cnt + total,
+                (double*)b_len.p, (float*)b_mass.p, (float2*)b_comf.p, (double2*)b_com.p, (double*)b_m64.p,
+                (Quad*)b_quad.p, (float4*)b_rec.p, (float4*)b_mom.p};
+    TC_CUDA_TRY(cudaMemsetAsync(cnt, 0, (size_t)2 * total * 4, s));
+    k_path_nodes<<<grid_for(n, 128), 128, 0, s>>>(keys, (const uint8_t*)b_depth.p, base, n, bbox, t);
+    if (mp)
+        k_path_moments<true><<<grid_for(total, 128), 128, 0, s>>>(total, t, psort, bbox, theta);
+    else
+        k_path_moments<false><<<grid_for(total, 128), 128, 0, s>>>(total, t, psort, bbox, theta);
+    bh_dispatch(kernel, softening, precision, mp, [&](auto ker, auto zero, auto m) {
+        k_path_traverse<decltype(zero), decltype(ker), decltype(m)::value>
+            <<<grid_for(n, kPathThreads, 1 << 20), kPathThreads, 0, s>>>(ker, n, total, t, psort, prel, order, theta,
+                                                                        d_grad_xy, zrow);
+    });
+    TC_CUDA_TRY(cudaGetLastError());
+    return TC_OK;
+}
+
+// The tree of any depth, level by level, and the per-point traversal
+int bh_level_solve(int kernel, double softening, int max_children, double theta, int precision, const double* d_pos_xy,
+                   uint32_t n, double* d_grad_xy, double* zrow, cudaStream_t s, bool mp, const double* bbox,
+                   uint32_t* err, size_t cap)
+{
+    int rc;
     DevBuf b_lo, b_hi, b_start, b_count, b_fc, b_nc, b_mass, b_com, b_comf, b_order, b_order2, b_nodeof, b_nodeof2,
-        b_q, b_ind, b_pre, b_nck, b_coff, b_tmp, b_bbox, b_zrow, b_err;
+        b_q, b_ind, b_pre, b_nck, b_coff, b_tmp;
     if ((rc = dalloc<double2>(b_lo, cap)) || (rc = dalloc<double2>(b_hi, cap)) || (rc = dalloc<uint32_t>(b_start, cap)) ||
         (rc = dalloc<uint32_t>(b_count, cap)) || (rc = dalloc<uint32_t>(b_fc, cap)) ||
         (rc = dalloc<uint32_t>(b_nc, cap)) || (rc = dalloc<float>(b_mass, cap)) || (rc = dalloc<double2>(b_com, cap)) ||
@@ -439,8 +917,7 @@ int bh_solve_impl(int kernel, double softening, int max_children, double theta, 
         (rc = dalloc<uint32_t>(b_nodeof2, n)) || (rc = dalloc<uint8_t>(b_q, n)) ||
         (rc = dalloc<uint32_t>(b_ind, (size_t)4 * n)) || (rc = dalloc<uint32_t>(b_pre, (size_t)4 * (n + 1))) ||
         (rc = dalloc<uint32_t>(b_nck, cap)) || (rc = dalloc<uint32_t>(b_coff, cap + 1)) ||
-        (rc = dalloc<uint32_t>(b_tmp, (size_t)scan_tmp_words((int64_t)cap + n) + 16)) ||
-        (rc = dalloc<double>(b_bbox, 4)) || (rc = dalloc<double>(b_zrow, n)) || (rc = dalloc<uint32_t>(b_err, 4)))
+        (rc = dalloc<uint32_t>(b_tmp, (size_t)scan_tmp_words((int64_t)cap + n) + 16)))
         return rc;
     DevBuf b_m64, b_quad;
     if (mp && ((rc = dalloc<double>(b_m64, cap)) || (rc = dalloc<Quad>(b_quad, cap)))) return rc;
@@ -453,11 +930,9 @@ int bh_solve_impl(int kernel, double softening, int max_children, double theta, 
     uint32_t* node_of2 = (uint32_t*)b_nodeof2.p;
     uint32_t* ind = (uint32_t*)b_ind.p;
     uint32_t* pre = (uint32_t*)b_pre.p;
-    TC_CUDA_TRY(cudaMemsetAsync(b_err.p, 0, 16, s));
-    if ((rc = bbox_keys(d_pos_xy, n64, (double*)b_bbox.p, (uint32_t*)b_err.p, s))) return rc;
     TC_CUDA_TRY(cudaMemsetAsync(node_of, 0, (size_t)n * 4, s));
     k_bh_iota<<<grid_for(n, 256), 256, 0, s>>>(order, n);
-    k_bh_root<<<1, 1, 0, s>>>((const double*)b_bbox.p, n, t);
+    k_bh_root<<<1, 1, 0, s>>>(bbox, n, t);
     std::vector<uint32_t> level_begin = {0}, level_end = {1};
     uint32_t total_nodes = 1;
     const int grid = grid_for(n, 256);
@@ -499,50 +974,83 @@ int bh_solve_impl(int kernel, double softening, int max_children, double theta, 
             k_bh_mass<<<grid_for(level_end[l] - level_begin[l], 128), 128, 0, s>>>(level_begin[l], level_end[l], t,
                                                                                    (const double2*)d_pos_xy, order);
     }
-    const double e2 = softening * softening;
-    const double2* P2 = (const double2*)d_pos_xy;
-    double* zr = (double*)b_zrow.p;
-    uint32_t* er = (uint32_t*)b_err.p;
-    const int gt = grid_for(n, 128);
-    if (precision == TC_PREC_FP64) {
-        if (kernel == TC_KERNEL_GRAVITY) {
-            if (mp)
-                k_bh_traverse<double, KGrav<double>, true>
-                    <<<gt, 128, 0, s>>>(KGrav<double>{e2}, P2, n, t, order, theta, d_grad_xy, zr, er);
-            else
-                k_bh_traverse<double, KGrav<double>, false>
-                    <<<gt, 128, 0, s>>>(KGrav<double>{e2}, P2, n, t, order, theta, d_grad_xy, zr, er);
-        } else {
-            if (mp)
-                k_bh_traverse<double, KTsne<double>, true>
-                    <<<gt, 128, 0, s>>>(KTsne<double>{}, P2, n, t, order, theta, d_grad_xy, zr, er);
-            else
-                k_bh_traverse<double, KTsne<double>, false>
-                    <<<gt, 128, 0, s>>>(KTsne<double>{}, P2, n, t, order, theta, d_grad_xy, zr, er);
-        }
-    } else {
-        if (kernel == TC_KERNEL_GRAVITY) {
-            if (mp)
-                k_bh_traverse<float, KGrav<float>, true>
-                    <<<gt, 128, 0, s>>>(KGrav<float>{(float)e2}, P2, n, t, order, theta, d_grad_xy, zr, er);
-            else
-                k_bh_traverse<float, KGrav<float>, false>
-                    <<<gt, 128, 0, s>>>(KGrav<float>{(float)e2}, P2, n, t, order, theta, d_grad_xy, zr, er);
-        } else {
-            if (mp)
-                k_bh_traverse<float, KTsne<float>, true>
-                    <<<gt, 128, 0, s>>>(KTsne<float>{}, P2, n, t, order, theta, d_grad_xy, zr, er);
-            else
-                k_bh_traverse<float, KTsne<float>, false>
-                    <<<gt, 128, 0, s>>>(KTsne<float>{}, P2, n, t, order, theta, d_grad_xy, zr, er);
-        }
+    const double2* pos = (const double2*)d_pos_xy;
+    bh_dispatch(kernel, softening, precision, mp, [&](auto ker, auto zero, auto m) {
+        k_bh_traverse<decltype(zero), decltype(ker), decltype(m)::value>
+            <<<grid_for(n, 128), 128, 0, s>>>(ker, pos, n, t, order, theta, d_grad_xy, zrow, err);
+    });
+    TC_CUDA_TRY(cudaGetLastError());
+    return TC_OK;
+}
+
+// host: the three arrays are host memory and pass through the workspace, on its stream
+int bh_solve_impl(int kernel, double softening, int max_children, double theta, int precision,
+                  const double* d_pos_xy, int64_t n64, double* d_grad_xy, double* d_total, void* stream, bool mp,
+                  bool host = false)
+{
+    if (!d_pos_xy || !d_grad_xy || n64 <= 0 || n64 > (1 << 30) || max_children <= 0 || !(theta > 0.0) ||
+        (kernel != TC_KERNEL_TSNE && kernel != TC_KERNEL_GRAVITY)) {
+        tc_set_error("tc_bh_solve_device: invalid arguments");
+        return TC_ERR_INVALID;
     }
-    DevBuf b_sum;
-    if ((rc = dalloc<double>(b_sum, sum_tmp_doubles()))) return rc;
-    if (d_total && (rc = sum_f64((const double*)b_zrow.p, n, nullptr, nullptr, d_total, 0, (double*)b_sum.p, s)))
+    const uint32_t n = (uint32_t)n64;
+    cudaStream_t s = (cudaStream_t)stream;
+    int rc = TC_OK;
+    int dev = 0;
+    TC_CUDA_TRY(cudaGetDevice(&dev));
+    BHWork& work = bh_work(dev);
+    std::lock_guard<std::mutex> work_lock(work.mu);
+    if (!work.done) TC_CUDA_TRY(cudaEventCreateWithFlags(&work.done, cudaEventDisableTiming));
+    if (host && !work.stream) TC_CUDA_TRY(cudaStreamCreateWithFlags(&work.stream, cudaStreamNonBlocking));
+    if (host) s = work.stream;
+    // the previous call's kernels (possibly on another stream) finish first
+    if (work.recorded) TC_CUDA_TRY(cudaStreamWaitEvent(s, work.done, 0));
+    WorkRelease release_on_exit{work, s};
+    g_work = &work;
+    g_slot = 0;
+    // node capacity (splits past it are refused, not written)
+    const size_t cap = (size_t)4 * n + 64;
+    DevBuf b_bbox, b_zrow, b_err, b_sum;
+    if ((rc = dalloc<double>(b_bbox, 4)) || (rc = dalloc<double>(b_zrow, n)) || (rc = dalloc<uint32_t>(b_err, 4)) ||
+        (rc = dalloc<double>(b_sum, sum_tmp_doubles())))
+        return rc;
+    const double* bbox = (const double*)b_bbox.p;
+    double* zrow = (double*)b_zrow.p;
+    uint32_t* err = (uint32_t*)b_err.p;
+    double *h_grad = nullptr, *h_total = nullptr;
+    if (host) {
+        DevBuf b_pos, b_grad, b_tot;
+        if ((rc = dalloc<double2>(b_pos, n)) || (rc = dalloc<double2>(b_grad, n)) || (rc = dalloc<double>(b_tot, 1)))
+            return rc;
+        TC_CUDA_TRY(cudaMemcpyAsync(b_pos.p, d_pos_xy, (size_t)n * 16, cudaMemcpyHostToDevice, s));
+        h_grad = d_grad_xy;
+        h_total = d_total;
+        d_pos_xy = (const double*)b_pos.p;
+        d_grad_xy = (double*)b_grad.p;
+        d_total = (double*)b_tot.p;
+    }
+    TC_CUDA_TRY(cudaMemsetAsync(b_err.p, 0, 16, s));
+    if ((rc = bbox_keys(d_pos_xy, n64, (double*)b_bbox.p, (uint32_t*)b_err.p, s))) return rc;
+    const int first_slot = g_slot;
+    rc = max_children <= kPathMaxLeaf ? bh_path_solve(kernel, softening, max_children, theta, precision,
+                                                      (const double2*)d_pos_xy, n, d_grad_xy, zrow, s, mp, bbox, err, cap)
+                                      : 1;
+    if (rc == 1) {
+        g_slot = first_slot;  // the same scratch, laid out anew (its kernels are done)
+        rc = bh_level_solve(kernel, softening, max_children, theta, precision, d_pos_xy, n, d_grad_xy, zrow, s, mp, bbox,
+                            err, cap);
+    }
+    if (rc) return rc;
+    if (d_total && (rc = sum_f64(zrow, n, nullptr, nullptr, d_total, 0, (double*)b_sum.p, s)))
         return rc;
     uint32_t herr = 0;
     TC_CUDA_TRY(cudaMemcpyAsync(&herr, b_err.p, 4, cudaMemcpyDeviceToHost, s));
+    if (h_grad) {
+        // written only by a solve that succeeded
+        TC_CUDA_TRY(cudaStreamSynchronize(s));
+        if (!herr) TC_CUDA_TRY(cudaMemcpyAsync(h_grad, d_grad_xy, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
+        if (!herr && h_total) TC_CUDA_TRY(cudaMemcpyAsync(h_total, d_total, 8, cudaMemcpyDeviceToHost, s));
+    }
     TC_CUDA_TRY(cudaStreamSynchronize(s));
     if (herr) {
         tc_set_error("tc_bh_solve_device: traversal stack exhausted");
@@ -570,11 +1078,6 @@ extern "C" int tc_bhmp_solve_device(int kernel, double softening, int max_childr
                          true);
 }
 
-struct OwnBuf {
-    void* p = nullptr;
-    ~OwnBuf() { if (p) cudaFree(p); }
-};
-
 static int bh_solve_host(int kernel, double softening, int max_children, double theta, int precision,
                          const double* pos_xy, int64_t n, double* grad_xy, double* total, bool mp)
 {
@@ -582,26 +1085,8 @@ static int bh_solve_host(int kernel, double softening, int max_children, double 
         tc_set_error("tc_bh_solve: invalid arguments");
         return TC_ERR_INVALID;
     }
-    cudaStream_t s;
-    TC_CUDA_TRY(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    OwnBuf dp, dg, dt;
-    int rc = TC_OK;
-    cudaError_t e = cudaMalloc(&dp.p, (size_t)n * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dg.p, (size_t)n * 16);
-    if (e == cudaSuccess) e = cudaMalloc(&dt.p, 8);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dp.p, pos_xy, (size_t)n * 16, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) {
-        rc = tc::bh_solve_impl(kernel, softening, max_children, theta, precision, (const double*)dp.p, n,
-                               (double*)dg.p, (double*)dt.p, s, mp);
-        if (rc == TC_OK) e = cudaMemcpyAsync(grad_xy, dg.p, (size_t)n * 16, cudaMemcpyDeviceToHost, s);
-        if (rc == TC_OK && e == cudaSuccess && total) e = cudaMemcpyAsync(total, dt.p, 8, cudaMemcpyDeviceToHost, s);
-    }
-    cudaError_t e2 = cudaStreamSynchronize(s);
-    cudaStreamDestroy(s);
-    if (rc) return rc;
-    if (e != cudaSuccess) return tc_cuda_fail(e, "tc_bh_solve");
-    if (e2 != cudaSuccess) return tc_cuda_fail(e2, "tc_bh_solve sync");
-    return TC_OK;
+    return tc::bh_solve_impl(kernel, softening, max_children, theta, precision, pos_xy, n, grad_xy, total, nullptr, mp,
+                             true);
 }
 
 extern "C" int tc_bh_solve(int kernel, double softening, int max_children, double theta, int precision,
