@@ -24,9 +24,18 @@
 // This file is compiled without FMA contraction: the fused operations above
 // are the explicit fma / fmaf calls.
 #include "common.cuh"
+#include "knn_gram.cuh"
 
 namespace tc {
 namespace {
+
+// sizes the tensor-core filter takes (tc_knn_device) and its scratch for a_ij
+#ifndef TC_KNN_GRAM_MIN_N
+#define TC_KNN_GRAM_MIN_N 1024
+#endif
+constexpr int64_t kGramMinN = TC_KNN_GRAM_MIN_N;
+constexpr int kGramMinDim = 1, kGramMaxDim = 4096;
+constexpr int64_t kGramBytes = 256ll << 20;
 
 // ------------------------------------------------------------------ exp, log
 constexpr double kLn2Hi = 0x1.62e42fee00000p-1;   // ln 2 to 32 significant bits
@@ -120,8 +129,9 @@ __device__ inline double aff_log(double x)
 //   a third of the SMs idle in the second wave.
 // A list entry is the 64-bit key (distance bits, index): distances are never
 // negative, so integer order is (distance, index) order, and NaNs sort last.
-// 20,000 x 784, k = 90: 70.0 ms before (4 x 4 blocks of scalar operations, a
-// block per 64 queries), 22.8 ms now.  8 x 8 blocks need fewer shared loads
+// 20,000 x 784, k = 90, all query blocks: 70.0 ms before (4 x 4 blocks of
+// scalar operations, a block per 64 queries), 22.8 ms now.  Inputs that the
+// tensor-core filter takes (knn_gram.cuh) come here only where it gave up.  8 x 8 blocks need fewer shared loads
 // but leave 8 or 12 warps an SM instead of 16: 23.9 and 25.4 ms.
 constexpr int kQ = 64;        // query rows per block
 constexpr int kC = 128;       // candidates per tile
@@ -165,6 +175,21 @@ __host__ __device__ inline int64_t knn_owner(int64_t u, int64_t units, int64_t r
     return ((u + 1) * runs - 1) / units;
 }
 
+// The units of the listed query blocks (all of them without a list) and the
+// runs they are dealt to.  With a list the runs are at most kListRuns a query
+// block, which bounds the partial lists that a row's merge holds.
+constexpr int kListRuns = 14;
+struct KnnRuns {
+    int64_t units, runs;
+    __host__ __device__ KnnRuns(int64_t qblocks, int64_t ctiles, int64_t max_runs, const uint32_t* nlist)
+    {
+        const int64_t q = nlist ? (int64_t)*nlist : qblocks;
+        units = q * ctiles;
+        runs = units < max_runs ? units : max_runs;
+        if (nlist && runs > kListRuns * q) runs = kListRuns * q;
+    }
+};
+
 // one key into a row's sorted list (k keys, unused ones all-ones), by a warp
 __device__ __forceinline__ void knn_insert(u64* __restrict__ list, int k, u64 key, int lane)
 {
@@ -188,7 +213,8 @@ __device__ __forceinline__ void knn_insert(u64* __restrict__ list, int k, u64 ke
 
 template <bool kVec>
 __global__ void __launch_bounds__(kKnnT, 2)
-    k_knn(const float* __restrict__ x, int64_t n, int dim, int k, int64_t ctiles, int64_t units, u64* __restrict__ part)
+    k_knn(const float* __restrict__ x, int64_t n, int dim, int k, int64_t ctiles, int64_t qblocks,
+          const uint32_t* __restrict__ list, const uint32_t* __restrict__ nlist, u64* __restrict__ part)
 {
     extern __shared__ __align__(16) uint8_t dyn[];
     float* stage = reinterpret_cast<float*>(dyn);          // [2][kKC][kQ + kC]
@@ -198,7 +224,10 @@ __global__ void __launch_bounds__(kKnnT, 2)
     const int ty = tid >> 4, tx = tid & 15;  // queries 4 ty + a; candidates 4 tx + b and 64 + 4 tx + b
     constexpr int kRows = kQ + kC;
     constexpr int kLoads = kRows * (kKC / 4) / kKnnT;  // 16-byte pieces a thread fetches per chunk
-    const int64_t runs = gridDim.x, run = blockIdx.x;
+    const KnnRuns kr(qblocks, ctiles, gridDim.x, nlist);
+    const int64_t units = kr.units, runs = kr.runs, run = blockIdx.x;
+    if (run >= runs) return;
+    auto qblock = [&](int64_t o) { return list ? (int64_t)list[o] : o; };
     const int64_t u0 = run * units / runs, u1 = (run + 1) * units / runs;
     const int chunks = (dim + kKC - 1) / kKC;
     float4 pre[kLoads];
@@ -234,9 +263,9 @@ __global__ void __launch_bounds__(kKnnT, 2)
             s[(t + 3) * kRows + r] = pre[j].w;
         }
     };
-    if (u0 < u1) fetch(u0 / ctiles * kQ, u0 % ctiles * kC, 0);
+    if (u0 < u1) fetch(qblock(u0 / ctiles) * kQ, u0 % ctiles * kC, 0);
     for (int64_t u = u0; u < u1; u++) {
-        const int64_t qb = u / ctiles, q0 = qb * kQ, c0 = u % ctiles * kC;
+        const int64_t o = u / ctiles, q0 = qblock(o) * kQ, c0 = u % ctiles * kC;
         if (u == u0 || u % ctiles == 0)
             for (int e = tid; e < kQ * k; e += kKnnT) lists[e] = ~0ull;
         u64 acc[4][4];
@@ -251,7 +280,7 @@ __global__ void __launch_bounds__(kKnnT, 2)
             if (c + 1 < chunks)
                 fetch(q0, c0, (c + 1) * kKC);
             else if (u + 1 < u1)
-                fetch((u + 1) / ctiles * kQ, (u + 1) % ctiles * kC, 0);
+                fetch(qblock((u + 1) / ctiles) * kQ, (u + 1) % ctiles * kC, 0);
 #pragma unroll
             for (int t = 0; t < kKC; t++) {
                 const float4 q = *reinterpret_cast<const float4*>(s + t * kRows + 4 * ty);
@@ -299,8 +328,8 @@ __global__ void __launch_bounds__(kKnnT, 2)
         }
         __syncthreads();
         if (u + 1 == u1 || (u + 1) % ctiles == 0) {
-            // runs and query blocks both grow along the units: run + query block numbers the partial lists
-            u64* dst = part + (run + qb) * (int64_t)(kQ * k);
+            // runs and query blocks both grow along the units: their sum numbers the partial lists
+            u64* dst = part + (run + o) * (int64_t)(kQ * k);
             for (int e = tid; e < kQ * k; e += kKnnT) dst[e] = lists[e];
             __syncthreads();
         }
@@ -312,19 +341,23 @@ __global__ void __launch_bounds__(kKnnT, 2)
 // other list, the number of that list's smaller entries.
 constexpr int kMergeWarps = 4;
 __global__ void __launch_bounds__(32 * kMergeWarps)
-    k_knn_merge(const u64* __restrict__ part, int64_t n, int k, int64_t ctiles, int64_t units, int64_t runs,
-                int maxseg, float* __restrict__ out_d, int32_t* __restrict__ out_i)
+    k_knn_merge(const u64* __restrict__ part, int64_t n, int k, int64_t ctiles, int64_t qblocks, int64_t max_runs,
+                const uint32_t* __restrict__ list, const uint32_t* __restrict__ nlist, int maxseg,
+                float* __restrict__ out_d, int32_t* __restrict__ out_i)
 {
     extern __shared__ __align__(16) uint8_t dyn[];
     const int lane = threadIdx.x & 31;
     u64* sl = reinterpret_cast<u64*>(dyn) + (size_t)(threadIdx.x >> 5) * maxseg * k;
-    const int64_t row = blockIdx.x * (int64_t)kMergeWarps + (threadIdx.x >> 5);
+    const KnnRuns kr(qblocks, ctiles, max_runs, nlist);
+    const int64_t units = kr.units, runs = kr.runs;
+    const int64_t at = blockIdx.x * (int64_t)kMergeWarps + (threadIdx.x >> 5), o = at / kQ;
+    if (o * ctiles >= units) return;
+    const int64_t row = (list ? (int64_t)list[o] : o) * kQ + at % kQ;
     if (row >= n) return;
-    const int64_t qb = row / kQ;
-    const int64_t b0 = knn_owner(qb * ctiles, units, runs), b1 = knn_owner((qb + 1) * ctiles - 1, units, runs);
+    const int64_t b0 = knn_owner(o * ctiles, units, runs), b1 = knn_owner((o + 1) * ctiles - 1, units, runs);
     const int nseg = (int)(b1 - b0 + 1) < maxseg ? (int)(b1 - b0 + 1) : maxseg;
     for (int sg = 0; sg < nseg; sg++) {
-        const u64* src = part + (b0 + sg + qb) * (int64_t)(kQ * k) + (row % kQ) * k;
+        const u64* src = part + (b0 + sg + o) * (int64_t)(kQ * k) + (row % kQ) * k;
         for (int e = lane; e < k; e += 32) sl[sg * k + e] = src[e];
     }
     __syncwarp();
@@ -333,12 +366,12 @@ __global__ void __launch_bounds__(32 * kMergeWarps)
         if (key == ~0ull) continue;
         const int sg = e / k;
         int place = e - sg * k;
-        for (int o = 0; o < nseg && place < k; o++) {
-            if (o == sg) continue;
-            int lo = 0, hi = k;  // the first entry of list o not below key
+        for (int l = 0; l < nseg && place < k; l++) {
+            if (l == sg) continue;
+            int lo = 0, hi = k;  // the first entry of list l not below key
             while (lo < hi) {
                 const int mid = (lo + hi) >> 1;
-                if (sl[o * k + mid] < key) lo = mid + 1;
+                if (sl[l * k + mid] < key) lo = mid + 1;
                 else hi = mid;
             }
             place += lo;
@@ -351,81 +384,188 @@ __global__ void __launch_bounds__(32 * kMergeWarps)
 }
 
 // ------------------------------------------------------------------ bandwidths
-// The entropy of one row in FP32.  It decides a bisection step wherever it is
-// farther from the target than its error: with all w <= 1 and one w = 1, and
-// <x> <= H <= ln k for x = beta d', the roundings of x (5 2^-24 x), of the
-// exponential (2^-22), of the k-term sums and of the logarithm move H by less
-// than (11 <x^2> + (2 ln k + 1) (k + 10)) 2^-24 < 1.6e-4 at k = 128, where
-// <x^2> <= 0.55 k.
+// FP64 issues at 1/64 of the FP32 rate and an evaluation of a row's entropy H
+// takes 24 FP64 operations a neighbour, so a bisection step is decided by the
+// cheapest evaluation that is certain to decide as the FP64 one does:
+// * FP32.  With all w <= 1, one w = 1 and <x> <= H <= ln k for x = beta d', the
+//   roundings of x (5 2^-24 x), of the exponential (2^-22), of the k-term sums
+//   and of the logarithm move H by less than
+//   (11 <x^2> + (2 ln k + 1) (k + 10)) 2^-24 < 1.6e-4 at k = 128 (<x^2> <= 0.55 k).
+// * FP32 with x to FP64 accuracy, an exponential good to 2.5e-7 and compensated
+//   sums.  Relative errors delta of the w move H by at most delta (1 + sd(x)),
+//   sd(x) <= 3.5 at k = 128: 1.4e-6 with the products' roundings; the logarithm
+//   (an ulp), the quotient and the sums of the last line 1.6e-6.
+// * FP64, as the definition says, where neither decides.
+// The steps are the same, to the bit.
 constexpr int kScreenK = 128;
-constexpr float kScreenErr = 2.0e-4f;
+constexpr float kScreenErr = 2.0e-4f, kScreenErr2 = 3.5e-6f;
 
-__device__ inline float entropy_f32(const float* __restrict__ d, int k, float beta)
+// exp(-x) of x = p + e >= 0, |e| tiny, to 2.5e-7: reduction by ln 2 in two parts, the exponential series to r^7
+__device__ __forceinline__ float screen_exp(float p, float e)
 {
-    const float dmin = d[0];
-    float s = 0.f, sd = 0.f;
-#pragma unroll 4
-    for (int j = 0; j < k; j++) {
-        const float dj = d[j] - dmin;
-        const float w = __expf(-dj * beta);
-        s += w;
-        sd = fmaf(dj, w, sd);
-    }
-    return __logf(s) + beta * sd / s;
+    const float t = rintf(fminf(p, 150.0f) * 1.44269504f);  // beyond 150 the result is zero
+    float r = fmaf(t, -0x1.62e4p-1f, p);                    // ln 2 to 15 bits: t times it is exact
+    r = fmaf(t, -0x1.7f7d1cp-20f, r) + e;
+    float q = -1.0f / 5040.0f;
+    q = fmaf(q, r, 1.0f / 720.0f);
+    q = fmaf(q, r, -1.0f / 120.0f);
+    q = fmaf(q, r, 1.0f / 24.0f);
+    q = fmaf(q, r, -1.0f / 6.0f);
+    q = fmaf(q, r, 0.5f);
+    q = fmaf(q, r, -1.0f);
+    q = fmaf(q, r, 1.0f);
+    // 2^-t in two factors (t up to 217)
+    const int ti = (int)t, h = ti >> 1;
+    return p > 150.0f ? 0.0f : q * __int_as_float((127 - h) << 23) * __int_as_float((127 - (ti - h)) << 23);
 }
 
-// A thread per row (the sums' order is part of the result).  FP64 issues at
-// 1/64 of the FP32 rate and an evaluation takes 24 FP64 operations a
-// neighbour, so only the steps that FP32 cannot decide, the last five or six of
-// some 22, are evaluated in FP64: the same steps, to the bit.  20,000 rows of
-// 90: 4.24 ms with every step in FP64, 2.0 ms now.  Small blocks spread few
-// rows over the SMs.
+// a / s by its correctly rounded reciprocal y: the quotient's remainder is exact in a fused operation and the
+// correction rounds as the division does (P. Markstein, 1990); far from the subnormal range only
+__device__ __forceinline__ double quotient(double a, double s, double y)
+{
+    if (!(a > 1e-280 && s < 1e280)) return a / s;
+    const double q = a * y;
+    return fma(fma(-q, s, a), y, q);
+}
+
+// kPerpLanes lanes share a row: they take its neighbours in turn, and for an
+// FP64 evaluation two of them then run the sums of w and of d' w, each a chain
+// in the order that defines the rows, over the staged terms.  20,000 rows of
+// 90: 4.24 ms with a thread per row and every step in FP64, 2.0 ms with the
+// first screen, 1.4 ms with the row's lanes (at 85 % of the FP64 pipe), 0.63 ms
+// with the second screen.
+constexpr int kPerpLanes = 8;
 constexpr int kPerpThreads = 64;
+constexpr int kPerpChunk = 64;  // neighbours staged at a time
 
 __global__ void __launch_bounds__(kPerpThreads)
     k_perplexity(const float* __restrict__ dist, int64_t n, int k, double perplexity, int max_iter, double tol,
                  double* __restrict__ p)
 {
+    constexpr int kRows = kPerpThreads / kPerpLanes;
+    // (w, d') of a row's chunk; the odd row length spreads the rows over the banks
+    __shared__ double2 s_term[kRows][kPerpChunk + 1];
+    const int sub = threadIdx.x % kPerpLanes, group = threadIdx.x / kPerpLanes;
+    double2* term = s_term[group];
     const double log_perp = aff_log(perplexity);
     const float screen = (float)tol + kScreenErr;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    // a warp's rows go through the loops together, finished ones idling
+    for (int64_t i0 = blockIdx.x * (int64_t)kRows; i0 < n; i0 += (int64_t)gridDim.x * kRows) {
+        const bool valid = i0 + group < n;
+        const int64_t i = valid ? i0 + group : n - 1;
         const float* d = dist + i * k;
-        const double dmin = (double)d[0];
-        double beta = 1.0, lo = 0.0, hi = INFINITY;
-        for (int it = 0; it < max_iter; it++) {
-            double diff;
-            const float quick = k <= kScreenK ? entropy_f32(d, k, (float)beta) - (float)log_perp : 0.f;
-            if (fabsf(quick) > screen) {  // false for NaN
-                diff = (double)quick;
-            } else {
-                double s = 0.0, sd = 0.0;
-#pragma unroll 4
-                for (int j = 0; j < k; j++) {
-                    const double dj = (double)d[j] - dmin;
+        const float dmin = d[0];
+        // sum of w_j = exp(-beta d'_j) in lane 0, of d'_j w_j in lane 1; out: the w_j are kept in the row of p
+        auto sums = [&](double beta, bool on, double* out) {
+            double chain = 0.0;
+            for (int j0 = 0; j0 < k; j0 += kPerpChunk) {
+                const int m = on ? min(k - j0, kPerpChunk) : 0;
+#pragma unroll 2
+                for (int j = sub; j < m; j += kPerpLanes) {
+                    const double dj = (double)d[j0 + j] - (double)dmin;
                     const double w = aff_exp(-dj * beta);
-                    s += w;
-                    sd = fma(dj, w, sd);
+                    term[j] = make_double2(w, dj);
+                    if (out) out[j0 + j] = w;
                 }
-                const double h = aff_log(s) + beta * sd / s;
-                diff = h - log_perp;
-                if (fabs(diff) < tol) break;
+                __syncwarp();
+                if (sub < 2) {
+#pragma unroll 8
+                    for (int j = 0; j < m; j++) {
+                        const double2 t = term[j];
+                        chain = fma(sub == 0 ? 1.0 : t.y, t.x, chain);  // fma(1, w, s) rounds as s + w
+                    }
+                }
+                __syncwarp();
             }
-            if (diff > 0.0) {
-                lo = beta;
-                beta = isinf(hi) ? beta * 2.0 : (lo + hi) * 0.5;
-            } else {
-                hi = beta;
-                beta = (lo + hi) * 0.5;
+            return chain;
+        };
+        // the screens' error bounds are for rows whose first entry is the smallest, as kNN rows are
+        bool ordered = k <= kScreenK;
+        for (int j = sub; j < k; j += kPerpLanes) ordered = ordered && d[j] >= dmin;
+        const uint32_t groups = __ballot_sync(0xffffffffu, ordered);
+        const uint32_t own = ((1u << kPerpLanes) - 1u) << (threadIdx.x % 32 / kPerpLanes * kPerpLanes);
+        const bool screened = (groups & own) == own;
+        double beta = 1.0, lo = 0.0, hi = INFINITY;
+        bool active = valid;
+        for (int it = 0; it < max_iter && __any_sync(0xffffffffu, active); it++) {
+            double diff = 0.0;
+            bool exact = active;
+            if (k <= kScreenK) {
+                const float b = (float)beta;
+                float s = 0.f, sd = 0.f;
+                for (int j = sub; j < k; j += kPerpLanes) {
+                    const float dj = d[j] - dmin;
+                    const float w = __expf(-dj * b);
+                    s += w;
+                    sd = fmaf(dj, w, sd);
+                }
+#pragma unroll
+                for (int o = 1; o < kPerpLanes; o <<= 1) {
+                    s += __shfl_xor_sync(0xffffffffu, s, o);
+                    sd += __shfl_xor_sync(0xffffffffu, sd, o);
+                }
+                const float quick = __logf(s) + b * sd / s - (float)log_perp;
+                if (screened && fabsf(quick) > screen) {  // false for NaN
+                    exact = false;
+                    diff = (double)quick;
+                }
+            }
+            if (k <= kScreenK && __any_sync(0xffffffffu, exact)) {
+                const float b = (float)beta, bl = (float)(beta - (double)b);
+                float s = 0.f, sd = 0.f, cs = 0.f, cd = 0.f;  // sums and their compensations
+                for (int j = sub; j < k; j += kPerpLanes) {
+                    const float dj = d[j] - dmin, dl = (d[j] - dj) - dmin;  // d' exactly, as a sum (T. Dekker)
+                    const float p0 = dj * b;
+                    const float w = screen_exp(p0, fmaf(dj, b, -p0) + fmaf(dj, bl, dl * b));
+                    const float y = w - cs, t = s + y;
+                    cs = (t - s) - y;
+                    s = t;
+                    const float yd = dj * w - cd, td = sd + yd;
+                    cd = (td - sd) - yd;
+                    sd = td;
+                }
+                double s64 = (double)s - (double)cs, d64 = (double)sd - (double)cd;
+#pragma unroll
+                for (int o = 1; o < kPerpLanes; o <<= 1) {
+                    s64 += __shfl_xor_sync(0xffffffffu, s64, o);
+                    d64 += __shfl_xor_sync(0xffffffffu, d64, o);
+                }
+                const float sf = (float)s64;
+                const float close = logf(sf) + b * ((float)d64 / sf) - (float)log_perp;
+                // beta and the sums in the normal range, where the error bounds hold
+                if (exact && screened && b > 1e-30f && b < 1e30f && d64 * beta > 1e-3) {
+                    if (fabsf(close) > (float)tol + kScreenErr2) {
+                        exact = false;
+                        diff = (double)close;
+                    } else if (fabsf(close) + kScreenErr2 < (float)tol) {
+                        exact = active = false;
+                    }
+                }
+            }
+            if (__any_sync(0xffffffffu, exact)) {
+                const double chain = sums(beta, exact, nullptr);
+                const double s = __shfl_sync(0xffffffffu, chain, 0, kPerpLanes);
+                const double sd = __shfl_sync(0xffffffffu, chain, 1, kPerpLanes);
+                if (exact) {
+                    const double h = aff_log(s) + beta * sd / s;
+                    diff = h - log_perp;
+                    if (fabs(diff) < tol) active = false;
+                }
+            }
+            if (active) {
+                if (diff > 0.0) {
+                    lo = beta;
+                    beta = isinf(hi) ? beta * 2.0 : (lo + hi) * 0.5;
+                } else {
+                    hi = beta;
+                    beta = (lo + hi) * 0.5;
+                }
             }
         }
-        double s = 0.0;
-#pragma unroll 4
-        for (int j = 0; j < k; j++) {
-            const double w = aff_exp(-((double)d[j] - dmin) * beta);
-            s += w;
-            p[i * k + j] = w;
-        }
-        for (int j = 0; j < k; j++) p[i * k + j] = p[i * k + j] / s;
+        double* row = p + i * k;
+        const double s = __shfl_sync(0xffffffffu, sums(beta, valid, row), 0, kPerpLanes);
+        const double y = 1.0 / s;
+        for (int j = sub; valid && j < k; j += kPerpLanes) row[j] = quotient(row[j], s, y);
     }
 }
 
@@ -503,23 +643,75 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
         return TC_ERR_INVALID;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    const int64_t qblocks = (n + kQ - 1) / kQ, ctiles = (n + kC - 1) / kC, units = qblocks * ctiles;
+    const int64_t qblocks = (n + kQ - 1) / kQ, ctiles = (n + kC - 1) / kC;
     // two resident blocks per SM (registers and shared memory), each one run of units
-    const int64_t runs = units < 2 * (int64_t)sm_count() ? units : 2 * (int64_t)sm_count();
-    // runs that share a query block: each holds at least units / runs of its ctiles units
-    const int64_t maxseg = runs / qblocks + 2 < ctiles ? runs / qblocks + 2 : ctiles;
-    const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
+    const int64_t max_runs = 2 * (int64_t)sm_count();
+    const int64_t runs = KnnRuns(qblocks, ctiles, max_runs, nullptr).runs;
     // 16-byte loads: every row starts on a 16-byte boundary
     const bool vec = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0;
+    // the filter on the tensor cores wherever its bound holds: 256 groups of four columns need 1,024 points, its row
+    // of inputs 16 KB of shared memory.  It is the faster one over all of that range, k = 90, against k_knn alone:
+    // 1,024 x 4: 91 us, 295; 2,000 x 32: 111, 573; 20,000 x 128: 1.28 ms, 6.70; 20,000 x 784: 3.0, 23.2 (4.6 when
+    // the inputs have low parts); 70,000 x 784: 22.2, 254.9
+    const bool gram = n >= kGramMinN && dim >= kGramMinDim && dim <= kGramMaxDim;
+    // runs that share a query block: each holds at least units / runs of its ctiles units
+    int64_t maxseg = gram ? kListRuns + 2 : runs / qblocks + 2;
+    if (maxseg > ctiles) maxseg = ctiles;
+    const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
     auto kernel = vec ? k_knn<true> : k_knn<false>;
     TC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
     TC_CUDA_TRY(cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mdyn));
-    void* part = nullptr;
-    TC_CUDA_TRY(cudaMallocAsync(&part, (size_t)(runs + qblocks) * kQ * k * 8, s));
-    kernel<<<(unsigned)runs, kKnnT, dyn, s>>>(d_x, n, dim, k, ctiles, units, static_cast<u64*>(part));
-    k_knn_merge<<<(unsigned)((n + kMergeWarps - 1) / kMergeWarps), 32 * kMergeWarps, mdyn, s>>>(
-        static_cast<const u64*>(part), n, k, ctiles, units, runs, (int)maxseg, d_dist, d_idx);
-    const cudaError_t e = cudaGetLastError(), ef = cudaFreeAsync(part, s);
+    auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+    // scratch: partial lists; for the filter the split inputs, norms, status, flags and list of query blocks, and
+    // a_ij of as many query rows as kGramBytes holds (at least one tile of rows)
+    const int dimp = (dim + 15) & ~15;
+    const int64_t npad = (n + kGramCols - 1) / kGramCols * kGramCols, rblocks = (n + kGramRows - 1) / kGramRows;
+    int64_t rb_chunk = kGramBytes / (npad * 4 * kGramRows);
+    rb_chunk = rb_chunk < 1 ? 1 : rb_chunk > rblocks ? rblocks : rb_chunk;
+    const size_t b_part = up((size_t)(runs + qblocks) * kQ * k * 8), b_half = up((size_t)npad * dimp * 2),
+                 b_norm = up((size_t)npad * 4), b_flag = up(sizeof(GramStat) + (size_t)qblocks * 4),
+                 b_list = up((size_t)qblocks * 4), b_gram = up((size_t)rb_chunk * kGramRows * npad * 4),
+                 b_gmin = b_gram / 4;
+    uint8_t* buf = nullptr;
+    TC_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&buf),
+                                b_part + (gram ? 2 * b_half + b_norm + b_flag + b_list + b_gram + b_gmin : 0), s));
+    u64* part = reinterpret_cast<u64*>(buf);
+    uint32_t *list = nullptr, *nlist = nullptr;
+    cudaError_t e = cudaSuccess;
+    if (gram) {
+        uint8_t *hi = buf + b_part, *lo = hi + b_half;
+        float* norm = reinterpret_cast<float*>(lo + b_half);
+        GramStat* st = reinterpret_cast<GramStat*>(reinterpret_cast<uint8_t*>(norm) + b_norm);
+        uint32_t* qflag = reinterpret_cast<uint32_t*>(st + 1);
+        list = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(st) + b_flag);
+        nlist = &st->nflagged;
+        float* a = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(list) + b_list);
+        float* gmin = a + b_gram / 4;
+        const size_t sdyn = (size_t)((dim + 31) & ~31) * 4;
+        auto select = vec ? k_knn_select<true> : k_knn_select<false>;
+        e = cudaFuncSetAttribute(k_gram, cudaFuncAttributeMaxDynamicSharedMemorySize, kGramSmem);
+        if (e == cudaSuccess) e = cudaMemsetAsync(st, 0, b_flag, s);
+        if (e == cudaSuccess) {
+            k_gram_split<<<(unsigned)(npad / 8), 256, 0, s>>>(d_x, n, dim, dimp, hi, lo, norm, st);
+            for (int64_t rb = 0; rb < rblocks; rb += rb_chunk) {
+                const int64_t nrb = rblocks - rb < rb_chunk ? rblocks - rb : rb_chunk;
+                const int64_t tiles = nrb * (npad / kGramCols), row0 = rb * kGramRows;
+                const int64_t rows = n - row0 < nrb * kGramRows ? n - row0 : nrb * kGramRows;
+                k_gram<<<(unsigned)(tiles < sm_count() ? tiles : sm_count()), kGramThreads, kGramSmem, s>>>(
+                    hi, lo, norm, n, npad, dimp, rb, (int)nrb, a, gmin, st);
+                select<<<(unsigned)rows, kSelT, sdyn, s>>>(d_x, n, dim, dimp, k, a, gmin, npad, nrb, row0, norm, st, d_dist,
+                                                          d_idx, qflag, kQ);
+            }
+            k_knn_flagged<<<1, 1024, 0, s>>>(qflag, qblocks, st, list);
+        }
+    }
+    if (e == cudaSuccess) {
+        kernel<<<(unsigned)runs, kKnnT, dyn, s>>>(d_x, n, dim, k, ctiles, qblocks, list, nlist, part);
+        k_knn_merge<<<(unsigned)(qblocks * (kQ / kMergeWarps)), 32 * kMergeWarps, mdyn, s>>>(
+            part, n, k, ctiles, qblocks, runs, list, nlist, (int)maxseg, d_dist, d_idx);
+        e = cudaGetLastError();
+    }
+    const cudaError_t ef = cudaFreeAsync(buf, s);
     if (e != cudaSuccess) return tc_cuda_fail(e, "tc_knn_device");
     TC_CUDA_TRY(ef);
     return TC_OK;
@@ -532,7 +724,7 @@ extern "C" int tc_perplexity_device(const float* d_dist, int64_t n, int k, doubl
         tc_set_error("tc_perplexity_device: invalid arguments (perplexity must exceed 1)");
         return TC_ERR_INVALID;
     }
-    k_perplexity<<<grid_for(n, kPerpThreads), kPerpThreads, 0, (cudaStream_t)stream>>>(d_dist, n, k, perplexity, max_iter, tol, d_p);
+    k_perplexity<<<grid_for(n * kPerpLanes, kPerpThreads), kPerpThreads, 0, (cudaStream_t)stream>>>(d_dist, n, k, perplexity, max_iter, tol, d_p);
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
 }

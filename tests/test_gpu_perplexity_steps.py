@@ -1,7 +1,7 @@
 """k_perplexity, whose bisection steps FP32 decides where it can, against the oracle's all-FP64 rows, bit for bit.
 
 Short rows, the longest rows of the FP32 screen and longer ones, perplexities that no bandwidth reaches, equal
-distances, and distances near both ends of the FP32 range.
+distances, distances near both ends of the FP32 range, and rows that do not start with their smallest.
 """
 import numpy as np
 import pytest
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("k", [1, 2, 31, 90, 128, 129, 300])
-@pytest.mark.parametrize("scale", [1.0, 1e-30, 1e-42, 1e30, "equal", "wide"])
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 1e-42, 1e30, "equal", "wide", "unordered"])
 @pytest.mark.parametrize("perplexity", [1.5, 30.0])
 def test_rows_match_the_oracle(k, scale, perplexity):
     import torch
@@ -23,6 +23,8 @@ def test_rows_match_the_oracle(k, scale, perplexity):
         d[:] = d[:, :1]
     elif scale == "wide":
         d = np.sort(10.0 ** rng.uniform(-35, 35, (193, k)), axis=1)
+    elif scale == "unordered":
+        d = d[:, ::-1].copy()
     else:
         d *= scale
     d = d.astype(np.float32)
