@@ -653,14 +653,8 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
     // of inputs 16 KB of shared memory.  It is the faster one over all of that range, k = 90, against k_knn alone:
     // 1,024 x 4: 91 us, 295; 2,000 x 32: 111, 573; 20,000 x 128: 1.28 ms, 6.70; 20,000 x 784: 3.0, 23.2 (4.6 when
     // the inputs have low parts); 70,000 x 784: 22.2, 254.9
-    const bool gram = n >= kGramMinN && dim >= kGramMinDim && dim <= kGramMaxDim;
-    // runs that share a query block: each holds at least units / runs of its ctiles units
-    int64_t maxseg = gram ? kListRuns + 2 : runs / qblocks + 2;
-    if (maxseg > ctiles) maxseg = ctiles;
-    const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
+    bool gram = n >= kGramMinN && dim >= kGramMinDim && dim <= kGramMaxDim;
     auto kernel = vec ? k_knn<true> : k_knn<false>;
-    TC_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-    TC_CUDA_TRY(cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mdyn));
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     // scratch: partial lists; for the filter the split inputs, norms, status, flags and list of query blocks, and
     // a_ij of as many query rows as kGramBytes holds (at least one tile of rows)
@@ -672,13 +666,24 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
                  b_norm = up((size_t)npad * 4), b_flag = up(sizeof(GramStat) + (size_t)qblocks * 4),
                  b_list = up((size_t)qblocks * 4), b_gram = up((size_t)rb_chunk * kGramRows * npad * 4),
                  b_gmin = b_gram / 4;
-    uint8_t* buf = nullptr;
-    TC_CUDA_TRY(cudaMallocAsync(reinterpret_cast<void**>(&buf),
-                                b_part + (gram ? 2 * b_half + b_norm + b_flag + b_list + b_gram + b_gmin : 0), s));
+    void* buf_p = nullptr;
+    if (gram && cudaMallocAsync(&buf_p, b_part + 2 * b_half + b_norm + b_flag + b_list + b_gram + b_gmin, s) !=
+                    cudaSuccess) {
+        cudaGetLastError();  // no room for the filter's scratch: every query block by k_knn
+        gram = false;
+    }
+    if (!gram) TC_CUDA_TRY(cudaMallocAsync(&buf_p, b_part, s));
+    uint8_t* buf = static_cast<uint8_t*>(buf_p);
+    // runs that share a query block: each holds at least units / runs of its ctiles units
+    int64_t maxseg = gram ? kListRuns + 2 : runs / qblocks + 2;
+    if (maxseg > ctiles) maxseg = ctiles;
+    const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
     u64* part = reinterpret_cast<u64*>(buf);
     uint32_t *list = nullptr, *nlist = nullptr;
-    cudaError_t e = cudaSuccess;
-    if (gram) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mdyn);
+    if (gram && e == cudaSuccess) {
         uint8_t *hi = buf + b_part, *lo = hi + b_half;
         float* norm = reinterpret_cast<float*>(lo + b_half);
         GramStat* st = reinterpret_cast<GramStat*>(reinterpret_cast<uint8_t*>(norm) + b_norm);
