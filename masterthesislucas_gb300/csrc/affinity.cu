@@ -746,7 +746,7 @@ extern "C" int tc_symmetrize_device(const int32_t* d_idx, const double* d_p, int
     const int64_t tw = radix_tmp_words(m) > scan_tmp_words(m) ? radix_tmp_words(m) : scan_tmp_words(m);
     // scratch (32-bit words): values (2m); column keys, rows, the two sorts' keys and permutations, their
     // alternates and the sorted order (9 arrays of m); flags (m); positions (m + 1); sort/scan temporaries
-    const size_t words = (size_t)m * 2 + (size_t)m * 9 + (size_t)m + (size_t)(m + 1) + (size_t)tw;
+    const size_t words = (size_t)m * 2 + (size_t)m * 9 + (size_t)m + (size_t)(m + 2) + (size_t)tw;
     void* buf = nullptr;
     TC_CUDA_TRY(cudaMallocAsync(&buf, words * 4 + 64, s));
     uint32_t* w = static_cast<uint32_t*>(buf);
@@ -762,16 +762,18 @@ extern "C" int tc_symmetrize_device(const int32_t* d_idx, const double* d_p, int
     uint32_t* ord = av + m;
     uint32_t* flag = ord + m;
     uint32_t* pos = flag + m;
-    uint32_t* tmp = pos + (m + 1);  // ends at w + words
+    uint32_t* tmp = pos + (m + 2) - (m & 1);  // 8-byte aligned; ends before w + words
+    uint32_t* gave_up = w + words;  // set by a sort whose bounded waits ran out
     int rc = TC_OK;
     const double c = 1.0 / (2.0 * (double)n);
     k_sym_entries<<<grid_for(n * k, 256), 256, 0, s>>>(d_idx, d_p, n, k, c, colk, row, v);
     // stable sort by column, then stable by row: rows sorted, columns sorted within a row
     cudaError_t e = cudaMemcpyAsync(k1, colk, (size_t)m * 4, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) rc = radix_sort_u32(k1, p1, ak, av, m, tmp, s, nullptr, 0);
+    if (e == cudaSuccess) e = cudaMemsetAsync(gave_up, 0, 4, s);
+    if (e == cudaSuccess) rc = radix_sort_u32(k1, p1, ak, av, m, tmp, s, nullptr, 0, gave_up);
     if (e == cudaSuccess && rc == TC_OK) {
         k_gather_u32<<<grid_for(m, 256), 256, 0, s>>>(row, p1, m, k2);
-        rc = radix_sort_u32(k2, p2, ak, av, m, tmp, s, nullptr, 0);
+        rc = radix_sort_u32(k2, p2, ak, av, m, tmp, s, nullptr, 0, gave_up);
     }
     if (e == cudaSuccess && rc == TC_OK) {
         k_sym_flags<<<grid_for(m, 256), 256, 0, s>>>(p1, p2, m, row, colk, ord, flag);
@@ -779,10 +781,15 @@ extern "C" int tc_symmetrize_device(const int32_t* d_idx, const double* d_p, int
     }
     if (e == cudaSuccess && rc == TC_OK) {
         k_sym_write<<<grid_for(m, 256), 256, 0, s>>>(ord, flag, pos, m, n, row, colk, v, d_row_ptr, d_col, d_val);
-        uint32_t cnt = 0;
+        uint32_t cnt = 0, bad = 0;
         e = cudaMemcpyAsync(&cnt, pos + m, 4, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, gave_up, 4, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         *nnz = cnt;
+        if (e == cudaSuccess && bad) {
+            tc_set_error("tc_symmetrize_device: a bounded wait of the sort gave up");
+            rc = TC_ERR_TIMEOUT;
+        }
     }
     const cudaError_t ef = cudaFreeAsync(buf, s);
     if (e != cudaSuccess) return tc_cuda_fail(e, "tc_symmetrize_device");

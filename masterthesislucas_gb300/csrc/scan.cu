@@ -1,4 +1,6 @@
-// Device-wide exclusive prefix sum of u32 (reduce -> scan partials -> scan).
+// Device-wide exclusive prefix sum of u32.  Few values: one block, chunk after
+// chunk.  More: the chunks' sums, then a scan of each chunk whose block adds up
+// the sums before it; from kSelfChunks chunks on the sums are scanned first.
 #include "common.cuh"
 
 namespace tc {
@@ -76,10 +78,75 @@ __device__ __forceinline__ void store_chunk(uint32_t* __restrict__ out, int64_t 
     }
 }
 
+// up to this many chunks a block of the scan adds up the sums before its own chunk (16 loads a thread) instead of
+// waiting for a launch that scans them
+constexpr int64_t kSelfChunks = 16 * kScanThreads;
+
+__device__ __forceinline__ uint32_t carry_before(const uint32_t* __restrict__ partial, bool sums)
+{
+    if (!partial) return 0u;
+    if (!sums) return partial[blockIdx.x];
+    uint32_t c = 0;
+    for (int64_t k = threadIdx.x; k < blockIdx.x; k += kScanThreads) c += partial[k];
+    c = warp_sum(c);
+    __shared__ uint32_t ws[kScanThreads / 32];
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = c;
+    __syncthreads();
+    uint32_t t = 0;
+    for (int w = 0; w < kScanThreads / 32; w++) t += ws[w];
+    return t;
+}
+
+// few values: one block (per array), kBlockScan values at a time.  5,462 values: one launch of 5 us for three of 9 us
+constexpr int kBlockScanThreads = 1024, kBlockScanItems = 8;
+constexpr int64_t kBlockScan = 2 * kBlockScanThreads * kBlockScanItems;
+__global__ void __launch_bounds__(kBlockScanThreads)
+    k_scan_block(const uint32_t* __restrict__ in0, uint32_t* __restrict__ out0, const uint32_t* __restrict__ in1,
+                 uint32_t* __restrict__ out1, int64_t n, uint32_t cap0, uint32_t cap1)
+{
+    constexpr int kChunk = kBlockScanThreads * kBlockScanItems;
+    __shared__ uint32_t sm[kChunk + kChunk / 32];
+    const uint32_t* in = blockIdx.y ? in1 : in0;
+    uint32_t* out = blockIdx.y ? out1 : out0;
+    const uint32_t cap = blockIdx.y ? cap1 : cap0;
+    uint32_t carry = 0;
+    for (int64_t base = 0; base < n; base += kChunk) {
+#pragma unroll
+        for (int i = 0; i < kBlockScanItems; i++) {
+            const int x = i * kBlockScanThreads + threadIdx.x;
+            sm[chunk_slot(x)] = base + x < n ? in[base + x] : 0u;
+        }
+        __syncthreads();
+        uint32_t v[kBlockScanItems], s = 0;
+#pragma unroll
+        for (int i = 0; i < kBlockScanItems; i++) {
+            v[i] = sm[chunk_slot(threadIdx.x * kBlockScanItems + i)];
+            s += v[i];
+        }
+        uint32_t tot;
+        uint32_t ex = block_exclusive_scan(s, tot) + carry;
+#pragma unroll
+        for (int i = 0; i < kBlockScanItems; i++) {
+            sm[chunk_slot(threadIdx.x * kBlockScanItems + i)] = min(ex, cap);
+            ex += v[i];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kBlockScanItems; i++) {
+            const int x = i * kBlockScanThreads + threadIdx.x;
+            if (base + x < n) out[base + x] = sm[chunk_slot(x)];
+        }
+        carry += tot;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) out[n] = min(carry, cap);
+}
+
 __global__ void k_scan_final(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int64_t n,
-                             const uint32_t* __restrict__ partial, int64_t nb)
+                             const uint32_t* __restrict__ partial, int64_t nb, int sums)
 {
     __shared__ uint32_t sm[kChunkWords];
+    const uint32_t carry = carry_before(partial, sums);
     const int64_t base = (int64_t)blockIdx.x * kScanChunk;
     uint32_t v[kScanItems];
     load_chunk(in, base, n, sm, v);
@@ -87,7 +154,7 @@ __global__ void k_scan_final(const uint32_t* __restrict__ in, uint32_t* __restri
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) s += v[i];
     uint32_t tot;
-    uint32_t ex = block_exclusive_scan(s, tot) + partial[blockIdx.x];
+    uint32_t ex = block_exclusive_scan(s, tot) + carry;
 #pragma unroll
     for (int i = 0; i < kScanItems; i++) {
         const uint32_t x = v[i];
@@ -95,7 +162,7 @@ __global__ void k_scan_final(const uint32_t* __restrict__ in, uint32_t* __restri
         ex += x;
     }
     store_chunk(out, base, n, sm, v);
-    if (blockIdx.x == nb - 1 && threadIdx.x == 0) out[n] = partial[blockIdx.x] + tot;
+    if (blockIdx.x == nb - 1 && threadIdx.x == 0) out[n] = carry + tot;
 }
 
 // two arrays at once: blockIdx.y selects (in0, out0) or (in1, out1); the
@@ -140,12 +207,12 @@ __global__ void k_scan_partials2(uint32_t* partial, int64_t nb)
 // clamped to cap0 / cap1.
 __global__ void k_scan_final2(const uint32_t* __restrict__ in0, uint32_t* __restrict__ out0,
                               const uint32_t* __restrict__ in1, uint32_t* __restrict__ out1, int64_t n,
-                              const uint32_t* __restrict__ partial, int64_t nb, uint32_t cap0, uint32_t cap1)
+                              const uint32_t* __restrict__ partial, int64_t nb, uint32_t cap0, uint32_t cap1, int sums)
 {
     const uint32_t* in = blockIdx.y ? in1 : in0;
     uint32_t* out = blockIdx.y ? out1 : out0;
     const uint32_t cap = blockIdx.y ? cap1 : cap0;
-    const uint32_t carry = partial ? partial[blockIdx.y * nb + blockIdx.x] : 0u;
+    const uint32_t carry = carry_before(partial ? partial + blockIdx.y * nb : nullptr, sums);
     __shared__ uint32_t sm[kChunkWords];
     const int64_t base = (int64_t)blockIdx.x * kScanChunk;
     uint32_t v[kScanItems];
@@ -238,13 +305,19 @@ int exclusive_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, uint32_t* t
     if (nb == 1) {
         // one array: blockIdx.y is 0, the second pair is never read
         k_scan_final2<<<dim3(1, 1), kScanThreads, 0, s>>>(in, out, nullptr, nullptr, n, nullptr, 1, UINT32_MAX,
-                                                          UINT32_MAX);
+                                                          UINT32_MAX, 0);
         TC_CUDA_TRY(cudaGetLastError());
         return TC_OK;
     }
+    if (n <= kBlockScan) {
+        k_scan_block<<<dim3(1, 1), kBlockScanThreads, 0, s>>>(in, out, nullptr, nullptr, n, UINT32_MAX, UINT32_MAX);
+        TC_CUDA_TRY(cudaGetLastError());
+        return TC_OK;
+    }
+    const int sums = nb <= kSelfChunks;
     k_scan_reduce<<<(unsigned)nb, kScanThreads, 0, s>>>(in, n, tmp);
-    k_scan_partials<<<1, 1024, 0, s>>>(tmp, nb);
-    k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, tmp, nb);
+    if (!sums) k_scan_partials<<<1, 1024, 0, s>>>(tmp, nb);
+    k_scan_final<<<(unsigned)nb, kScanThreads, 0, s>>>(in, out, n, tmp, nb, sums);
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
 }
@@ -259,11 +332,15 @@ int exclusive_scan2_u32(const uint32_t* in0, uint32_t* out0, const uint32_t* in1
     }
     int64_t nb = (n + kScanChunk - 1) / kScanChunk;
     if (nb == 1) {
-        k_scan_final2<<<dim3(1, 2), kScanThreads, 0, s>>>(in0, out0, in1, out1, n, nullptr, 1, cap0, cap1);
+        k_scan_final2<<<dim3(1, 2), kScanThreads, 0, s>>>(in0, out0, in1, out1, n, nullptr, 1, cap0, cap1, 0);
+    } else if (n <= kBlockScan) {
+        k_scan_block<<<dim3(1, 2), kBlockScanThreads, 0, s>>>(in0, out0, in1, out1, n, cap0, cap1);
     } else {
+        const int sums = nb <= kSelfChunks;
         k_scan_reduce2<<<dim3((unsigned)nb, 2), kScanThreads, 0, s>>>(in0, in1, n, tmp, nb);
-        k_scan_partials2<<<2, 1024, 0, s>>>(tmp, nb);
-        k_scan_final2<<<dim3((unsigned)nb, 2), kScanThreads, 0, s>>>(in0, out0, in1, out1, n, tmp, nb, cap0, cap1);
+        if (!sums) k_scan_partials2<<<2, 1024, 0, s>>>(tmp, nb);
+        k_scan_final2<<<dim3((unsigned)nb, 2), kScanThreads, 0, s>>>(in0, out0, in1, out1, n, tmp, nb, cap0, cap1,
+                                                                     sums);
     }
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
