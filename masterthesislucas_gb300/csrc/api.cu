@@ -407,6 +407,7 @@ static int update_common(Handle& h, const double* d_pos, int64_t n, const double
     const bool coarse = split && h.nosync && far_coarse_applies(h);
     h.items_ready = false;
     h.coarse_ready = false;
+    h.err_read = false;
     h.split_mu = split;
     int rc = split ? ensure_near_stream(h) : TC_OK;
     if (!rc) rc = build_tree(h, d_pos, n, mn[0], mn[1], mx[0], mx[1]);
@@ -459,9 +460,12 @@ static int update_common(Handle& h, const double* d_pos, int64_t n, const double
         if (!rc && e != cudaSuccess) rc = tc_cuda_fail(e, "side-stream join");
     }
     if (rc) return rc;
-    TC_CUDA_TRY(cudaMemcpyAsync(h.h_words + 8, h.err.p, 4, cudaMemcpyDeviceToHost, h.stream));
-    if (h.nosync) return TC_OK;  // the caller reads the flags after its own synchronisation
-    TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    if (!h.err_read) {
+        TC_CUDA_TRY(cudaMemcpyAsync(h.h_words + 8, h.err.p, 4, cudaMemcpyDeviceToHost, h.stream));
+        if (h.nosync) return TC_OK;  // the caller reads the flags after its own synchronisation
+        TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    }
+    if (h.err_read) h.h_words[8] = h.h_words[kWordErr];  // where tc_async_status looks for it
     if (h.h_words[8]) {
         h.tree_ready = false;
         tc_set_error("a position is NaN or lies outside the bounding box");

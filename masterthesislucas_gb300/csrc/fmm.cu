@@ -94,19 +94,30 @@ struct Geo {
     int variant;       // 1: the non-symmetric FMM_MORTON leaf stage
 };
 
-template <typename real, typename K>
-__global__ void __launch_bounds__(128) k_m2l(K ker, int l, real hl, const uint32_t* __restrict__ nn_ptr,
-                                             const uint32_t* __restrict__ nn_idx, const real* __restrict__ comrel,
-                                             const real* __restrict__ m0r, const real* __restrict__ m2t,
-                                             real* __restrict__ loc, double* __restrict__ zpart)
+// box / 2^l, exactly
+__device__ __forceinline__ float level_size(float box, int l) { return box * __int_as_float((127 - l) << 23); }
+__device__ __forceinline__ double level_size(double box, int l)
 {
-    const uint32_t li = level_index(l);
-    const int64_t nl = (int64_t)1 << (2 * l);
+    return box * __longlong_as_double((long long)(1023 - l) << 52);
+}
+
+// all levels from 1 on in one launch (nodes n0 .. n1 of the level-dense numbering): they do not depend on one another
+template <typename real, typename K>
+__global__ void __launch_bounds__(128) k_m2l(K ker, int64_t n0, int64_t n1, real box, LevelLists lists,
+                                             const real* __restrict__ comrel, const real* __restrict__ m0r,
+                                             const real* __restrict__ m2t, real* __restrict__ loc,
+                                             double* __restrict__ zpart)
+{
     const int lane = threadIdx.x & 31;
     const int64_t wstride = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t a = blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); a < nl; a += wstride) {
-        const uint32_t b0 = nn_ptr[a], b1 = nn_ptr[a + 1];
-        const int64_t na = li + a;
+    for (int64_t na = n0 + blockIdx.x * (int64_t)(blockDim.x >> 5) + (threadIdx.x >> 5); na < n1; na += wstride) {
+        const int l = level_of((uint32_t)na);
+        const uint32_t li = level_index(l);
+        const int64_t nl = (int64_t)1 << (2 * l), a = na - li;
+        const real hl = level_size(box, l);
+        const uint32_t* nn_ptr = lists.ptr[l];
+        const uint32_t* nn_idx = lists.idx[l];
+        const uint32_t b0 = nn_ptr[a], b1 = nn_ptr[list_end(nl, a)];
         if (b0 == b1) {
             if (lane < L_NCOEF) loc[na * L_NCOEF + lane] = real(0);
             if (lane == 0) zpart[na] = 0.0;
@@ -245,7 +256,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
         const int isx = (int)compact16((uint32_t)si), isy = (int)compact16((uint32_t)si >> 1);
         const real csx = comrel[2 * S], csy = comrel[2 * S + 1];
         const real mS = m0r[S];
-        const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
+        const uint32_t e0 = near_ptr[si], e1 = near_ptr[list_end(nl, si)];
 #pragma unroll
         for (int c = 0; c < L_NCOEF; c++) C[c] = real(0);
         real zA = real(0);
@@ -452,7 +463,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
         const uint32_t m = min(32u, count[S] - c0);
         const int isx = (int)compact16((uint32_t)si), isy = (int)compact16((uint32_t)si >> 1);
         const real csx = comrel[2 * S], csy = comrel[2 * S + 1];
-        const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
+        const uint32_t e0 = near_ptr[si], e1 = near_ptr[list_end(nl, si)];
         const uint32_t lg = 5u - (32u - __clz(m - 1u));  // log2 g, g * m <= 32
         const uint32_t g = 1u << lg, r = lane & (g - 1u), sk = lane >> lg;
         const bool act = sk < m;
@@ -686,12 +697,9 @@ int solve_t(Handle& h, K ker, double* d_grad, int accumulate, int scatter, doubl
     TC_CUDA_TRY(cudaMemsetAsync(zp, 0, 8, s));
     const uint32_t* ptr = P<uint32_t>(h.ptr_pool);
     const uint32_t* idx = P<uint32_t>(h.idx_pool);
-    for (int l = 1; l <= dep; l++) {
-        const int64_t nl = (int64_t)1 << (2 * l);
-        const real hl = (real)(h.L / (double)(1u << l));
-        k_m2l<real, K><<<grid_for(nl * 32, 128, sm_count() * 64), 128, 0, s>>>(
-            ker, l, hl, ptr + h.lists.nn_ptr_off[l], idx + h.lists.nn_idx_off[l], P<real>(h.comrel), P<real>(h.m0r),
-            P<real>(h.m2t), loc, zp);
+    if (dep > 0) {
+        k_m2l<real, K><<<grid_for((nn - 1) * 32, 128, sm_count() * 64), 128, 0, s>>>(
+            ker, 1, nn, (real)h.L, level_lists(h), P<real>(h.comrel), P<real>(h.m0r), P<real>(h.m2t), loc, zp);
         h.launches++;
     }
     Geo geo;

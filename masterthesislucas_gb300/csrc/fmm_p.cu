@@ -528,25 +528,30 @@ __global__ void __launch_bounds__(128, L2L ? (P >= 8 ? TC_M2L_FUSED_MIN_BLOCKS :
 // idle behind each node's serial list: one warp per node instead, the lanes
 // taking the list's entries in turn (entry e to lane e mod 32) into their own
 // accumulators, then a fixed butterfly sum over the lanes.
+// The levels do not depend on one another, so levels l0 .. l1 share a launch:
+// one by one, seven levels of a 70,000-point tree took 109 us at order 8, most
+// of it the latency of each level's longest lists, and take 64 us us together.
 template <int P>
-__global__ void __launch_bounds__(128) k_m2l_warp(int l, float hl, PotParams pp, const uint32_t* __restrict__ nn_ptr,
-                                                  const uint32_t* __restrict__ nn_idx, const float* __restrict__ comrel,
-                                                  const float* __restrict__ mu, float* __restrict__ loc,
-                                                  double* __restrict__ zpart, const uint32_t* __restrict__ act,
-                                                  const uint32_t* __restrict__ act_pos)
+__global__ void __launch_bounds__(128) k_m2l_warp(int l0, int l1, float box, PotParams pp, LevelLists lists,
+                                                  const float* __restrict__ comrel, const float* __restrict__ mu,
+                                                  float* __restrict__ loc, double* __restrict__ zpart,
+                                                  const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
 {
     constexpr int K = ncoef(P), KS = kstride(P);
-    const uint32_t li = level_index(l);
-    const int64_t nl = (int64_t)1 << (2 * l);
-    const float ih = 1.0f / hl;
     const float2* comrel2 = reinterpret_cast<const float2*>(comrel);
     const int lane = threadIdx.x & 31;
-    const uint32_t k1 = act_pos[li + nl];
+    const uint32_t k0 = act_pos[level_index(l0)], k1 = act_pos[level_index(l1 + 1)];
     const uint32_t wstride = gridDim.x * (blockDim.x >> 5);
-    for (uint32_t k = act_pos[li] + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += wstride) {
+    for (uint32_t k = k0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += wstride) {
         const int64_t na = act[k];
-        const int64_t a = na - li;
-        const uint32_t b0 = nn_ptr[a], b1 = nn_ptr[a + 1];
+        const int l = level_of((uint32_t)na);
+        const uint32_t li = level_index(l);
+        const int64_t a = na - li, nl = (int64_t)1 << (2 * l);
+        const float hl = box * __int_as_float((127 - l) << 23);  // box / 2^l, exact
+        const float ih = 1.0f / hl;
+        const uint32_t* nn_ptr = lists.ptr[l];
+        const uint32_t* nn_idx = lists.idx[l];
+        const uint32_t b0 = nn_ptr[a], b1 = nn_ptr[list_end(nl, a)];
         float L[K];
 #pragma unroll
         for (int c = 0; c < K; c++) L[c] = 0.f;
@@ -678,7 +683,7 @@ __global__ void __launch_bounds__(128) k_m2l_mixed_warp(int l, float hl, PotPara
     for (uint32_t k = act_pos[li] + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += wstride) {
         const int64_t na = act[k];
         const int64_t a = na - li;
-        const uint32_t p0 = nn_ptr[a], b1 = nn_ptr[a + 1];
+        const uint32_t p0 = nn_ptr[a], b1 = nn_ptr[list_end(nl, a)];
         float L[K];
 #pragma unroll
         for (int c = 0; c < K; c++) L[c] = 0.f;
@@ -763,6 +768,9 @@ __global__ void __launch_bounds__(128) k_l2l(int l, float hl, const uint32_t* __
 // (measured: at level 9 of a 4M-particle tree the thread-per-node form is
 // already faster)
 constexpr int64_t kM2lWarpLevelNodes = (int64_t)1 << 16;
+// the finer levels' lists are always placed by a scan, so a list ends where the next starts (one cache line instead of
+// two: 472 us for 512 of a 4M-particle step's fine levels)
+static_assert(kListsOnceNodes <= kM2lWarpLevelNodes, "k_m2l_p and k_m2l_mixed read CSR lists");
 
 // ------------------------------------------------------------------ near field
 constexpr int kNearWarps = 4;
@@ -888,7 +896,7 @@ __device__ __forceinline__ float near_item(const KN& ker, int dep, float h, cons
     float gx = 0.f, gy = 0.f, zs = 0.f;
     uint32_t fill = 0, staged = 0;
     bool has_self = false;
-    const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
+    const uint32_t e0 = near_ptr[si], e1 = near_ptr[list_end((int64_t)1 << (2 * dep), si)];
     for (uint32_t eb = e0; eb < e1; eb += 32) {
         const uint32_t nt = min(32u, e1 - eb);
         uint32_t mf = 0, mc = 0;
@@ -1010,7 +1018,7 @@ __device__ __noinline__ float near_split_item(const KN& ker, int dep, float h, c
     const uint32_t s = fS + c0 + (act ? sk : 0u);
     const int isx = (int)compact16((uint32_t)si), isy = (int)compact16((uint32_t)si >> 1);
     const float2 p2 = act ? prel2[s] : make_float2(0.f, 0.f);
-    const uint32_t e0 = near_ptr[si], e1 = near_ptr[si + 1];
+    const uint32_t e0 = near_ptr[si], e1 = near_ptr[list_end((int64_t)1 << (2 * dep), si)];
     // the list's length in particles, and whether it holds the leaf itself
     uint32_t total = 0;
     bool has_self = false;
@@ -1304,6 +1312,7 @@ int m2l_tensor(Handle& h, const PotParams& pp)
     const uint32_t* count = P<uint32_t>(h.count);
     const uint32_t* ptr = P<uint32_t>(h.ptr_pool);
     const uint32_t* idx = P<uint32_t>(h.idx_pool);
+    const LevelLists lists = level_lists(h);
     // levels with few parents keep the SIMT kernels: a tile's offsets run one after another, so a level
     // needs tiles for every SM before the tensor cores pay
     int lmin = dep + 1;
@@ -1319,9 +1328,8 @@ int m2l_tensor(Handle& h, const PotParams& pp)
         const int64_t nl = (int64_t)1 << (2 * l);
         if (l < lmin) {
             if (nl <= kM2lWarpLevelNodes)
-                k_m2l_warp<Q><<<grid_for(nl * 32, 128), 128, 0, s>>>(l, hl, pp, ptr + h.lists.nn_ptr_off[l],
-                                                                   idx + h.lists.nn_idx_off[l], comrel, mu, loc,
-                                                                   zp, act, act_pos);
+                k_m2l_warp<Q><<<grid_for(nl * 32, 128), 128, 0, s>>>(l, l, (float)h.L, pp, lists, comrel, mu, loc, zp, act,
+                                                                     act_pos);
             else
                 k_m2l_p<Q><<<grid_for(nl, 128), 128, 0, s>>>(l, hl, pp, ptr + h.lists.nn_ptr_off[l],
                                                              idx + h.lists.nn_idx_off[l], count, comrel, mu, loc,
@@ -1416,6 +1424,7 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
     const float* comrel = P<float>(h.comrel);
     const uint32_t* count = P<uint32_t>(h.count);
     auto hl = [&](int l) { return (float)(h.L / (double)(1u << l)); };
+    const LevelLists lists = level_lists(h);
     if (h.mu_stride != kstride(ORD)) {
         tc_set_error("order-p solve: multipoles of another order (update the tree first)");
         return TC_ERR_STATE;
@@ -1434,14 +1443,21 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
         TC_CUDA_TRY(cudaMemsetAsync(loc, 0, kstride(ORD) * 4, s));
         TC_CUDA_TRY(cudaMemsetAsync(zp, 0, nn * 8, s));
     }
-    int nfused = 0;
+    // levels of one order and few nodes: all in one launch, unless an update has done them
+    int coarse_last = 0;
+    while (!tc_m2l && !per_pair && coarse_last < dep && ((int64_t)1 << (2 * (coarse_last + 1))) <= kM2lWarpLevelNodes)
+        coarse_last++;
     if (tc_m2l) {
         if ((rc = m2l_tensor<ORD>(h, pp))) return rc;
+    } else if (coarse_last > 0 && !coarse_done) {
+        const int64_t nn2 = (int64_t)level_index(coarse_last + 1);
+        k_m2l_warp<ORD><<<grid_for(nn2 * 32, 128), 128, 0, s>>>(1, coarse_last, (float)h.L, pp, lists, comrel, mu, loc,
+                                                                zp, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
+        h.launches++;
     }
-    for (int l = 1; l <= dep && !tc_m2l; l++) {
+    for (int l = coarse_last + 1; l <= dep && !tc_m2l; l++) {
         const int64_t nl = (int64_t)1 << (2 * l);
-        if (fuse && nl > kM2lWarpLevelNodes) continue;
-        if (coarse_done && nl <= kM2lWarpLevelNodes) continue;
+        if (fuse) continue;  // with the level's L2L below
         const uint32_t* np_ = ptr + h.lists.nn_ptr_off[l];
         const uint32_t* ni_ = idx + h.lists.nn_idx_off[l];
         bool mixed = false;
@@ -1477,14 +1493,10 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
                 mixed = true;
             }
         }
-        if (!mixed) {
-            if (nl <= kM2lWarpLevelNodes)
-                k_m2l_warp<ORD><<<grid_for(nl * 32, 128), 128, 0, s>>>(l, hl(l), pp, np_, ni_, comrel, mu, loc, zp,
-                                                                       act, act_pos);
-            else
-                k_m2l_p<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), pp, np_, ni_, count, comrel, mu, loc, zp,
-                                                               act, act_pos);
-        }
+        if (!mixed)
+            k_m2l_p<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), pp, np_, ni_, count, comrel, mu, loc, zp, act,
+                                                           act_pos);
+        h.launches++;
     }
     for (int l = 1; l <= dep; l++) {
         const int64_t nl = (int64_t)1 << (2 * l);
@@ -1494,7 +1506,7 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
                 k_m2l_p<ORD, true><<<grid_for(nl, 128), 128, 0, s>>>(
                     l, hl(l), pp, ptr + h.lists.nn_ptr_off[l], idx + h.lists.nn_idx_off[l], count, comrel, mu, loc,
                     zp, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
-                nfused++;
+                h.launches++;
                 continue;
             }
         }
@@ -1502,6 +1514,7 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
             k_l2l_stream<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, loc, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
         else
             k_l2l<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, loc, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
+        h.launches++;
     }
     // the far field's pair-sum parts, one word per node, summed on its stream while the near field runs
     const int64_t nsum = sum_tmp_doubles();
@@ -1530,9 +1543,9 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
     if ((rc = record(h, 6))) return rc;
     // the pair sum: the far field's total plus the near field's per-item words
     if ((rc = sum_f64(zfar, 1, P<double>(h.zwork), nz, d_total, 1, P<double>(h.sumtmp) + nsum, s))) return rc;
-    // far field (an M2L and an L2L launch per level, one fused launch per fine level), the near field, the
-    // L2P and two two-kernel sums; the item tables and a captured update's coarse levels count themselves
-    h.launches += 2 * dep - nfused + 6 - (coarse_done ? 2 * kFarCoarseLevel : 0);
+    // the near field, the L2P and two two-kernel sums; the far field, the item tables and a captured update's coarse
+    // levels count themselves
+    h.launches += 6;
     TC_CUDA_TRY(cudaGetLastError());
     if (tc_m2l) {
         // the tensor-core M2L's status word (list offsets beyond its operators, a bounded wait that gave up)
@@ -1638,17 +1651,13 @@ int far_coarse_p(Handle& h, const PotParams& pp)
     auto hl = [&](int l) { return (float)(h.L / (double)(1u << l)); };
     TC_CUDA_TRY(cudaMemsetAsync(loc, 0, kstride(ORD) * 4, s));
     TC_CUDA_TRY(cudaMemsetAsync(zp, 0, h.nnodes * 8, s));
-    for (int l = 1; l <= lc; l++) {
-        const int64_t nl = (int64_t)1 << (2 * l);
-        k_m2l_warp<ORD><<<grid_for(nl * 32, 128), 128, 0, s>>>(l, hl(l), pp, ptr + h.lists.nn_ptr_off[l],
-                                                               idx + h.lists.nn_idx_off[l], comrel, mu, loc, zp, act,
-                                                               act_pos);
-    }
+    k_m2l_warp<ORD><<<grid_for((int64_t)level_index(lc + 1) * 32, 128), 128, 0, s>>>(
+        1, lc, (float)h.L, pp, level_lists(h), comrel, mu, loc, zp, act, act_pos);
     for (int l = 1; l <= lc; l++) {
         const int64_t nl = (int64_t)1 << (2 * l);
         k_l2l<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, loc, act, act_pos);
     }
-    h.launches += 2 * lc;
+    h.launches += 1 + lc;
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
 }

@@ -17,6 +17,8 @@
 #include "controller.cuh"
 #include "expansion.cuh"
 #include "kernels.cuh"
+#include <vector>
+
 #include "state.cuh"
 
 namespace tc {
@@ -174,11 +176,24 @@ extern "C" int tc_get_list(tc_handle* t, int level, int kind, uint32_t* ptr, uin
         TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
         return TC_OK;
     }
+    // a level's lists may lie in any order, and the words of empty nodes are not set: CSR in node order from the
+    // starts, ends and particle counts
     const uint32_t* dptr = P<uint32_t>(h.ptr_pool) + (kind ? L.near_ptr_off[level] : L.nn_ptr_off[level]);
     const uint32_t* didx = P<uint32_t>(h.idx_pool) + (kind ? L.near_idx_off[level] : L.nn_idx_off[level]);
-    if (ptr) TC_CUDA_TRY(cudaMemcpyAsync(ptr, dptr, (nl + 1) * 4, cudaMemcpyDeviceToHost, h.stream));
-    if (idx && tot) TC_CUDA_TRY(cudaMemcpyAsync(idx, didx, tot * 4, cudaMemcpyDeviceToHost, h.stream));
+    std::vector<uint32_t> se(list_ptr_words(nl)), cnt(nl), raw(idx ? tot : 0);
+    TC_CUDA_TRY(cudaMemcpyAsync(se.data(), dptr, se.size() * 4, cudaMemcpyDeviceToHost, h.stream));
+    TC_CUDA_TRY(cudaMemcpyAsync(cnt.data(), P<uint32_t>(h.count) + level_index(level), nl * 4, cudaMemcpyDeviceToHost,
+                                h.stream));
+    if (!raw.empty()) TC_CUDA_TRY(cudaMemcpyAsync(raw.data(), didx, tot * 4, cudaMemcpyDeviceToHost, h.stream));
     TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    int64_t at = 0;
+    for (int64_t a = 0; a < nl; a++) {
+        if (ptr) ptr[a] = (uint32_t)at;
+        const int64_t b0 = se[a], b1 = cnt[a] ? se[list_end(nl, a)] : b0;
+        for (int64_t e = b0; idx && e < b1 && e < tot; e++) idx[at + (e - b0)] = raw[e];
+        at += b1 - b0;
+    }
+    if (ptr) ptr[nl] = (uint32_t)at;
     return TC_OK;
 }
 

@@ -66,12 +66,6 @@ __device__ inline bool mac_accept_fast(int dix, int diy, real hl, real thr2, con
     return variant ? mac_accept_m(a, b, len, theta) : mac_accept(a, b, len, inv_theta);
 }
 
-// levels of up to this many cells (4^TC_LISTS_WARP_LEVEL) build their lists with a warp per node
-#ifndef TC_LISTS_WARP_LEVEL
-#define TC_LISTS_WARP_LEVEL 8
-#endif
-constexpr int64_t kListsWarpLevelNodes = (int64_t)1 << (2 * TC_LISTS_WARP_LEVEL);
-
 // Squared-ratio thresholds of the per-pair order rule: an accepted pair with
 // (b_A + b_B)^2 <= t[o] |dcom|^2 takes order bucket o (orders 4, 6, 8, 10, 12);
 // t[o] = (slack theta^(p + 1))^(2 / (q_o + 1)) below the handle's order p,
@@ -88,8 +82,8 @@ __global__ void k_lists(int l, double inv_theta, double theta, int variant, real
                         const double2* __restrict__ com64, const real* __restrict__ comrel,
                         const double* __restrict__ bblen, const uint32_t* __restrict__ pnear_ptr,
                         const uint32_t* __restrict__ pnear_idx, uint32_t pcap, uint32_t* __restrict__ nn_cnt,
-                        uint32_t* __restrict__ near_cnt, const uint32_t* __restrict__ nn_ptr,
-                        uint32_t* __restrict__ nn_idx, uint32_t nn_cap, const uint32_t* __restrict__ near_ptr,
+                        uint32_t* __restrict__ near_cnt, uint32_t* __restrict__ nn_ptr,
+                        uint32_t* __restrict__ nn_idx, uint32_t nn_cap, uint32_t* __restrict__ near_ptr,
                         uint32_t* __restrict__ near_idx, uint32_t near_cap, uint32_t* __restrict__ ovf, int fill,
                         const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos,
                         const float* __restrict__ bmax, float theta2, uint8_t* __restrict__ nn_ord, OrderRule rule,
@@ -120,7 +114,7 @@ __global__ void k_lists(int l, double inv_theta, double theta, int variant, real
                 const real cra[2] = {comrel[2 * (li + a)], comrel[2 * (li + a) + 1]};
                 const float ba = bmax ? bmax[li + a] : 0.f;
                 const uint32_t p = (uint32_t)(a >> 2);
-                const uint32_t pe0 = pnear_ptr[p], pe1 = pnear_ptr[p + 1] < pcap ? pnear_ptr[p + 1] : pcap;
+                const uint32_t pe0 = pnear_ptr[p], pe1 = min(pnear_ptr[list_end(np, p)], pcap);
                 // p2p_cut (leaf level only; 0 off): an accepted pair of leaves with at most p2p_cut
                 // particle pairs goes to the near list, where direct P2P is cheaper than an M2L
                 const uint32_t ca_n = p2p_cut ? count[li + a] : 0u;
@@ -246,6 +240,9 @@ __global__ void k_lists(int l, double inv_theta, double theta, int variant, real
         if (!fill) {
             nn_cnt[a] = nn;
             near_cnt[a] = nr;
+        } else {
+            nn_ptr[list_end(nl, a)] = nn_ptr[a + 1];
+            near_ptr[list_end(nl, a)] = near_ptr[a + 1];
         }
     }
 }
@@ -266,8 +263,8 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
                                                     const uint32_t* __restrict__ pnear_ptr,
                                                     const uint32_t* __restrict__ pnear_idx, uint32_t pcap,
                                                     uint32_t* __restrict__ nn_cnt, uint32_t* __restrict__ near_cnt,
-                                                    const uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ nn_idx,
-                                                    uint32_t nn_cap, const uint32_t* __restrict__ near_ptr,
+                                                    uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ nn_idx,
+                                                    uint32_t nn_cap, uint32_t* __restrict__ near_ptr,
                                                     uint32_t* __restrict__ near_idx, uint32_t near_cap,
                                                     uint32_t* __restrict__ ovf, int fill,
                                                     const uint32_t* __restrict__ act,
@@ -284,9 +281,12 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
     for (uint32_t k = k0 + blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); k < k1; k += wstride) {
         const int64_t a = act ? (int64_t)act[k] - li : (int64_t)k;
         if (!act && count[li + a] == 0) {
-            if (!fill && lane == 0) {
+            if (lane == 0 && !fill) {
                 nn_cnt[a] = 0;
                 near_cnt[a] = 0;
+            } else if (lane == 0) {
+                nn_ptr[list_end(nl, a)] = nn_ptr[a + 1];
+                near_ptr[list_end(nl, a)] = near_ptr[a + 1];
             }
             continue;
         }
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
         const float ba = bmax ? bmax[li + a] : 0.f;
         const uint32_t ca_n = p2p_cut ? count[li + a] : 0u;
         const uint32_t p = (uint32_t)(a >> 2);
-        const uint32_t pe0 = pnear_ptr[p], pe1 = pnear_ptr[p + 1] < pcap ? pnear_ptr[p + 1] : pcap;
+        const uint32_t pe0 = pnear_ptr[p], pe1 = min(pnear_ptr[list_end(np, p)], pcap);
         const uint32_t ncand = 4u * (pe1 > pe0 ? pe1 - pe0 : 0u);
         uint32_t nn = 0, nr = 0;
         const uint32_t nb0 = fill ? nn_ptr[a] : 0u, rb0 = fill ? near_ptr[a] : 0u;
@@ -343,9 +343,180 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
             nn += __popc(m_acc);
             nr += __popc(m_rej);
         }
-        if (!fill && lane == 0) {
+        if (lane == 0 && !fill) {
             nn_cnt[a] = nn;
             near_cnt[a] = nr;
+        } else if (lane == 0) {
+            nn_ptr[list_end(nl, a)] = nn_ptr[a + 1];
+            near_ptr[list_end(nl, a)] = near_ptr[a + 1];
+        }
+    }
+}
+
+// The root's lists, and the counters of the levels that k_lists_once builds
+__global__ void k_lists_root(uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ near_ptr,
+                             uint32_t* __restrict__ near_idx, unsigned long long* __restrict__ total, int nlev,
+                             uint32_t* __restrict__ ovf)
+{
+    if ((int)threadIdx.x < nlev) total[threadIdx.x] = threadIdx.x == 0 ? 1ull : 0ull;  // the root is near itself
+    if (threadIdx.x == 0) {
+        nn_ptr[0] = nn_ptr[list_end(1, 0)] = 0;
+        near_ptr[0] = 0;
+        near_ptr[list_end(1, 0)] = 1;
+        near_idx[0] = 0;
+        *ovf = 0;
+    }
+}
+
+// A coarse level in one pass, where the lists' regions are sized beforehand: a
+// warp per non-empty node decides on its candidates as k_lists_warp does,
+// reserves room for both lists by one addition to the level's totals, and
+// writes them.  Consumers read a list by its start and end, so where a list
+// lies does not matter; its entries and their order are k_lists_warp's.  What
+// bounds a level is the chain of dependent loads (parent's list, node
+// records): 128 candidates are taken at a time, their loads in flight
+// together, and their outcomes kept in shared memory for the writing.  Against
+// counting, scanning and filling (two clears, three to five launches a level):
+// 70,000 points, seven levels: 190 us before, 66 us now.
+constexpr int kOnceWarps = 4;
+constexpr int kOnceBatches = 64;  // outcomes kept; candidates beyond 32 times that are decided again
+
+template <typename real>
+__global__ void __launch_bounds__(32 * kOnceWarps)
+    k_lists_once(int l, double inv_theta, double theta, int variant, real hl, const uint32_t* __restrict__ count,
+                 const double2* __restrict__ com64, const real* __restrict__ comrel, const double* __restrict__ bblen,
+                 const uint32_t* __restrict__ pnear_ptr, const uint32_t* __restrict__ pnear_idx, uint32_t pcap,
+                 uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ nn_idx, uint32_t nn_cap,
+                 uint32_t* __restrict__ near_ptr, uint32_t* __restrict__ near_idx, uint32_t near_cap,
+                 unsigned long long* __restrict__ total, uint32_t* __restrict__ ovf, const uint32_t* __restrict__ act,
+                 const uint32_t* __restrict__ act_pos, const float* __restrict__ bmax, float theta2, uint32_t p2p_cut)
+{
+    __shared__ uint2 s_mask[kOnceWarps][kOnceBatches];
+    const uint32_t np = 1u << (2 * (l - 1));
+    const uint32_t li = level_index(l);
+    const int64_t nl = (int64_t)1 << (2 * l);
+    const int lane = threadIdx.x & 31;
+    uint2* mask = s_mask[threadIdx.x >> 5];
+    const uint32_t lt = (1u << lane) - 1u;
+    const uint32_t k0 = act ? act_pos[li] : 0u, k1 = act ? act_pos[li + nl] : (uint32_t)nl;
+    for (uint32_t k = k0 + blockIdx.x * kOnceWarps + (threadIdx.x >> 5); k < k1; k += gridDim.x * kOnceWarps) {
+        const int64_t a = act ? (int64_t)act[k] - li : (int64_t)k;
+        const uint32_t ca_n = count[li + a];
+        if (ca_n == 0) {  // without an active-node list
+            if (lane == 0) {
+                nn_ptr[a] = nn_ptr[list_end(nl, a)] = 0;
+                near_ptr[a] = near_ptr[list_end(nl, a)] = 0;
+            }
+            continue;
+        }
+        const double len = bblen[li + a];
+        const real thr = (real)((len + len) * inv_theta);
+        const real thr2 = thr * thr;
+        const int iax = (int)compact16((uint32_t)a), iay = (int)compact16((uint32_t)a >> 1);
+        const real cra[2] = {comrel[2 * (li + a)], comrel[2 * (li + a) + 1]};
+        const float ba = bmax ? bmax[li + a] : 0.f;
+        const uint32_t p = (uint32_t)(a >> 2);
+        const uint32_t pe0 = pnear_ptr[p], pe1 = min(pnear_ptr[list_end(np, p)], pcap);
+        const uint32_t ncand = 4u * (pe1 > pe0 ? pe1 - pe0 : 0u);
+        // candidates c0 + 32 u + lane, u < 4: their nodes, and their two outcomes as ballots
+        auto decide = [&](uint32_t c0, uint32_t (&b)[4], uint2 (&m)[4]) {
+            uint32_t cb[4];
+            real crx[4], cry[4];
+            float bb[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t c = c0 + 32u * u + lane;
+                const uint32_t bp = c < ncand ? pnear_idx[pe0 + (c >> 2)] : np;
+                b[u] = bp < np ? 4 * bp + (c & 3) : 0xFFFFFFFFu;  // beyond: only after an overflowed parent level
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const bool in = b[u] != 0xFFFFFFFFu;
+                const uint32_t j = in ? li + b[u] : li + (uint32_t)a;
+                cb[u] = in ? count[j] : 0u;
+                crx[u] = comrel[2 * (int64_t)j];
+                cry[u] = comrel[2 * (int64_t)j + 1];
+                bb[u] = bmax ? bmax[j] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const bool valid = cb[u] != 0;
+                bool acc = false;
+                if (valid) {
+                    const int dix = iax - (int)compact16(b[u]), diy = iay - (int)compact16(b[u] >> 1);
+                    if (bmax) {
+                        const float dx = (float)dix * (float)hl + (float)(cra[0] - crx[u]);
+                        const float dy = (float)diy * (float)hl + (float)(cra[1] - cry[u]);
+                        const float rb = ba + bb[u];
+                        acc = theta2 * fmaf(dx, dx, dy * dy) > rb * rb;
+                    } else {
+                        // mac_accept_fast, its FP64 records read only where FP32 does not decide
+                        const real dx = (real)dix * hl + (cra[0] - crx[u]), dy = (real)diy * hl + (cra[1] - cry[u]);
+                        const real d2 = dx * dx + dy * dy;
+                        acc = d2 > thr2 * (real)(1.0 + 1e-5);
+                        if (sizeof(real) == 8 || !(acc || d2 < thr2 * (real)(1.0 - 1e-5))) {
+                            const double2 A = com64[li + a], Bc = com64[li + b[u]];
+                            acc = variant ? mac_accept_m(A, Bc, len, theta) : mac_accept(A, Bc, len, inv_theta);
+                        }
+                    }
+                    if (acc && p2p_cut && ca_n * cb[u] <= p2p_cut) acc = false;
+                }
+                m[u].x = __ballot_sync(0xffffffffu, valid && acc);
+                m[u].y = __ballot_sync(0xffffffffu, valid && !acc);
+            }
+        };
+        uint32_t nn = 0, nr = 0;
+        uint32_t b[4];
+        uint2 m[4];
+        __syncwarp();
+        for (uint32_t c0 = 0; c0 < ncand; c0 += 128) {
+            decide(c0, b, m);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                nn += __popc(m[u].x);
+                nr += __popc(m[u].y);
+                if (lane == 0 && c0 / 32 + u < kOnceBatches) mask[c0 / 32 + u] = m[u];
+            }
+        }
+        unsigned long long at = 0;
+        if (lane == 0) at = atomicAdd(total, (unsigned long long)nn << 32 | nr);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        const uint32_t nb0 = (uint32_t)(at >> 32), rb0 = (uint32_t)at;
+        if (lane == 0) {
+            // an overflowed level's lists end at their region's end (and the flag asks for another build)
+            if (nb0 + nn > nn_cap || rb0 + nr > near_cap) atomicOr(ovf, 1u);
+            nn_ptr[a] = min(nb0, nn_cap);
+            nn_ptr[list_end(nl, a)] = min(nb0 + nn, nn_cap);
+            near_ptr[a] = min(rb0, near_cap);
+            near_ptr[list_end(nl, a)] = min(rb0 + nr, near_cap);
+        }
+        uint32_t pn = nb0, pr = rb0;
+        const bool one = ncand <= 128;  // the nodes and outcomes are still at hand
+        for (uint32_t c0 = 0; c0 < ncand; c0 += 128) {
+            if (!one) {
+                if (c0 / 32 + 4 <= kOnceBatches) {
+#pragma unroll
+                    for (int u = 0; u < 4; u++) {
+                        const uint32_t c = c0 + 32u * u + lane;
+                        m[u] = c0 / 32 + u < (ncand + 31) / 32 ? mask[c0 / 32 + u] : make_uint2(0u, 0u);
+                        b[u] = c < ncand ? 4 * pnear_idx[pe0 + (c >> 2)] + (c & 3) : 0u;
+                    }
+                } else {
+                    decide(c0, b, m);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                if (m[u].x >> lane & 1u) {
+                    const uint32_t pos = pn + __popc(m[u].x & lt);
+                    if (pos < nn_cap) nn_idx[pos] = b[u];
+                } else if (m[u].y >> lane & 1u) {
+                    const uint32_t pos = pr + __popc(m[u].y & lt);
+                    if (pos < near_cap) near_idx[pos] = b[u];
+                }
+                pn += __popc(m[u].x);
+                pr += __popc(m[u].y);
+            }
         }
     }
 }
@@ -415,7 +586,7 @@ __global__ void __launch_bounds__(32 * ctrl::kWarps) k_lists_ctrl_count(
         if (active) {
             const uint32_t p = (uint32_t)(a >> 2);
             e = pnear_ptr[p];
-            e1 = pnear_ptr[p + 1] < pcap ? pnear_ptr[p + 1] : pcap;
+            e1 = min(pnear_ptr[list_end(np, p)], pcap);
             iax = (int)compact16((uint32_t)a);
             iay = (int)compact16((uint32_t)a >> 1);
             cax = comrel[2 * (li + a)] * ih;
@@ -483,8 +654,8 @@ __global__ void __launch_bounds__(32 * ctrl::kWarps) k_lists_ctrl_count(
 // that the M2L launch of one bucket reads one contiguous range per node.
 __global__ void k_lists_ctrl_fill(int l, const uint32_t* __restrict__ count, const uint32_t* __restrict__ pnear_ptr,
                                   const uint32_t* __restrict__ pnear_idx, uint32_t pcap, const uint8_t* __restrict__ dec,
-                                  const uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ nn_idx,
-                                  uint8_t* __restrict__ nn_ord, uint32_t nn_cap, const uint32_t* __restrict__ near_ptr,
+                                  uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ nn_idx,
+                                  uint8_t* __restrict__ nn_ord, uint32_t nn_cap, uint32_t* __restrict__ near_ptr,
                                   uint32_t* __restrict__ near_idx, uint32_t near_cap, uint32_t* __restrict__ ovf,
                                   const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
 {
@@ -497,7 +668,7 @@ __global__ void k_lists_ctrl_fill(int l, const uint32_t* __restrict__ count, con
         const int64_t a = (int64_t)act[k] - li;
         const uint32_t p = (uint32_t)(a >> 2);
         const uint32_t pe0 = pnear_ptr[p];
-        const uint32_t pe1 = pnear_ptr[p + 1] < pcap ? pnear_ptr[p + 1] : pcap;
+        const uint32_t pe1 = min(pnear_ptr[list_end(np, p)], pcap);
         uint32_t start[TC_MLP_OUT] = {0, 0, 0, 0, 0};
         for (uint32_t e = pe0; e < pe1; e++) {
             const uint32_t bp = pnear_idx[e];
@@ -537,16 +708,30 @@ __global__ void k_lists_ctrl_fill(int l, const uint32_t* __restrict__ count, con
                 }
             }
         }
+        nn_ptr[list_end(nl, a)] = nn_ptr[a + 1];
+        near_ptr[list_end(nl, a)] = near_ptr[a + 1];
     }
 }
 
-// per-level list totals (last entries of the CSR pointer arrays)
-__global__ void k_list_totals(const uint32_t* __restrict__ ptr, const int64_t* __restrict__ offs, int nlev,
+// what the host reads after a build: per level the totals of both kinds (from
+// the scans' last words, or the counters of the levels built in one pass), at
+// kWordOvf the overflow flag and at kWordErr the tree's error flag
+struct ListOffs {
+    int64_t nn[16], near[16];
+};
+__global__ void k_list_totals(const uint32_t* __restrict__ ptr, ListOffs offs, int nlev,
+                              const unsigned long long* __restrict__ total, int nonce, const uint32_t* __restrict__ err,
                               uint32_t* __restrict__ out)
 {
-    for (int k = threadIdx.x; k < 2 * nlev; k += blockDim.x) {
-        const int l = k >> 1;
-        out[k] = ptr[offs[k] + ((int64_t)1 << (2 * l))];
+    const int l = threadIdx.x;
+    if (l < nlev) {
+        const int64_t nl = (int64_t)1 << (2 * l);
+        out[2 * l] = l < nonce ? (uint32_t)(total[l] >> 32) : ptr[offs.nn[l] + nl];
+        out[2 * l + 1] = l < nonce ? (uint32_t)total[l] : ptr[offs.near[l] + nl];
+    }
+    if (l == 0) {
+        out[kWordOvf] = err[1];
+        out[kWordErr] = err[0];
     }
 }
 
@@ -588,18 +773,18 @@ int build_lists(Handle& h)
     L.near_ptr_off.assign(depth + 1, 0);
     L.nn_idx_off.assign(depth + 1, 0);
     L.near_idx_off.assign(depth + 1, 0);
-    // pointer pool: two (4^l + 1)-word CSR pointer arrays per level
+    // pointer pool: the starts and ends of both kinds per level
     int64_t ptr_words = 0;
     for (int l = 0; l <= depth; l++) {
         int64_t nl = (int64_t)1 << (2 * l);
         L.nn_ptr_off[l] = ptr_words;
-        ptr_words += nl + 1;
+        ptr_words += list_ptr_words(nl);
         L.near_ptr_off[l] = ptr_words;
-        ptr_words += nl + 1;
+        ptr_words += list_ptr_words(nl);
     }
     const int64_t nleaf = (int64_t)1 << (2 * depth);
     int rc;
-    if ((rc = ensure(h.ptr_pool, ptr_words * 4)) || (rc = ensure(h.cnt_tmp, 2 * nleaf * 4 + 64)) ||
+    if ((rc = ensure(h.ptr_pool, ptr_words * 4)) || (rc = ensure(h.lstat, 16 * 8 + 64 * 4)) || (rc = ensure(h.cnt_tmp, 2 * nleaf * 4 + 64)) ||
         (rc = ensure(h.tmp, (radix_tmp_words(h.n) > 2 * scan_tmp_words(nleaf) ? radix_tmp_words(h.n)
                                                                                : 2 * scan_tmp_words(nleaf)) * 4)))
         return rc;
@@ -622,7 +807,7 @@ int build_lists(Handle& h)
     const double inv_theta = 1.0 / h.cfg.theta;
     uint32_t* ovf_flag = P<uint32_t>(h.err) + 1;
     auto launch = [&](int l, const uint32_t* pnp, const uint32_t* pni, uint32_t pcap, uint32_t* nnc, uint32_t* nrc,
-                      const uint32_t* nnp, uint32_t* nni, uint32_t nncap, const uint32_t* nrp, uint32_t* nri,
+                      uint32_t* nnp, uint32_t* nni, uint32_t nncap, uint32_t* nrp, uint32_t* nri,
                       uint32_t nrcap, int fill) -> int {
         const int64_t nl = (int64_t)1 << (2 * l);
         const double hl = h.L / (double)(1u << l);
@@ -641,7 +826,7 @@ int build_lists(Handle& h)
                                                                     P<uint8_t>(h.dec), nnp, nni, ordp, nncap, nrp,
                                                                     nri, nrcap, ovf_flag, act, act_pos);
             }
-        } else if (h.cfg.precision == TC_PREC_FP64 && l > 0 && nl <= kListsWarpLevelNodes) {
+        } else if (h.cfg.precision == TC_PREC_FP64 && l > 0 && nl <= kListsOnceNodes) {
             k_lists_warp<double><<<grid_for(nl * 32, 128), 128, 0, s>>>(
                 l, inv_theta, h.cfg.theta, h.variant, hl, P<uint32_t>(h.count), P<double2>(h.com64),
                 P<double>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnc, nrc, nnp, nni, nncap, nrp, nri, nrcap,
@@ -660,7 +845,7 @@ int build_lists(Handle& h)
                 int rc2 = ensure(h.dec, (size_t)pcap * 4 + 64);
                 if (rc2) return rc2;
             }
-            if (!adapt && l > 0 && nl <= kListsWarpLevelNodes) {
+            if (!adapt && l > 0 && nl <= kListsOnceNodes) {
                 k_lists_warp<float><<<grid_for(nl * 32, 128), 128, 0, s>>>(
                     l, inv_theta, h.cfg.theta, h.variant, (float)hl, P<uint32_t>(h.count), P<double2>(h.com64),
                     P<float>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnc, nrc, nnp, nni, nncap, nrp, nri, nrcap,
@@ -698,7 +883,6 @@ int build_lists(Handle& h)
         h.launches++;
     }
     uint32_t* ovf = P<uint32_t>(h.err) + 1;
-    TC_CUDA_TRY(cudaMemsetAsync(ovf, 0, 4, s));
     // Fast mode: per-level regions sized from the last exact totals (x1.25),
     // no host round trip between levels; one synchronisation at the end
     // verifies that no level overflowed, else the exact mode reruns.
@@ -717,11 +901,44 @@ int build_lists(Handle& h)
         }
         if ((rc = ensure(h.idx_pool, (size_t)words * 4 + 64))) return rc;
         if ((h.ctrl_on || adapt) && (rc = ensure(h.ord_pool, h.idx_pool.bytes / 4 + 64))) return rc;
-        for (int l = 0; l <= depth; l++) {
+        // levels 0 .. nonce - 1 in one pass each: levels of up to kListsOnceNodes cells without per-pair orders
+        unsigned long long* total = P<unsigned long long>(h.lstat);
+        int nonce = 0;
+        if (!h.ctrl_on && !adapt)
+            while (nonce <= depth && ((int64_t)1 << (2 * nonce)) <= kListsOnceNodes) nonce++;
+        if (nonce) {
+            k_lists_root<<<1, 32, 0, s>>>(ptr + L.nn_ptr_off[0], ptr + L.near_ptr_off[0],
+                                          P<uint32_t>(h.idx_pool) + L.near_idx_off[0], total, depth + 1, ovf);
+            h.launches++;
+            if (h.lists_event_level == 0) TC_CUDA_TRY(cudaEventRecord(h.ev_lists, s));
+        } else {
+            TC_CUDA_TRY(cudaMemsetAsync(ovf, 0, 4, s));
+        }
+        for (int l = nonce ? 1 : 0; l <= depth; l++) {
             const int64_t nl = (int64_t)1 << (2 * l);
             const uint32_t* pnp = l ? ptr + L.near_ptr_off[l - 1] : nullptr;
             const uint32_t* pni = l ? P<uint32_t>(h.idx_pool) + L.near_idx_off[l - 1] : nullptr;
             const uint32_t pcap = l ? L.near_cap[l - 1] : 0u;
+            if (l < nonce) {
+                const double hl = h.L / (double)(1u << l);
+                uint32_t *nnp = ptr + L.nn_ptr_off[l], *nrp = ptr + L.near_ptr_off[l];
+                uint32_t *nni = P<uint32_t>(h.idx_pool) + L.nn_idx_off[l], *nri = P<uint32_t>(h.idx_pool) + L.near_idx_off[l];
+                if (h.cfg.precision == TC_PREC_FP64)
+                    k_lists_once<double><<<grid_for(nl, kOnceWarps), 32 * kOnceWarps, 0, s>>>(
+                        l, inv_theta, h.cfg.theta, h.variant, hl, P<uint32_t>(h.count), P<double2>(h.com64),
+                        P<double>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnp, nni, L.nn_cap[l], nrp, nri,
+                        L.near_cap[l], total + l, ovf, nullptr, nullptr, nullptr, 0.f, 0u);
+                else
+                    k_lists_once<float><<<grid_for(nl, kOnceWarps), 32 * kOnceWarps, 0, s>>>(
+                        l, inv_theta, h.cfg.theta, h.variant, (float)hl, P<uint32_t>(h.count), P<double2>(h.com64),
+                        P<float>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnp, nni, L.nn_cap[l], nrp, nri,
+                        L.near_cap[l], total + l, ovf, act, act_pos, bmax, (float)(h.cfg.theta * h.cfg.theta),
+                        act && l == depth ? h.p2p_cut : 0u);
+                h.launches++;
+                // the levels so far are final: work that reads only them may start on another stream
+                if (l == h.lists_event_level) TC_CUDA_TRY(cudaEventRecord(h.ev_lists, s));
+                continue;
+            }
             if (act) {
                 TC_CUDA_TRY(cudaMemsetAsync(nn_cnt, 0, nl * 4, s));
                 TC_CUDA_TRY(cudaMemsetAsync(near_cnt, 0, nl * 4, s));
@@ -746,25 +963,23 @@ int build_lists(Handle& h)
         }
         if (h.nosync) {
             // captured step: the overflow flag lands in pinned memory for the caller to check
-            TC_CUDA_TRY(cudaMemcpyAsync(h.h_words + 40, ovf, 4, cudaMemcpyDeviceToHost, s));
+            TC_CUDA_TRY(cudaMemcpyAsync(h.h_words + kWordOvf, ovf, 4, cudaMemcpyDeviceToHost, s));
             TC_CUDA_TRY(cudaGetLastError());
             return TC_OK;
         }
-        // totals of every level plus the overflow flag, in one round trip
-        std::vector<int64_t> offs(2 * (depth + 1));
+        // totals of every level plus the overflow and error flags, in one round trip
+        ListOffs offs;
         for (int l = 0; l <= depth; l++) {
-            offs[2 * l] = L.nn_ptr_off[l];
-            offs[2 * l + 1] = L.near_ptr_off[l];
+            offs.nn[l] = L.nn_ptr_off[l];
+            offs.near[l] = L.near_ptr_off[l];
         }
-        if ((rc = ensure(h.lstat, offs.size() * 8 + 4 * 64))) return rc;
-        TC_CUDA_TRY(cudaMemcpyAsync(h.lstat.p, offs.data(), offs.size() * 8, cudaMemcpyHostToDevice, s));
-        uint32_t* dtot = (uint32_t*)((char*)h.lstat.p + offs.size() * 8);
-        k_list_totals<<<1, 64, 0, s>>>(ptr, P<int64_t>(h.lstat), depth + 1, dtot);
+        uint32_t* dtot = reinterpret_cast<uint32_t*>(total + 16);
+        k_list_totals<<<1, 32, 0, s>>>(ptr, offs, depth + 1, total, nonce, P<uint32_t>(h.err), dtot);
         h.launches++;
-        TC_CUDA_TRY(cudaMemcpyAsync(h.h_words, dtot, 4 * 2 * (depth + 1), cudaMemcpyDeviceToHost, s));
-        TC_CUDA_TRY(cudaMemcpyAsync(h.h_words + 40, ovf, 4, cudaMemcpyDeviceToHost, s));
+        TC_CUDA_TRY(cudaMemcpyAsync(h.h_words, dtot, 4 * (kWordErr + 1), cudaMemcpyDeviceToHost, s));
         TC_CUDA_TRY(cudaStreamSynchronize(s));
-        bool over = h.h_words[40] != 0;
+        h.err_read = true;
+        bool over = h.h_words[kWordOvf] != 0;
         for (int l = 0; l <= depth; l++) {
             L.nn_total[l] = h.h_words[2 * l];
             L.near_total[l] = h.h_words[2 * l + 1];
@@ -774,8 +989,8 @@ int build_lists(Handle& h)
             TC_CUDA_TRY(cudaGetLastError());
             return record(h, 3);
         }
-        TC_CUDA_TRY(cudaMemsetAsync(ovf, 0, 4, s));
     }
+    TC_CUDA_TRY(cudaMemsetAsync(ovf, 0, 4, s));
     // exact mode: the host reads each level's totals before the next level
     // (the first call, and after a fast-mode overflow)
     int64_t idx_words = 0;

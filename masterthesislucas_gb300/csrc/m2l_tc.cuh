@@ -39,6 +39,7 @@
 #include <cuda_bf16.h>
 
 #include "expansion.cuh"
+#include "state.cuh"
 #include "tcgen05.cuh"
 
 namespace tc {
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(128, 1)
         const uint32_t a = kk < k1 ? 4u * (act[kk] - lp) + (tile & 3u) : 0u;  // level-local child index
         const int64_t na = (int64_t)li + a;
         const bool row_ok = kk < k1 && count[na] != 0;
-        const uint32_t e0 = row_ok ? nn_ptr[a] : 0u, e1 = row_ok ? nn_ptr[a + 1] : 0u;
+        const uint32_t e0 = row_ok ? nn_ptr[a] : 0u, e1 = row_ok ? nn_ptr[list_end((int64_t)1 << (2 * l), a)] : 0u;
         const int iax = (int)compact16(a), iay = (int)compact16(a >> 1);
         auto offset_of = [&](uint32_t b, int& oid) {
             const int ox = iax - (int)compact16(b), oy = iay - (int)compact16(b >> 1);

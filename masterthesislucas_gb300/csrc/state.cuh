@@ -29,13 +29,36 @@ struct Buf {
 };
 
 struct Lists {
-    // per level l (0..depth): CSR over the 4^l nodes of the level (dense index)
+    // per level l (0..depth) and kind: starts of the 4^l nodes' lists (dense index; one more word, the total, where
+    // a scan placed them), then their ends (list_end).  A level built in one pass places its nodes' lists in no
+    // particular order
     std::vector<uint32_t> nn_total, near_total;  // host copies of the totals
     std::vector<int64_t> nn_ptr_off, near_ptr_off;   // word offsets into ptr pool
     std::vector<int64_t> nn_idx_off, near_idx_off;   // word offsets into idx pool
     std::vector<uint32_t> nn_cap, near_cap;          // region sizes of the fast build
     int caps_depth = -1;
 };
+
+// words of h_words that a list build writes: the overflow and error flags (the totals come before)
+constexpr int kWordOvf = 40, kWordErr = 41;
+// levels of up to this many cells (4^TC_LISTS_WARP_LEVEL) build their lists with a warp per node, in one pass where
+// their sizes are known beforehand
+#ifndef TC_LISTS_WARP_LEVEL
+#define TC_LISTS_WARP_LEVEL 8
+#endif
+constexpr int64_t kListsOnceNodes = (int64_t)1 << (2 * TC_LISTS_WARP_LEVEL);
+// end of node a's list in a level of nl nodes
+__host__ __device__ inline int64_t list_end(int64_t nl, int64_t a) { return nl + 1 + a; }
+// words of one kind's starts and ends
+inline int64_t list_ptr_words(int64_t nl) { return 2 * nl + 1; }
+
+// the accepted-pair lists of all levels, for kernels that take several levels at once
+struct LevelLists {
+    const uint32_t* ptr[16];
+    const uint32_t* idx[16];
+};
+// level of node i of the level-dense numbering (level_index(l) = (4^l - 1) / 3 nodes come before level l)
+__device__ inline int level_of(uint32_t i) { return (63 - __clzll((long long)(3ull * i + 1ull))) >> 1; }
 
 struct Handle {
     tc_config cfg;
@@ -47,6 +70,7 @@ struct Handle {
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_tree = nullptr, ev_grad = nullptr;
     bool wait_grad = false;
+    bool err_read = false;  // the list build has brought the tree's error flag to h_words[kWordErr]
     // order-p solves: the near field on near_stream beside the far field on far_stream (higher priority),
     // both forked by ev_fork and joined by ev_join / ev_far before the L2P; the near field's FP32 forces
     // in nearf (sorted order)
@@ -154,6 +178,16 @@ inline T* P(const Buf& b) { return reinterpret_cast<T*>(b.p); }
 
 // tree.cu
 int build_tree(Handle& h, const double* d_pos, int64_t n, double minx, double miny, double maxx, double maxy);
+inline LevelLists level_lists(const Handle& h)
+{
+    LevelLists r{};
+    for (int l = 0; l <= h.depth; l++) {
+        r.ptr[l] = static_cast<const uint32_t*>(h.ptr_pool.p) + h.lists.nn_ptr_off[l];
+        r.idx[l] = static_cast<const uint32_t*>(h.idx_pool.p) + h.lists.nn_idx_off[l];
+    }
+    return r;
+}
+
 // lists.cu
 int build_lists(Handle& h);
 // fmm.cu

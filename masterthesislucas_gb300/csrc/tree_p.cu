@@ -181,18 +181,18 @@ __device__ __forceinline__ void bottom_up_node(int l, int64_t i, double minx, do
     uint32_t fp = 0;
     float sx = 0.f, sy = 0.f;
     float2 g[4];
-    double2 bbox = make_double2(0.0, 0.0);
+    // bottomUpNodeConstruction's box (:381-470): offset[j] * L_child + BBcentre_child of the lowest non-empty child
+    // (bit 0 of the child slot is x)
+    const int j0 = c4[0] ? 0 : c4[1] ? 1 : c4[2] ? 2 : 3;
+    const double cl = bblen[fc + j0];
+    const double2 cb = bbc[fc + j0];
+    const double2 bbox = make_double2(__dadd_rn(__dmul_rn((j0 & 1) ? -0.5 : 0.5, cl), cb.x),
+                                      __dadd_rn(__dmul_rn((j0 & 2) ? -0.5 : 0.5, cl), cb.y));
+    fp = first[fc + j0];
 #pragma unroll
     for (int j = 3; j >= 0; j--) {
         g[j] = make_float2(0.f, 0.f);
         if (c4[j] == 0) continue;
-        fp = first[fc + j];
-        // bottomUpNodeConstruction's box (:381-470): offset[j] * L_child + BBcentre_child, the lowest
-        // non-empty child last (bit 0 of the child slot is x)
-        const double cl = bblen[fc + j];
-        const double2 cb = bbc[fc + j];
-        bbox = make_double2(__dadd_rn(__dmul_rn((j & 1) ? -0.5 : 0.5, cl), cb.x),
-                           __dadd_rn(__dmul_rn((j & 2) ? -0.5 : 0.5, cl), cb.y));
         const float2 r = cr2[fc + j];
         g[j] = make_float2(r.x + ((j & 1) ? q : -q), r.y + ((j & 2) ? q : -q));
         sx = fmaf((float)c4[j], g[j].x, sx);
@@ -234,10 +234,12 @@ __global__ void k_bottom_up_p(int l, double minx, double miny, double hl, uint32
         bottom_up_node(l, i, minx, miny, hl, count, first, com64, m0, m2, bbc, bblen, comrel, m0r, m2t, bmax, box);
 }
 
-// levels l0 .. 0 in one block (the coarse levels, a few thousand nodes at
-// most: per-level launches would cost more than their work), a barrier
-// between levels; hl0 is level l0's cell size
-constexpr int kBottomUpCoarseLevel = 6;
+// levels l0 .. 0 in one block (the coarse levels, 341 nodes at most), a
+// barrier between levels; hl0 is level l0's cell size.  A node takes some 15
+// FP64 operations, which one SM issues at 1/64 of the FP32 rate: from level 6
+// on (5,461 nodes) this was 53 us of a step against 31 us with levels 5 and 6
+// launched by themselves.
+constexpr int kBottomUpCoarseLevel = 4;
 __global__ void __launch_bounds__(1024) k_bottom_up_coarse(int l0, double minx, double miny, double hl0,
                                                            uint32_t* __restrict__ count, uint32_t* __restrict__ first,
                                                            double2* __restrict__ com64, double* __restrict__ m0,

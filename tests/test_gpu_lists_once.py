@@ -1,0 +1,45 @@
+"""Interaction lists built in one pass per level (a handle's later builds) against the counted, scanned and filled ones
+(its first build): the same lists, entry for entry.
+
+Candidates within one batch of 128, several, and more than the outcomes kept for the writing (2,048); empty cells;
+every MAC and both precisions of the records; leaf pairs sent to P2P.
+"""
+import ctypes
+
+import numpy as np
+import pytest
+
+from masterthesislucas_gb300 import NBodySolverFMM_MORTON, NBodySolverFMM_SYM_MORTON, Points, datasets
+from masterthesislucas_gb300._lib import check, lib, ptr
+
+pytestmark = pytest.mark.gpu
+
+
+def lists(solver, depth):
+    out = []
+    for level in range(depth + 1):
+        for kind in (0, 1):
+            p, tot = np.zeros((1 << (2 * level)) + 1, np.uint32), ctypes.c_int64(0)
+            check(lib().tc_get_list(solver._h, level, kind, ptr(p), None, ctypes.byref(tot)))
+            idx = np.zeros(max(tot.value, 1), np.uint32)
+            check(lib().tc_get_list(solver._h, level, kind, ptr(p), ptr(idx), ctypes.byref(tot)))
+            assert p[-1] == tot.value
+            out += [p, idx[:tot.value]]
+    return out
+
+
+@pytest.mark.parametrize("depth,theta", [(0, 0.5), (1, 0.5), (4, 0.9), (5, 0.05), (6, 0.5), (9, 0.8)])
+@pytest.mark.parametrize("kind", ["sym", "sym64", "morton", "order_cell", "order_bmax", "order_p2p"])
+def test_one_pass_lists_equal_counted_ones(depth, theta, kind):
+    cls = NBodySolverFMM_MORTON if kind == "morton" else NBodySolverFMM_SYM_MORTON
+    kw = dict(order_cell=dict(order=4, mac="cell"), order_bmax=dict(order=4, mac="bmax"),
+              order_p2p=dict(order=8, mac="bmax", leaf_p2p=64), sym64=dict(precision="fp64")).get(kind, {})
+    pos = datasets.gaussian_mixture(3000, seed=depth).astype(np.float64)
+    s = cls("gravity", tree_depth=depth, theta=theta, softening=1e-3, **kw)
+    pts = Points.from_positions(pos)
+    s.updateTree(pts, pos.min(0), pos.max(0))
+    counted = lists(s, depth)
+    pts = Points.from_positions(pos)
+    s.updateTree(pts, pos.min(0), pos.max(0))
+    for a, b in zip(counted, lists(s, depth)):
+        np.testing.assert_array_equal(a, b)
