@@ -272,9 +272,8 @@ __global__ void __launch_bounds__(128) k_m2m_stream(int l, float hl, const uint3
 // coarse levels: four lanes per node, one per child, summed by two butterfly
 // steps (the fine levels keep one thread per node and its children in turn)
 template <int P>
-__global__ void __launch_bounds__(128) k_m2m_quad(int l, float hl, const uint32_t* __restrict__ count,
-                                                  const float* __restrict__ comrel, float* __restrict__ mu,
-                                                  const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
+__device__ __forceinline__ void m2m_quad(int l, float hl, const uint32_t* count, const float* comrel, float* mu,
+                                         const uint32_t* act, const uint32_t* act_pos, uint32_t block, uint32_t blocks)
 {
     constexpr int K = ncoef(P), KS = kstride(P);
     const uint32_t li = level_index(l), lc = level_index(l + 1);
@@ -282,9 +281,9 @@ __global__ void __launch_bounds__(128) k_m2m_quad(int l, float hl, const uint32_
     const float ih = 1.0f / hl;
     const int j = threadIdx.x & 3;
     const uint32_t k0 = act_pos[li], k1 = act_pos[li + nl];
-    const uint32_t nodes_per_pass = gridDim.x * (blockDim.x >> 2);
+    const uint32_t nodes_per_pass = blocks * (blockDim.x >> 2);
     for (uint32_t base = k0; base < k1; base += nodes_per_pass) {
-        const uint32_t k = base + blockIdx.x * (blockDim.x >> 2) + (threadIdx.x >> 2);
+        const uint32_t k = base + block * (blockDim.x >> 2) + (threadIdx.x >> 2);
         const bool valid = k < k1;
         float acc[K];
 #pragma unroll
@@ -315,6 +314,28 @@ __global__ void __launch_bounds__(128) k_m2m_quad(int l, float hl, const uint32_
             acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], 2);
         }
         if (valid && j == 0) store_coefs<K, KS>(mu + node * KS, acc);
+    }
+}
+
+template <int P>
+__global__ void __launch_bounds__(128) k_m2m_quad(int l, float hl, const uint32_t* __restrict__ count,
+                                                  const float* __restrict__ comrel, float* __restrict__ mu,
+                                                  const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
+{
+    m2m_quad<P>(l, hl, count, comrel, mu, act, act_pos, blockIdx.x, gridDim.x);
+}
+
+// levels first .. 0 (kTopM2m at most: 64 nodes) in one block, a barrier between levels: launched by themselves they are
+// 6 us each of latency
+constexpr int kTopM2m = 3;
+template <int P>
+__global__ void __launch_bounds__(256) k_m2m_top(int first, float box, const uint32_t* __restrict__ count,
+                                                 const float* __restrict__ comrel, float* __restrict__ mu,
+                                                 const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
+{
+    for (int l = first; l >= 0; l--) {
+        m2m_quad<P>(l, box * __int_as_float((127 - l) << 23), count, comrel, mu, act, act_pos, 0u, 1u);
+        __syncthreads();
     }
 }
 
@@ -736,31 +757,54 @@ __global__ void __launch_bounds__(128) k_m2l_mixed_warp(int l, float hl, PotPara
 // ------------------------------------------------------------------ L2L
 // one thread per node of level l >= 1: L_fin = L_own + shift(L_fin(parent))
 template <int P>
-__global__ void __launch_bounds__(128) k_l2l(int l, float hl, const uint32_t* __restrict__ count,
-                                             const float* __restrict__ comrel, float* __restrict__ loc, const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
+__device__ __forceinline__ void l2l_node(int64_t node, uint32_t li, uint32_t lp, float ih, const float* comrel, float* loc)
 {
     constexpr int K = ncoef(P);
+    const int64_t i = node - li;
+    const int64_t par = lp + (i >> 2);
+    const int j = (int)(i & 3);
+    // node COM - parent COM in units of the node's cell size h: the child
+    // cell centre sits (+-1/2, +-1/2) h from the parent's
+    const float ox = ((j & 1) ? 0.5f : -0.5f), oy = ((j & 2) ? 0.5f : -0.5f);
+    const float ddx = ox + (comrel[2 * node] - comrel[2 * par]) * ih;
+    const float ddy = oy + (comrel[2 * node + 1] - comrel[2 * par + 1]) * ih;
+    float in[K], w[K], acc[K];
+    load_coefs<K, kstride(P)>(loc + par * kstride(P), in);
+    halve_by_degree<K>(in);  // parent scale 2h -> child scale h
+    load_coefs<K, kstride(P)>(loc + node * kstride(P), acc);
+    monomials<P>(ddx, ddy, w);
+    shift_down<P>(in, w, acc);
+    store_coefs<K, kstride(P)>(loc + node * kstride(P), acc);
+}
+
+template <int P>
+__global__ void __launch_bounds__(128) k_l2l(int l, float hl, const float* __restrict__ comrel, float* __restrict__ loc,
+                                             const uint32_t* __restrict__ act, const uint32_t* __restrict__ act_pos)
+{
     const uint32_t li = level_index(l), lp = level_index(l - 1);
     const int64_t nl = (int64_t)1 << (2 * l);
     const float ih = 1.0f / hl;
     const uint32_t k1 = act_pos[li + nl];
-    for (uint32_t k = act_pos[li] + blockIdx.x * blockDim.x + threadIdx.x; k < k1; k += gridDim.x * blockDim.x) {
-        const int64_t node = act[k];
-        const int64_t i = node - li;
-        const int64_t par = lp + (i >> 2);
-        const int j = (int)(i & 3);
-        // node COM - parent COM in units of the node's cell size h: the child
-        // cell centre sits (+-1/2, +-1/2) h from the parent's
-        const float ox = ((j & 1) ? 0.5f : -0.5f), oy = ((j & 2) ? 0.5f : -0.5f);
-        const float ddx = ox + (comrel[2 * node] - comrel[2 * par]) * ih;
-        const float ddy = oy + (comrel[2 * node + 1] - comrel[2 * par + 1]) * ih;
-        float in[K], w[K], acc[K];
-        load_coefs<K, kstride(P)>(loc + par * kstride(P), in);
-        halve_by_degree<K>(in);  // parent scale 2h -> child scale h
-        load_coefs<K, kstride(P)>(loc + node * kstride(P), acc);
-        monomials<P>(ddx, ddy, w);
-        shift_down<P>(in, w, acc);
-        store_coefs<K, kstride(P)>(loc + node * kstride(P), acc);
+    for (uint32_t k = act_pos[li] + blockIdx.x * blockDim.x + threadIdx.x; k < k1; k += gridDim.x * blockDim.x)
+        l2l_node<P>(act[k], li, lp, ih, comrel, loc);
+}
+
+// levels 1 .. last (kTopL2l at most: 340 nodes) in one block, a barrier between levels: launched by themselves they
+// are 6 us each of latency
+constexpr int kTopL2l = 4;
+template <int P>
+__global__ void __launch_bounds__(256) k_l2l_top(int last, float box, const float* __restrict__ comrel,
+                                                 float* __restrict__ loc, const uint32_t* __restrict__ act,
+                                                 const uint32_t* __restrict__ act_pos)
+{
+    float hl = box;
+    for (int l = 1; l <= last; l++) {
+        hl *= 0.5f;
+        const uint32_t li = level_index(l), lp = level_index(l - 1), k1 = act_pos[level_index(l + 1)];
+        const float ih = 1.0f / hl;
+        for (uint32_t k = act_pos[li] + threadIdx.x; k < k1; k += blockDim.x)
+            l2l_node<P>(act[k], li, lp, ih, comrel, loc);
+        __syncthreads();
     }
 }
 
@@ -1498,7 +1542,16 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
                                                            act_pos);
         h.launches++;
     }
-    for (int l = 1; l <= dep; l++) {
+    int top_last = 0;
+    if constexpr (ORD < 10) {
+        if (!coarse_done && dep > 0) {
+            top_last = dep < kTopL2l ? dep : kTopL2l;
+            k_l2l_top<ORD><<<1, 256, 0, s>>>(top_last, (float)h.L, comrel, loc, P<uint32_t>(h.act),
+                                             P<uint32_t>(h.act_pos));
+            h.launches++;
+        }
+    }
+    for (int l = top_last + 1; l <= dep; l++) {
         const int64_t nl = (int64_t)1 << (2 * l);
         if (coarse_done && nl <= kM2lWarpLevelNodes) continue;
         if constexpr (ORD < 10) {
@@ -1513,7 +1566,7 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
         if constexpr (ORD >= 10)
             k_l2l_stream<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, loc, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
         else
-            k_l2l<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, loc, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
+            k_l2l<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), comrel, loc, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
         h.launches++;
     }
     // the far field's pair-sum parts, one word per node, summed on its stream while the near field runs
@@ -1581,7 +1634,8 @@ int multipoles_p(Handle& h)
     k_p2m<ORD><<<grid_for((h.n / (kLeafSmall + 1) + 1) * 32, 128), 128, 0, s>>>(
         dep, hl(dep), count, P<uint32_t>(h.first), comrel, P<float>(h.prel), P<uint32_t>(h.bigleaf),
         huge_leaves(h.n), mu);
-    for (int l = dep - 1; l >= 0; l--) {
+    const int top = dep - 1 < kTopM2m ? dep - 1 : kTopM2m;
+    for (int l = dep - 1; l > top; l--) {
         const int64_t nl = (int64_t)1 << (2 * l);
         if (nl <= kM2mQuadLevelNodes)
             k_m2m_quad<ORD><<<grid_for(nl * 4, 128), 128, 0, s>>>(l, hl(l), count, comrel, mu, P<uint32_t>(h.act),
@@ -1591,7 +1645,9 @@ int multipoles_p(Handle& h)
         else
             k_m2m<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, mu, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
     }
-    h.launches += 2 + dep;
+    if (top >= 0)
+        k_m2m_top<ORD><<<1, 256, 0, s>>>(top, (float)h.L, count, comrel, mu, P<uint32_t>(h.act), P<uint32_t>(h.act_pos));
+    h.launches += 2 + dep - top;
     h.mu_stride = kstride(ORD);
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
@@ -1653,11 +1709,13 @@ int far_coarse_p(Handle& h, const PotParams& pp)
     TC_CUDA_TRY(cudaMemsetAsync(zp, 0, h.nnodes * 8, s));
     k_m2l_warp<ORD><<<grid_for((int64_t)level_index(lc + 1) * 32, 128), 128, 0, s>>>(
         1, lc, (float)h.L, pp, level_lists(h), comrel, mu, loc, zp, act, act_pos);
-    for (int l = 1; l <= lc; l++) {
+    const int top_last = lc < kTopL2l ? lc : kTopL2l;
+    k_l2l_top<ORD><<<1, 256, 0, s>>>(top_last, (float)h.L, comrel, loc, act, act_pos);
+    for (int l = top_last + 1; l <= lc; l++) {
         const int64_t nl = (int64_t)1 << (2 * l);
-        k_l2l<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), count, comrel, loc, act, act_pos);
+        k_l2l<ORD><<<grid_for(nl, 128), 128, 0, s>>>(l, hl(l), comrel, loc, act, act_pos);
     }
-    h.launches += 1 + lc;
+    h.launches += 2 + lc - top_last;
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
 }

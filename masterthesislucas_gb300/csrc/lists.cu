@@ -353,21 +353,6 @@ __global__ void __launch_bounds__(128) k_lists_warp(int l, double inv_theta, dou
     }
 }
 
-// The root's lists, and the counters of the levels that k_lists_once builds
-__global__ void k_lists_root(uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ near_ptr,
-                             uint32_t* __restrict__ near_idx, unsigned long long* __restrict__ total, int nlev,
-                             uint32_t* __restrict__ ovf)
-{
-    if ((int)threadIdx.x < nlev) total[threadIdx.x] = threadIdx.x == 0 ? 1ull : 0ull;  // the root is near itself
-    if (threadIdx.x == 0) {
-        nn_ptr[0] = nn_ptr[list_end(1, 0)] = 0;
-        near_ptr[0] = 0;
-        near_ptr[list_end(1, 0)] = 1;
-        near_idx[0] = 0;
-        *ovf = 0;
-    }
-}
-
 // A coarse level in one pass, where the lists' regions are sized beforehand: a
 // warp per non-empty node decides on its candidates as k_lists_warp does,
 // reserves room for both lists by one addition to the level's totals, and
@@ -381,25 +366,45 @@ __global__ void k_lists_root(uint32_t* __restrict__ nn_ptr, uint32_t* __restrict
 constexpr int kOnceWarps = 4;
 constexpr int kOnceBatches = 64;  // outcomes kept; candidates beyond 32 times that are decided again
 
+// where a level's lists go
+struct ListDst {
+    uint32_t *nn_ptr, *nn_idx, *near_ptr, *near_idx;
+    uint32_t nn_cap, near_cap;
+};
+// the records the decisions read (pointers written in the same launch are neither const nor restrict)
 template <typename real>
-__global__ void __launch_bounds__(32 * kOnceWarps)
-    k_lists_once(int l, double inv_theta, double theta, int variant, real hl, const uint32_t* __restrict__ count,
-                 const double2* __restrict__ com64, const real* __restrict__ comrel, const double* __restrict__ bblen,
-                 const uint32_t* __restrict__ pnear_ptr, const uint32_t* __restrict__ pnear_idx, uint32_t pcap,
-                 uint32_t* __restrict__ nn_ptr, uint32_t* __restrict__ nn_idx, uint32_t nn_cap,
-                 uint32_t* __restrict__ near_ptr, uint32_t* __restrict__ near_idx, uint32_t near_cap,
-                 unsigned long long* __restrict__ total, uint32_t* __restrict__ ovf, const uint32_t* __restrict__ act,
-                 const uint32_t* __restrict__ act_pos, const float* __restrict__ bmax, float theta2, uint32_t p2p_cut)
+struct ListSrc {
+    const uint32_t* count;
+    const double2* com64;
+    const real* comrel;
+    const double* bblen;
+    const uint32_t* act;
+    const uint32_t* act_pos;
+    const float* bmax;
+};
+
+// the nodes first, first + stride, ... of level l, one by one, by one warp; parent: the level above
+template <typename real>
+__device__ __forceinline__ void lists_once(int l, double inv_theta, double theta, int variant, real hl,
+                                           const ListSrc<real>& src, const ListDst& parent, const ListDst& dst,
+                                           unsigned long long* total, uint32_t* ovf, float theta2, uint32_t p2p_cut,
+                                           uint2* mask, uint32_t first, uint32_t stride)
 {
-    __shared__ uint2 s_mask[kOnceWarps][kOnceBatches];
+    const uint32_t* count = src.count;
+    const real* comrel = src.comrel;
+    const uint32_t *act = src.act, *act_pos = src.act_pos;
+    const float* bmax = src.bmax;
+    uint32_t *nn_ptr = dst.nn_ptr, *nn_idx = dst.nn_idx, *near_ptr = dst.near_ptr, *near_idx = dst.near_idx;
+    const uint32_t nn_cap = dst.nn_cap, near_cap = dst.near_cap;
+    const uint32_t *pnear_ptr = parent.near_ptr, *pnear_idx = parent.near_idx;
+    const uint32_t pcap = parent.near_cap;
     const uint32_t np = 1u << (2 * (l - 1));
     const uint32_t li = level_index(l);
     const int64_t nl = (int64_t)1 << (2 * l);
     const int lane = threadIdx.x & 31;
-    uint2* mask = s_mask[threadIdx.x >> 5];
     const uint32_t lt = (1u << lane) - 1u;
     const uint32_t k0 = act ? act_pos[li] : 0u, k1 = act ? act_pos[li + nl] : (uint32_t)nl;
-    for (uint32_t k = k0 + blockIdx.x * kOnceWarps + (threadIdx.x >> 5); k < k1; k += gridDim.x * kOnceWarps) {
+    for (uint32_t k = k0 + first; k < k1; k += stride) {
         const int64_t a = act ? (int64_t)act[k] - li : (int64_t)k;
         const uint32_t ca_n = count[li + a];
         if (ca_n == 0) {  // without an active-node list
@@ -409,7 +414,7 @@ __global__ void __launch_bounds__(32 * kOnceWarps)
             }
             continue;
         }
-        const double len = bblen[li + a];
+        const double len = src.bblen[li + a];
         const real thr = (real)((len + len) * inv_theta);
         const real thr2 = thr * thr;
         const int iax = (int)compact16((uint32_t)a), iay = (int)compact16((uint32_t)a >> 1);
@@ -455,7 +460,7 @@ __global__ void __launch_bounds__(32 * kOnceWarps)
                         const real d2 = dx * dx + dy * dy;
                         acc = d2 > thr2 * (real)(1.0 + 1e-5);
                         if (sizeof(real) == 8 || !(acc || d2 < thr2 * (real)(1.0 - 1e-5))) {
-                            const double2 A = com64[li + a], Bc = com64[li + b[u]];
+                            const double2 A = src.com64[li + a], Bc = src.com64[li + b[u]];
                             acc = variant ? mac_accept_m(A, Bc, len, theta) : mac_accept(A, Bc, len, inv_theta);
                         }
                     }
@@ -518,6 +523,48 @@ __global__ void __launch_bounds__(32 * kOnceWarps)
                 pr += __popc(m[u].y);
             }
         }
+    }
+}
+
+template <typename real>
+__global__ void __launch_bounds__(32 * kOnceWarps)
+    k_lists_once(int l, double inv_theta, double theta, int variant, real hl, ListSrc<real> src, ListDst parent,
+                 ListDst dst, unsigned long long* total, uint32_t* ovf, float theta2, uint32_t p2p_cut)
+{
+    __shared__ uint2 s_mask[kOnceWarps][kOnceBatches];
+    lists_once<real>(l, inv_theta, theta, variant, hl, src, parent, dst, total, ovf, theta2, p2p_cut,
+                     s_mask[threadIdx.x >> 5], blockIdx.x * kOnceWarps + (threadIdx.x >> 5), gridDim.x * kOnceWarps);
+}
+
+// The root's lists, the counters of the levels built in one pass, and the
+// first of those levels, up to kTopLevel (85 nodes), in one block: launched by
+// themselves they are 6 us each of latency.
+constexpr int kTopLevel = 3, kTopWarps = 16;
+struct ListTop {
+    ListDst dst[kTopLevel + 1];
+};
+template <typename real>
+__global__ void __launch_bounds__(32 * kTopWarps)
+    k_lists_top(int last, int nlev, double inv_theta, double theta, int variant, real box, ListSrc<real> src,
+                ListTop top, unsigned long long* total, uint32_t* ovf, float theta2, uint32_t p2p_cut_last)
+{
+    __shared__ uint2 s_mask[kTopWarps][kOnceBatches];
+    const uint32_t w = threadIdx.x >> 5;
+    if ((int)threadIdx.x < nlev) total[threadIdx.x] = threadIdx.x == 0 ? 1ull : 0ull;  // the root is near itself
+    if (threadIdx.x == 0) {
+        const ListDst& r = top.dst[0];
+        r.nn_ptr[0] = r.nn_ptr[list_end(1, 0)] = 0;
+        r.near_ptr[0] = 0;
+        r.near_ptr[list_end(1, 0)] = 1;
+        r.near_idx[0] = 0;
+        *ovf = 0;
+    }
+    real hl = box;
+    for (int l = 1; l <= last; l++) {
+        __syncthreads();
+        hl *= real(0.5);
+        lists_once<real>(l, inv_theta, theta, variant, hl, src, top.dst[l - 1], top.dst[l], total + l, ovf, theta2,
+                         l == last ? p2p_cut_last : 0u, s_mask[w], w, kTopWarps);
     }
 }
 
@@ -906,36 +953,50 @@ int build_lists(Handle& h)
         int nonce = 0;
         if (!h.ctrl_on && !adapt)
             while (nonce <= depth && ((int64_t)1 << (2 * nonce)) <= kListsOnceNodes) nonce++;
+        auto dst = [&](int l) {
+            uint32_t* pool = P<uint32_t>(h.idx_pool);
+            return ListDst{ptr + L.nn_ptr_off[l], pool + L.nn_idx_off[l], ptr + L.near_ptr_off[l],
+                           pool + L.near_idx_off[l], L.nn_cap[l], L.near_cap[l]};
+        };
+        const ListSrc<double> src64{P<uint32_t>(h.count), P<double2>(h.com64), P<double>(h.comrel),
+                                    P<double>(h.bblen), nullptr, nullptr, nullptr};
+        const ListSrc<float> src32{P<uint32_t>(h.count), P<double2>(h.com64), P<float>(h.comrel), P<double>(h.bblen),
+                                   act, act_pos, bmax};
+        const bool f64 = h.cfg.precision == TC_PREC_FP64;
+        const float theta2 = (float)(h.cfg.theta * h.cfg.theta);
+        const int top_last = nonce - 1 < kTopLevel ? nonce - 1 : kTopLevel;
         if (nonce) {
-            k_lists_root<<<1, 32, 0, s>>>(ptr + L.nn_ptr_off[0], ptr + L.near_ptr_off[0],
-                                          P<uint32_t>(h.idx_pool) + L.near_idx_off[0], total, depth + 1, ovf);
+            ListTop top{};
+            for (int l = 0; l <= top_last; l++) top.dst[l] = dst(l);
+            if (f64)
+                k_lists_top<double><<<1, 32 * kTopWarps, 0, s>>>(top_last, depth + 1, inv_theta, h.cfg.theta, h.variant,
+                                                                 h.L, src64, top, total, ovf, 0.f, 0u);
+            else
+                k_lists_top<float><<<1, 32 * kTopWarps, 0, s>>>(
+                    top_last, depth + 1, inv_theta, h.cfg.theta, h.variant, (float)h.L, src32, top, total, ovf, theta2,
+                    act && top_last == depth ? h.p2p_cut : 0u);
             h.launches++;
-            if (h.lists_event_level == 0) TC_CUDA_TRY(cudaEventRecord(h.ev_lists, s));
+            // the levels so far are final: work that reads only them may start on another stream
+            if (h.lists_event_level >= 0 && h.lists_event_level <= top_last)
+                TC_CUDA_TRY(cudaEventRecord(h.ev_lists, s));
         } else {
             TC_CUDA_TRY(cudaMemsetAsync(ovf, 0, 4, s));
         }
-        for (int l = nonce ? 1 : 0; l <= depth; l++) {
+        for (int l = nonce ? top_last + 1 : 0; l <= depth; l++) {
             const int64_t nl = (int64_t)1 << (2 * l);
             const uint32_t* pnp = l ? ptr + L.near_ptr_off[l - 1] : nullptr;
             const uint32_t* pni = l ? P<uint32_t>(h.idx_pool) + L.near_idx_off[l - 1] : nullptr;
             const uint32_t pcap = l ? L.near_cap[l - 1] : 0u;
             if (l < nonce) {
                 const double hl = h.L / (double)(1u << l);
-                uint32_t *nnp = ptr + L.nn_ptr_off[l], *nrp = ptr + L.near_ptr_off[l];
-                uint32_t *nni = P<uint32_t>(h.idx_pool) + L.nn_idx_off[l], *nri = P<uint32_t>(h.idx_pool) + L.near_idx_off[l];
-                if (h.cfg.precision == TC_PREC_FP64)
+                if (f64)
                     k_lists_once<double><<<grid_for(nl, kOnceWarps), 32 * kOnceWarps, 0, s>>>(
-                        l, inv_theta, h.cfg.theta, h.variant, hl, P<uint32_t>(h.count), P<double2>(h.com64),
-                        P<double>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnp, nni, L.nn_cap[l], nrp, nri,
-                        L.near_cap[l], total + l, ovf, nullptr, nullptr, nullptr, 0.f, 0u);
+                        l, inv_theta, h.cfg.theta, h.variant, hl, src64, dst(l - 1), dst(l), total + l, ovf, 0.f, 0u);
                 else
                     k_lists_once<float><<<grid_for(nl, kOnceWarps), 32 * kOnceWarps, 0, s>>>(
-                        l, inv_theta, h.cfg.theta, h.variant, (float)hl, P<uint32_t>(h.count), P<double2>(h.com64),
-                        P<float>(h.comrel), P<double>(h.bblen), pnp, pni, pcap, nnp, nni, L.nn_cap[l], nrp, nri,
-                        L.near_cap[l], total + l, ovf, act, act_pos, bmax, (float)(h.cfg.theta * h.cfg.theta),
-                        act && l == depth ? h.p2p_cut : 0u);
+                        l, inv_theta, h.cfg.theta, h.variant, (float)hl, src32, dst(l - 1), dst(l), total + l, ovf,
+                        theta2, act && l == depth ? h.p2p_cut : 0u);
                 h.launches++;
-                // the levels so far are final: work that reads only them may start on another stream
                 if (l == h.lists_event_level) TC_CUDA_TRY(cudaEventRecord(h.ev_lists, s));
                 continue;
             }
