@@ -143,11 +143,13 @@ __global__ void k_bbox(const double2* __restrict__ pos, int64_t n, double* __res
     }
 }
 
-__global__ void k_bbox_init(double* out)
+// err (may be null) is cleared too
+__global__ void k_bbox_init(double* out, uint32_t* err)
 {
     unsigned long long* o = reinterpret_cast<unsigned long long*>(out);
     o[0] = o[1] = 0xFFFFFFFFFFFFFFFFull;
     o[2] = o[3] = 0ull;
+    if (err) *err = 0u;
 }
 
 inline double unkey(unsigned long long k)
@@ -186,7 +188,7 @@ __global__ void k_prel(const double2* __restrict__ pos64, const uint32_t* __rest
 
 int bbox_keys(const double* d_pos, int64_t n, double* d_keys4, uint32_t* d_err, cudaStream_t s)
 {
-    k_bbox_init<<<1, 1, 0, s>>>(d_keys4);
+    k_bbox_init<<<1, 1, 0, s>>>(d_keys4, nullptr);
     k_bbox<<<grid_for(n, 256, sm_count() * 4), 256, 0, s>>>((const double2*)d_pos, n, d_keys4, d_err);
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;
@@ -196,13 +198,13 @@ int device_bbox(Handle& h, const double* d_pos, int64_t n, double mn[2], double 
 {
     int rc;
     if ((rc = ensure(h.err, 64)) || (rc = ensure(h.dtotal, 64))) return rc;
+    // the four keys and the error flag side by side: one copy brings them to the host
     double* o = P<double>(h.dtotal) + 2;
-    TC_CUDA_TRY(cudaMemsetAsync(h.err.p, 0, 4, h.stream));
-    k_bbox_init<<<1, 1, 0, h.stream>>>(o);
-    k_bbox<<<grid_for(n, 256, sm_count() * 4), 256, 0, h.stream>>>((const double2*)d_pos, n, o, P<uint32_t>(h.err));
+    uint32_t* err = reinterpret_cast<uint32_t*>(o + 4);
+    k_bbox_init<<<1, 1, 0, h.stream>>>(o, err);
+    k_bbox<<<grid_for(n, 256, sm_count() * 4), 256, 0, h.stream>>>((const double2*)d_pos, n, o, err);
     h.launches += 2;
-    TC_CUDA_TRY(cudaMemcpyAsync(h.h_words, o, 32, cudaMemcpyDeviceToHost, h.stream));
-    TC_CUDA_TRY(cudaMemcpyAsync(h.h_words + 8, h.err.p, 4, cudaMemcpyDeviceToHost, h.stream));
+    TC_CUDA_TRY(cudaMemcpyAsync(h.h_words, o, 36, cudaMemcpyDeviceToHost, h.stream));
     TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
     if (h.h_words[8]) {
         tc_set_error("positions contain NaN or infinity");

@@ -31,6 +31,7 @@ constexpr uint32_t kLeafBlock = 512;
 // kind's (which the first includes) huge_leaves(n) words on
 constexpr int kBigLeaves = 2;
 __host__ __device__ inline int64_t huge_leaves(int64_t n) { return kBigLeaves + n / (kLeafSmall + 1) + 1; }
+inline int64_t bigleaf_words(int64_t n) { return huge_leaves(n) + n / (kLeafBlock + 1) + 1; }
 
 __host__ __device__ inline uint32_t spread16(uint32_t x)
 {
@@ -137,11 +138,11 @@ int exclusive_scan2_u32(const uint32_t* in0, uint32_t* out0, const uint32_t* in1
                         uint32_t* tmp, cudaStream_t s, uint32_t cap0 = UINT32_MAX, uint32_t cap1 = UINT32_MAX);
 
 // Deterministic FP64 sum of a[0..na) followed by c[0..*nc) (nc a device
-// pointer, may be NULL) into *out (+= when accumulate).  tmp holds
-// sum_tmp_doubles() doubles.
+// pointer, may be NULL, at most cmax) into *out (+= when accumulate).  tmp
+// holds sum_tmp_doubles() doubles.
 int64_t sum_tmp_doubles();
 int sum_f64(const double* a, int64_t na, const double* c, const uint32_t* nc, double* out, int accumulate,
-            double* tmp, cudaStream_t s);
+            double* tmp, cudaStream_t s, int64_t cmax = INT64_MAX / 2);
 
 // Exact bounding box of n device points (x, y doubles) as four order-preserving
 // 64-bit keys (min x, min y, max x, max y) in d_keys4; NaN/inf sets *d_err.

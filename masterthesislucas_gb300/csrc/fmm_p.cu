@@ -1595,7 +1595,7 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
                                                      (reinterpret_cast<uintptr_t>(d_grad) & 15) == 0);
     if ((rc = record(h, 6))) return rc;
     // the pair sum: the far field's total plus the near field's per-item words
-    if ((rc = sum_f64(zfar, 1, P<double>(h.zwork), nz, d_total, 1, P<double>(h.sumtmp) + nsum, s))) return rc;
+    if ((rc = sum_f64(zfar, 1, P<double>(h.zwork), nz, d_total, 1, P<double>(h.sumtmp) + nsum, s, wmax))) return rc;
     // the near field, the L2P and two two-kernel sums; the far field, the item tables and a captured update's coarse
     // levels count themselves
     h.launches += 6;

@@ -120,13 +120,33 @@ __global__ void __launch_bounds__(kMortonThreads)
     if (threadIdx.x == 0) qcount[blockIdx.x] = s_count;
 }
 
+// what the tree build clears and tabulates before its leaves, done by k_morton_exact (as clears and a launch of their
+// own they were four operations): the leaves' first and end indices, the large leaves' counters, the cell centres
+// relative to the box corner, (i + 0.5) h for i < w
+struct TreePrep {
+    uint32_t* first;
+    uint32_t* endp;
+    int64_t nleaf;
+    uint32_t* big;  // kBigLeaves words, may be null
+    double* off;    // may be null
+    int w;
+    double h;
+};
+
 // the queued points of k_morton_fast, in the reference's FP64 arithmetic: block
 // b of the same grid takes region b
 __global__ void __launch_bounds__(kMortonThreads)
     k_morton_exact(const double2* __restrict__ pos, int64_t n, double minx, double miny, double L,
                    const uint32_t* __restrict__ queue, const uint32_t* __restrict__ qcount,
-                   uint32_t* __restrict__ codes)
+                   uint32_t* __restrict__ codes, TreePrep prep)
 {
+    const int64_t id = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, step = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = id; i < prep.nleaf; i += step) {
+        prep.first[i] = 0;
+        prep.endp[i] = 0;
+    }
+    if (prep.big && id < kBigLeaves) prep.big[id] = 0;
+    for (int64_t i = id; prep.off && i < prep.w; i += step) prep.off[i] = ((double)i + 0.5) * prep.h;
     const double nmx = -minx, nmy = -miny;
     const double s65536 = 65536.0 / L;
     const uint32_t* region = queue + (int64_t)blockIdx.x * morton_region(n, gridDim.x);
@@ -158,13 +178,6 @@ __global__ void k_gather_bounds(const uint32_t* __restrict__ codes, const uint32
         if (k == 0 || (depth ? (codes[k - 1] >> shift) : 0u) != leaf) first[li + leaf] = (uint32_t)k;
         if (k == n - 1 || (depth ? (codes[k + 1] >> shift) : 0u) != leaf) endp[li + leaf] = (uint32_t)(k + 1);
     }
-}
-
-// cell centres relative to the box corner, (i + 0.5) h for i < 2^depth
-__global__ void k_cell_offsets(int w, double h, double* __restrict__ off)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < w; i += gridDim.x * blockDim.x)
-        off[i] = ((double)i + 0.5) * h;
 }
 
 // k_gather_bounds for FP32 compute copies: p - centre as (p - min) - (i + 0.5) h
@@ -517,18 +530,27 @@ int build_tree(Handle& h, const double* d_pos, int64_t n, double minx, double mi
     k_morton_fast<<<mgrid, kMortonThreads, 0, s>>>((const double2*)d_pos, n, minx, miny, maxx, maxy,
                                                    (float)(65536.0 / L), P<uint32_t>(h.codes), P<uint32_t>(h.err), mq,
                                                    mcount);
+    const uint32_t li = level_index(depth);
+    const int64_t nleaf = (int64_t)1 << (2 * depth);
+    const double hleaf = L / (double)(1u << depth);
+    const int w = 1 << depth;
+    if (!f64 && (rc = ensure(h.celloff, (size_t)w * 8))) return rc;
+    if (physics && (rc = ensure(h.bigleaf, (size_t)bigleaf_words(n) * 4))) return rc;
+    // (a tree of many more leaves than points is cleared faster by itself than by the points' few blocks)
+    const bool sparse = nleaf > 16 * n;
+    if (sparse) {
+        TC_CUDA_TRY(cudaMemsetAsync(P<uint32_t>(h.count) + li, 0, nleaf * 4, s));
+        TC_CUDA_TRY(cudaMemsetAsync(P<uint32_t>(h.first) + li, 0, nleaf * 4, s));
+    }
+    const TreePrep prep{P<uint32_t>(h.first) + li, P<uint32_t>(h.count) + li, sparse ? 0 : nleaf,
+                        physics ? P<uint32_t>(h.bigleaf) : nullptr, f64 ? nullptr : P<double>(h.celloff), w, hleaf};
     k_morton_exact<<<mgrid, kMortonThreads, 0, s>>>((const double2*)d_pos, n, minx, miny, L, mq, mcount,
-                                                    P<uint32_t>(h.codes));
+                                                    P<uint32_t>(h.codes), prep);
     h.launches += 2;
     TC_CUDA_TRY(cudaGetLastError());
     rc = radix_sort_u32(P<uint32_t>(h.codes), P<uint32_t>(h.perm), P<uint32_t>(h.alt_keys), P<uint32_t>(h.alt_vals), n,
                         P<uint32_t>(h.tmp), s, &h.launches, 0, P<uint32_t>(h.err));
     if (rc || (rc = record(h, 1))) return rc;
-    const uint32_t li = level_index(depth);
-    const int64_t nleaf = (int64_t)1 << (2 * depth);
-    TC_CUDA_TRY(cudaMemsetAsync(P<uint32_t>(h.count) + li, 0, nleaf * 4, s));
-    TC_CUDA_TRY(cudaMemsetAsync(P<uint32_t>(h.first) + li, 0, nleaf * 4, s));
-    const double hleaf = L / (double)(1u << depth);
     if (f64) {
         k_gather_bounds<double><<<grid_for(n, 256), 256, 0, s>>>(P<uint32_t>(h.codes), P<uint32_t>(h.perm),
                                                                  (const double2*)d_pos, n, depth, minx, miny, hleaf,
@@ -539,15 +561,11 @@ int build_tree(Handle& h, const double* d_pos, int64_t n, double minx, double mi
             P<double2>(h.com64), P<double>(h.m0), P<double>(h.m2), P<double2>(h.bbc), P<double>(h.bblen),
             P<double>(h.comrel), P<double>(h.m0r), P<double>(h.m2t));
     } else {
-        const int w = 1 << depth;
-        if ((rc = ensure(h.celloff, (size_t)w * 8))) return rc;
-        k_cell_offsets<<<grid_for(w, 256), 256, 0, s>>>(w, hleaf, P<double>(h.celloff));
         k_gather_bounds_f32<<<grid_for(n, 256), 256, 0, s>>>(P<uint32_t>(h.codes), P<uint32_t>(h.perm),
                                                              (const double2*)d_pos, n, depth, minx, miny,
                                                              P<double>(h.celloff), P<double2>(h.pos64),
                                                              P<float2>(h.prel), P<uint32_t>(h.first),
                                                              P<uint32_t>(h.count));
-        h.launches++;
         if (physics) {
             if ((rc = build_records_p(h, hleaf))) return rc;
         } else {

@@ -270,8 +270,7 @@ int build_records_p(Handle& h, double hleaf)
     const int box = h.centre == TC_CENTRE_BOX;
     int rc;
     const int64_t huge = huge_leaves(h.n);
-    if ((rc = ensure(h.bigleaf, (huge + h.n / (kLeafBlock + 1) + 1) * 4)) || (rc = ensure(h.bmax, h.nnodes * 4))) return rc;
-    TC_CUDA_TRY(cudaMemsetAsync(h.bigleaf.p, 0, 4 * kBigLeaves, s));
+    if ((rc = ensure(h.bmax, h.nnodes * 4))) return rc;
     k_leaf_small_p<<<grid_for(nleaf, 128), 128, 0, s>>>(
         depth, h.minx, h.miny, hleaf, P<uint32_t>(h.count), P<uint32_t>(h.first), P<float2>(h.prel),
         P<double2>(h.com64), P<double>(h.m0), P<double>(h.m2), P<double2>(h.bbc), P<double>(h.bblen),
