@@ -332,78 +332,111 @@ __global__ void __launch_bounds__(kMomThreads)
     }
 }
 
-// bottomUpNodeConstruction (:381-470) for one level l
+// the arrays of the reference's node records and their compute copies
 template <typename real>
-__global__ void k_bottom_up(int l, double minx, double miny, double hl, uint32_t* __restrict__ count,
-                            uint32_t* __restrict__ first, double2* __restrict__ com64, double* __restrict__ m0,
-                            double* __restrict__ m2, double2* __restrict__ bbc, double* __restrict__ bblen,
-                            real* __restrict__ comrel, real* __restrict__ m0r, real* __restrict__ m2t)
+struct NodeRecords {
+    uint32_t* count;
+    uint32_t* first;
+    double2* com64;
+    double* m0;
+    double* m2;
+    double2* bbc;
+    double* bblen;
+    real* comrel;
+    real* m0r;
+    real* m2t;
+};
+
+// bottomUpNodeConstruction (:381-470) for node i of level l
+template <typename real>
+__device__ __forceinline__ void bottom_up_node(int l, int64_t i, double minx, double miny, double hl, const NodeRecords<real>& t)
 {
-    const uint32_t li = level_index(l), lc = level_index(l + 1);
-    const int64_t nl = (int64_t)1 << (2 * l);
-    const double offx[4] = {0.5, -0.5, 0.5, -0.5};
-    const double offy[4] = {0.5, 0.5, -0.5, -0.5};
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nl; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t node = li + i;
-        const int64_t fc = lc + 4 * i;
-        uint32_t cnt = 0, fp = 0;
-        double cx = 0.0, cy = 0.0, M0 = 0.0, bx = 0.0, by = 0.0, len = 0.0;
-        for (int j = 3; j >= 0; j--) {
-            const int64_t ch = fc + j;
-            uint32_t cc = count[ch];
-            if (cc == 0) continue;
-            double clen = bblen[ch];
-            double2 cb = bbc[ch];
-            bx = offx[j] * clen + cb.x;
-            by = offy[j] * clen + cb.y;
-            len = 2.0 * clen;
-            fp = first[ch];
-            cnt += cc;
-            double cm = m0[ch];
-            double2 cc2 = com64[ch];
-            cx += cm * cc2.x;
-            cy += cm * cc2.y;
-            M0 += cm;
-        }
-        uint32_t ix = compact16((uint32_t)i), iy = compact16((uint32_t)i >> 1);
-        double ccx = minx + ((double)ix + 0.5) * hl;
-        double ccy = miny + ((double)iy + 0.5) * hl;
-        count[node] = cnt;
-        first[node] = fp;
-        if (cnt == 0) {
-            com64[node] = make_double2(0.0, 0.0);
-            m0[node] = 0.0;
-            m2[3 * node] = m2[3 * node + 1] = m2[3 * node + 2] = 0.0;
-            bbc[node] = make_double2(0.0, 0.0);
-            bblen[node] = 0.0;
-            write_compute<real>(node, ccx, ccy, 0.0, 0.0, 0.0, 0.0, ccx, ccy, comrel, m0r, m2t);
-            continue;
-        }
-        cx /= M0;
-        cy /= M0;
-        double a = 0.0, b = 0.0, d = 0.0;
-        for (int j = 0; j < 4; j++) {
-            const int64_t ch = fc + j;
-            double cm = m0[ch];
-            if (cm == 0.0) continue;
-            double2 cc2 = com64[ch];
-            double rx = cc2.x - cx, ry = cc2.y - cy;
-            a += rx * rx;
-            b += rx * ry;
-            d += ry * ry;
-            a += m2[3 * ch];
-            b += m2[3 * ch + 1];
-            d += m2[3 * ch + 2];
-        }
-        com64[node] = make_double2(cx, cy);
-        m0[node] = M0;
-        m2[3 * node] = a;
-        m2[3 * node + 1] = b;
-        m2[3 * node + 2] = d;
-        bbc[node] = make_double2(bx, by);
-        bblen[node] = len;
-        write_compute<real>(node, cx, cy, M0, a, b, d, ccx, ccy, comrel, m0r, m2t);
+    const int64_t node = level_index(l) + i;
+    const int64_t fc = level_index(l + 1) + 4 * i;
+    uint32_t cnt = 0;
+    int low = -1;  // the lowest non-empty child, whose box and first particle the reference's loop leaves
+    double cx = 0.0, cy = 0.0, M0 = 0.0;
+    for (int j = 3; j >= 0; j--) {
+        const int64_t ch = fc + j;
+        const uint32_t cc = t.count[ch];
+        if (cc == 0) continue;
+        low = j;
+        cnt += cc;
+        const double cm = t.m0[ch];
+        const double2 cc2 = t.com64[ch];
+        cx += cm * cc2.x;
+        cy += cm * cc2.y;
+        M0 += cm;
     }
+    const uint32_t ix = compact16((uint32_t)i), iy = compact16((uint32_t)i >> 1);
+    const double ccx = minx + ((double)ix + 0.5) * hl;
+    const double ccy = miny + ((double)iy + 0.5) * hl;
+    t.count[node] = cnt;
+    if (cnt == 0) {
+        t.first[node] = 0;
+        t.com64[node] = make_double2(0.0, 0.0);
+        t.m0[node] = 0.0;
+        t.m2[3 * node] = t.m2[3 * node + 1] = t.m2[3 * node + 2] = 0.0;
+        t.bbc[node] = make_double2(0.0, 0.0);
+        t.bblen[node] = 0.0;
+        write_compute<real>(node, ccx, ccy, 0.0, 0.0, 0.0, 0.0, ccx, ccy, t.comrel, t.m0r, t.m2t);
+        return;
+    }
+    const double clen = t.bblen[fc + low];
+    const double2 cb = t.bbc[fc + low];
+    t.first[node] = t.first[fc + low];
+    cx /= M0;
+    cy /= M0;
+    double a = 0.0, b = 0.0, d = 0.0;
+    for (int j = 0; j < 4; j++) {
+        const int64_t ch = fc + j;
+        const double cm = t.m0[ch];
+        if (cm == 0.0) continue;
+        const double2 cc2 = t.com64[ch];
+        const double rx = cc2.x - cx, ry = cc2.y - cy;
+        a += rx * rx;
+        b += rx * ry;
+        d += ry * ry;
+        a += t.m2[3 * ch];
+        b += t.m2[3 * ch + 1];
+        d += t.m2[3 * ch + 2];
+    }
+    t.com64[node] = make_double2(cx, cy);
+    t.m0[node] = M0;
+    t.m2[3 * node] = a;
+    t.m2[3 * node + 1] = b;
+    t.m2[3 * node + 2] = d;
+    t.bbc[node] = make_double2(((low & 1) ? -0.5 : 0.5) * clen + cb.x, ((low & 2) ? -0.5 : 0.5) * clen + cb.y);
+    t.bblen[node] = 2.0 * clen;
+    write_compute<real>(node, cx, cy, M0, a, b, d, ccx, ccy, t.comrel, t.m0r, t.m2t);
+}
+
+template <typename real>
+__global__ void k_bottom_up(int l, double minx, double miny, double hl, NodeRecords<real> t)
+{
+    const int64_t nl = (int64_t)1 << (2 * l);
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nl; i += (int64_t)gridDim.x * blockDim.x)
+        bottom_up_node<real>(l, i, minx, miny, hl, t);
+}
+
+// levels l0 (kTopBottomUp at most: 64 nodes) .. 0 in one block, a barrier between levels: launched by themselves they
+// are 9 us each of latency
+constexpr int kTopBottomUp = 3;
+template <typename real>
+__global__ void __launch_bounds__(64) k_bottom_up_top(int l0, double minx, double miny, double L, NodeRecords<real> t)
+{
+    for (int l = l0; l >= 0; l--) {
+        if ((int64_t)threadIdx.x < ((int64_t)1 << (2 * l)))
+            bottom_up_node<real>(l, threadIdx.x, minx, miny, L / (double)(1u << l), t);
+        __syncthreads();
+    }
+}
+
+template <typename real>
+NodeRecords<real> node_records(Handle& h)
+{
+    return {P<uint32_t>(h.count), P<uint32_t>(h.first), P<double2>(h.com64), P<double>(h.m0), P<double>(h.m2),
+            P<double2>(h.bbc), P<double>(h.bblen), P<real>(h.comrel), P<real>(h.m0r), P<real>(h.m2t)};
 }
 
 }  // namespace
@@ -576,20 +609,21 @@ int build_tree(Handle& h, const double* d_pos, int64_t n, double minx, double mi
         }
     }
     h.launches += physics ? 1 : 2;
-    for (int l = depth - 1; l >= 0 && !physics; l--) {
-        const double hl = L / (double)(1u << l);
-        const int64_t nl = (int64_t)1 << (2 * l);
+    if (!physics && depth > 0) {
+        const int top = depth - 1 < kTopBottomUp ? depth - 1 : kTopBottomUp;
+        for (int l = depth - 1; l > top; l--) {
+            const double hl = L / (double)(1u << l);
+            const int64_t nl = (int64_t)1 << (2 * l);
+            if (f64)
+                k_bottom_up<double><<<grid_for(nl, 64), 64, 0, s>>>(l, minx, miny, hl, node_records<double>(h));
+            else
+                k_bottom_up<float><<<grid_for(nl, 64), 64, 0, s>>>(l, minx, miny, hl, node_records<float>(h));
+        }
         if (f64)
-            k_bottom_up<double><<<grid_for(nl, 128), 128, 0, s>>>(
-                l, minx, miny, hl, P<uint32_t>(h.count), P<uint32_t>(h.first), P<double2>(h.com64), P<double>(h.m0),
-                P<double>(h.m2), P<double2>(h.bbc), P<double>(h.bblen), P<double>(h.comrel), P<double>(h.m0r),
-                P<double>(h.m2t));
+            k_bottom_up_top<double><<<1, 64, 0, s>>>(top, minx, miny, L, node_records<double>(h));
         else
-            k_bottom_up<float><<<grid_for(nl, 128), 128, 0, s>>>(
-                l, minx, miny, hl, P<uint32_t>(h.count), P<uint32_t>(h.first), P<double2>(h.com64), P<double>(h.m0),
-                P<double>(h.m2), P<double2>(h.bbc), P<double>(h.bblen), P<float>(h.comrel), P<float>(h.m0r),
-                P<float>(h.m2t));
-        h.launches++;
+            k_bottom_up_top<float><<<1, 64, 0, s>>>(top, minx, miny, L, node_records<float>(h));
+        h.launches += depth - top;
     }
     TC_CUDA_TRY(cudaGetLastError());
     if (h.cfg.order && (rc = build_active(h))) return rc;
