@@ -40,7 +40,7 @@ constexpr int kGramSmem = kGramStages * (kGramA + kGramB) + 1024;
 constexpr int kGramThreads = 192;  // a producer warp, an MMA warp, four epilogue warps
 constexpr int kCand = 384;         // candidates a row may have
 constexpr int kSelT = 128;         // threads of the selection
-constexpr int kSelGroups = 256;    // groups of a row whose smallest values bound it (more than k)
+constexpr int kSelGroups = 256;    // groups of a row whose smallest values bound it (at most; more than k are needed)
 constexpr float kGramHuge = 1.0e15f;
 
 struct GramStat {
