@@ -650,9 +650,10 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
     // 16-byte loads: every row starts on a 16-byte boundary
     const bool vec = dim % 4 == 0 && (reinterpret_cast<uintptr_t>(d_x) & 15) == 0;
     // the filter on the tensor cores wherever its bound holds: a row's bound needs more than k groups of eight columns
-    // (1,024 points have 128; a row that finds too few goes to k_knn), its inputs 16 KB of shared memory.  It is the faster one over all of that range, k = 90, against k_knn alone:
-    // 1,024 x 4: 91 us, 295; 2,000 x 32: 111, 573; 20,000 x 128: 1.28 ms, 6.70; 20,000 x 784: 3.0, 23.2 (4.6 when
-    // the inputs have low parts); 70,000 x 784: 22.2, 254.9
+    // (1,024 points have 128; a row that finds too few goes to k_knn), its inputs 16 KB of shared memory.  It is the
+    // faster one over all of that range, k = 90, against k_knn alone: 1,024 x 4: 91 us, 295; 2,000 x 32: 111, 573;
+    // 20,000 x 128: 1.28 ms, 6.70; 20,000 x 784: 3.0, 23.2 (4.6 when the inputs have low parts); 70,000 x 784: 22.2,
+    // 254.9
     bool gram = n >= kGramMinN && dim >= kGramMinDim && dim <= kGramMaxDim;
     auto kernel = vec ? k_knn<true> : k_knn<false>;
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
