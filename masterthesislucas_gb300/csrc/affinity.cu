@@ -764,17 +764,15 @@ extern "C" int tc_symmetrize_device(const int32_t* d_idx, const double* d_p, int
     uint32_t* flag = ord + m;
     uint32_t* pos = flag + m;
     uint32_t* tmp = pos + (m + 2) - (m & 1);  // 8-byte aligned; ends before w + words
-    uint32_t* gave_up = w + words;  // set by a sort whose bounded waits ran out
     int rc = TC_OK;
     const double c = 1.0 / (2.0 * (double)n);
     k_sym_entries<<<grid_for(n * k, 256), 256, 0, s>>>(d_idx, d_p, n, k, c, colk, row, v);
     // stable sort by column, then stable by row: rows sorted, columns sorted within a row
     cudaError_t e = cudaMemcpyAsync(k1, colk, (size_t)m * 4, cudaMemcpyDeviceToDevice, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(gave_up, 0, 4, s);
-    if (e == cudaSuccess) rc = radix_sort_u32(k1, p1, ak, av, m, tmp, s, nullptr, 0, gave_up);
+    if (e == cudaSuccess) rc = radix_sort_u32(k1, p1, ak, av, m, tmp, s, nullptr, 0);
     if (e == cudaSuccess && rc == TC_OK) {
         k_gather_u32<<<grid_for(m, 256), 256, 0, s>>>(row, p1, m, k2);
-        rc = radix_sort_u32(k2, p2, ak, av, m, tmp, s, nullptr, 0, gave_up);
+        rc = radix_sort_u32(k2, p2, ak, av, m, tmp, s, nullptr, 0);
     }
     if (e == cudaSuccess && rc == TC_OK) {
         k_sym_flags<<<grid_for(m, 256), 256, 0, s>>>(p1, p2, m, row, colk, ord, flag);
@@ -782,15 +780,10 @@ extern "C" int tc_symmetrize_device(const int32_t* d_idx, const double* d_p, int
     }
     if (e == cudaSuccess && rc == TC_OK) {
         k_sym_write<<<grid_for(m, 256), 256, 0, s>>>(ord, flag, pos, m, n, row, colk, v, d_row_ptr, d_col, d_val);
-        uint32_t cnt = 0, bad = 0;
+        uint32_t cnt = 0;
         e = cudaMemcpyAsync(&cnt, pos + m, 4, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&bad, gave_up, 4, cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
         *nnz = cnt;
-        if (e == cudaSuccess && bad) {
-            tc_set_error("tc_symmetrize_device: a bounded wait of the sort gave up");
-            rc = TC_ERR_TIMEOUT;
-        }
     }
     const cudaError_t ef = cudaFreeAsync(buf, s);
     if (e != cudaSuccess) return tc_cuda_fail(e, "tc_symmetrize_device");

@@ -854,8 +854,7 @@ int bh_path_solve(int kernel, double softening, int max_children, double theta, 
     double2* psort = (double2*)b_psort.p;
     float4* prel = (float4*)b_prel.p;
     k_path_keys<<<grid_for(n, 128), 128, 0, s>>>(pos, n, bbox, keys);
-    if ((rc = radix_sort_u32(keys, perm, (uint32_t*)b_akeys.p, (uint32_t*)b_avals.p, n, (uint32_t*)b_tmp.p, s, nullptr,
-                             0, err)))
+    if ((rc = radix_sort_u32(keys, perm, (uint32_t*)b_akeys.p, (uint32_t*)b_avals.p, n, (uint32_t*)b_tmp.p, s, nullptr)))
         return rc;
     k_path_leaves<<<grid_for(n, 128), 128, 0, s>>>(keys, perm, n, (uint32_t)max_children, pos, bbox,
                                                    (uint8_t*)b_depth.p, (uint32_t*)b_nbegin.p, order, psort, prel,
@@ -866,7 +865,7 @@ int bh_path_solve(int kernel, double softening, int max_children, double theta, 
     TC_CUDA_TRY(cudaMemcpyAsync(flags, err, 8, cudaMemcpyDeviceToHost, s));
     TC_CUDA_TRY(cudaStreamSynchronize(s));
     if (flags[0]) {
-        tc_set_error("tc_bh_solve_device: positions contain NaN or infinity, or the sort gave up");
+        tc_set_error("tc_bh_solve_device: positions contain NaN or infinity");
         return TC_ERR_INVALID;
     }
     if (flags[1] || total > cap) return 1;

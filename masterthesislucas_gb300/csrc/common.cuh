@@ -163,10 +163,9 @@ __host__ __device__ inline double bbox_unkey(unsigned long long k)
 // with 32-bit values; the result lands in keys/vals, alt_* are scratch of n
 // entries each.  With an odd number of passes the input keys must be in
 // alt_keys instead of keys.  The values are the input positions (iota).  tmp
-// holds radix_tmp_words(n) u32, 8-byte aligned.  *err (device, may be null) gets
-// bit 0 when a bounded wait inside gave up; the result is then incomplete.
+// holds radix_tmp_words(n) u32, 8-byte aligned.
 int64_t radix_tmp_words(int64_t n);
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, uint32_t* alt_keys, uint32_t* alt_vals, int64_t n,
-                   uint32_t* tmp, cudaStream_t s, int* launches, int lo_bit = 0, uint32_t* err = nullptr);
+                   uint32_t* tmp, cudaStream_t s, int* launches, int lo_bit = 0);
 
 }  // namespace tc

@@ -413,10 +413,9 @@ __global__ void k_pm_gather(const double2* __restrict__ pos, int64_t n, const ui
     }
 }
 
-// a sort whose bounded waits gave up leaves no sum to report
-__global__ void k_pm_total(double* __restrict__ total, double n, const uint32_t* __restrict__ gave_up)
+__global__ void k_pm_total(double* __restrict__ total, double n)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) *total = *gave_up ? NAN : *total - n;
+    if (threadIdx.x == 0 && blockIdx.x == 0) *total = *total - n;
 }
 
 // ------------------------------------------------------------------ per-device workspace
@@ -583,10 +582,8 @@ static int pm_solve(int n_interp, double cell_size, int min_intervals, const dou
     k_pm_points<<<grid_for(n, 256), 256, 0, s>>>(pos2, n, g, P<uint32_t>(w.key), P<double>(w.wx), P<double>(w.wy));
     TC_CUDA_TRY(cudaMemcpyAsync(w.skey.p, w.key.p, n * 4, cudaMemcpyDeviceToDevice, s));
     int launches = 0;
-    uint32_t* gave_up = P<uint32_t>(w.mm) + 8;
-    TC_CUDA_TRY(cudaMemsetAsync(gave_up, 0, 4, s));
     if ((rc = radix_sort_u32(P<uint32_t>(w.skey), P<uint32_t>(w.perm), P<uint32_t>(w.alt_k), P<uint32_t>(w.alt_v), n,
-                             P<uint32_t>(w.sort_tmp), s, &launches, 0, gave_up)))
+                             P<uint32_t>(w.sort_tmp), s, &launches)))
         return rc;
     TC_CUDA_TRY(cudaMemsetAsync(w.bstart.p, 0, nbox * 4, s));
     TC_CUDA_TRY(cudaMemsetAsync(w.bend.p, 0, nbox * 4, s));
@@ -621,7 +618,7 @@ static int pm_solve(int n_interp, double cell_size, int min_intervals, const dou
     k_pm_gather<<<grid_for(n, 128), 128, 0, s>>>(pos2, n, P<uint32_t>(w.skey), P<uint32_t>(w.perm), P<double>(w.wx), P<double>(w.wy),
                                                 P<double>(w.fout), g, d_grad, P<double>(w.zterm));
     if ((rc = sum_f64(P<double>(w.zterm), n, nullptr, nullptr, d_total, 0, P<double>(w.sumtmp), s))) return rc;
-    k_pm_total<<<1, 32, 0, s>>>(d_total, (double)n, gave_up);
+    k_pm_total<<<1, 32, 0, s>>>(d_total, (double)n);
     TC_CUDA_TRY(cudaGetLastError());
     if (host) {
         TC_CUDA_TRY(cudaMemcpyAsync(h_grad, d_grad, n * 16, cudaMemcpyDeviceToHost, s));

@@ -33,10 +33,14 @@ constexpr int kMaxPass = 4;
 constexpr int64_t kLookBack = (int64_t)1 << 20;
 // a tile's word for a digit: 0 not there yet, the tile's own count, or the count of all tiles up to it (top two bits)
 enum : uint32_t { kOwn = 1u << 30, kUpTo = 2u << 30, kValue = (1u << 30) - 1u };
-constexpr uint32_t kMaxPolls = 1u << 22;  // about a second or two
+// looks at words that are not there yet, before a block counts for itself (about a second or two)
+#ifndef TC_SORT_POLLS
+#define TC_SORT_POLLS (1u << 22)
+#endif
+constexpr uint32_t kMaxPolls = TC_SORT_POLLS;
 
-// scratch: [0, 4) tile tickets of the passes, [4] set when a wait gave up, [8, 8 + 4 * 256) digit counts of the
-// passes, then per pass nb * 256 words of the tiles
+// scratch: [0, 4) tile tickets of the passes, [8, 8 + 4 * 256) digit counts of the passes, then per pass nb * 256
+// words of the tiles
 constexpr int kHistAt = 8, kTilesAt = kHistAt + kMaxPass * RADIX;
 
 __global__ void __launch_bounds__(RT) k_radix_hist(const uint32_t* __restrict__ keys, int64_t n, int lo_bit, int npass,
@@ -94,8 +98,7 @@ template <bool kLook>
 __global__ void __launch_bounds__(RT) k_radix_pass(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                                    uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int64_t n,
                                                    int shift, int pass, uint32_t* scratch,
-                                                   const uint32_t* __restrict__ offs, int nblocks, int iota_vals,
-                                                   uint32_t* __restrict__ err)
+                                                   const uint32_t* __restrict__ offs, int nblocks, int iota_vals)
 {
     __shared__ uint32_t s_keys[RTILE];
     __shared__ uint32_t s_vals[RTILE];
@@ -179,11 +182,24 @@ __global__ void __launch_bounds__(RT) k_radix_pass(const uint32_t* __restrict__ 
         t -= u;
         if (u == 0) lost = ++polls > kMaxPolls;
     }
-    if (kLook && tile > 0) tiles[tile * RADIX + tid] = ((before + run) & kValue) | kUpTo;
-    if (lost && err) atomicOr(err, 1u);
+    auto publish = [&] {
+        if (kLook && tile > 0) tiles[tile * RADIX + tid] = (before + run) | kUpTo;
+    };
+    if (!lost) publish();
     s_gofs[tid] = digit_start + before - st;  // global position of tile slot j of digit d: s_gofs[d] + j (mod 2^32)
-    // after a lost wait nothing is written: the offsets are not known
-    if (__syncthreads_or(lost)) return;
+    // a wait that ran out: the block counts the digits of the tiles before it itself (up to kLookBack keys, which no
+    // block of this pass writes), so the sort is complete however long a tile stalls
+    if (__syncthreads_or(lost)) {
+        uint32_t* cnt = s_wh[0];
+        cnt[tid] = 0;
+        __syncthreads();
+        for (int64_t p = tid; p < tile * RTILE; p += RT) atomicAdd(&cnt[(kin[p] >> shift) & 255u], 1u);
+        __syncthreads();
+        before = cnt[tid];
+        publish();
+        s_gofs[tid] = digit_start + before - st;
+        __syncthreads();
+    }
     const int64_t rem = n - tile * RTILE;
     const int cnt = rem < RTILE ? (int)rem : RTILE;
 #pragma unroll
@@ -192,10 +208,8 @@ __global__ void __launch_bounds__(RT) k_radix_pass(const uint32_t* __restrict__ 
         if (j < cnt) {
             const uint32_t k = s_keys[j];
             const uint32_t o = s_gofs[(k >> shift) & 255u] + (uint32_t)j;
-            if (o < n) {  // always, unless a tile before gave up
-                kout[o] = k;
-                vout[o] = s_vals[j];
-            }
+            kout[o] = k;
+            vout[o] = s_vals[j];
         }
     }
 }
@@ -286,7 +300,7 @@ int64_t radix_tmp_words(int64_t n)
 }
 
 int radix_sort_u32(uint32_t* keys, uint32_t* vals, uint32_t* alt_keys, uint32_t* alt_vals, int64_t n,
-                   uint32_t* tmp, cudaStream_t s, int* launches, int lo_bit, uint32_t* err)
+                   uint32_t* tmp, cudaStream_t s, int* launches, int lo_bit)
 {
     if (n <= 0) return TC_OK;
     const int npass = (32 - lo_bit + 7) / 8;
@@ -317,12 +331,12 @@ int radix_sort_u32(uint32_t* keys, uint32_t* vals, uint32_t* alt_keys, uint32_t*
     for (int pass = 0; pass < npass; pass++) {
         const int shift = lo_bit + 8 * pass;
         if (look) {
-            k_radix_pass<true><<<nb, RT, 0, s>>>(ki, vi, ko, vo, n, shift, pass, tmp, nullptr, nb, pass == 0, err);
+            k_radix_pass<true><<<nb, RT, 0, s>>>(ki, vi, ko, vo, n, shift, pass, tmp, nullptr, nb, pass == 0);
         } else {
             k_radix_tile_hist<<<nb, RT, 0, s>>>(ki, n, shift, hist, nb);
             int rc = exclusive_scan_u32(hist, offs, h, stmp, s);
             if (rc) return rc;
-            k_radix_pass<false><<<nb, RT, 0, s>>>(ki, vi, ko, vo, n, shift, pass, nullptr, offs, nb, pass == 0, err);
+            k_radix_pass<false><<<nb, RT, 0, s>>>(ki, vi, ko, vo, n, shift, pass, nullptr, offs, nb, pass == 0);
         }
         if (launches) *launches += look ? 1 : 4;
         uint32_t* t = ki; ki = ko; ko = t;

@@ -582,7 +582,7 @@ int build_tree(Handle& h, const double* d_pos, int64_t n, double minx, double mi
     h.launches += 2;
     TC_CUDA_TRY(cudaGetLastError());
     rc = radix_sort_u32(P<uint32_t>(h.codes), P<uint32_t>(h.perm), P<uint32_t>(h.alt_keys), P<uint32_t>(h.alt_vals), n,
-                        P<uint32_t>(h.tmp), s, &h.launches, 0, P<uint32_t>(h.err));
+                        P<uint32_t>(h.tmp), s, &h.launches, 0);
     if (rc || (rc = record(h, 1))) return rc;
     if (f64) {
         k_gather_bounds<double><<<grid_for(n, 256), 256, 0, s>>>(P<uint32_t>(h.codes), P<uint32_t>(h.perm),
