@@ -483,6 +483,7 @@ __device__ __forceinline__ void lists_once(int l, double inv_theta, double theta
                 if (lane == 0 && c0 / 32 + u < kOnceBatches) mask[c0 / 32 + u] = m[u];
             }
         }
+        __syncwarp();  // lane 0's outcomes, read back below
         unsigned long long at = 0;
         if (lane == 0) at = atomicAdd(total, (unsigned long long)nn << 32 | nr);
         at = __shfl_sync(0xffffffffu, at, 0);

@@ -43,3 +43,17 @@ def test_one_pass_lists_equal_counted_ones(depth, theta, kind):
     s.updateTree(pts, pos.min(0), pos.max(0))
     for a, b in zip(counted, lists(s, depth)):
         np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("depth", [4, 5, 6])
+def test_kept_outcomes_of_several_batches(depth):
+    """Every pair near (256, 1,024 and 4,096 candidates a node, of which 2,048 are kept), built over and over."""
+    pos = np.random.default_rng(depth).random((4000, 2))
+    mn, mx = np.zeros(2), np.ones(2)
+    s = NBodySolverFMM_SYM_MORTON("tsne", tree_depth=depth, theta=0.01, order=4)
+    s.updateTree(Points.from_positions(pos), mn, mx)
+    counted = lists(s, depth)
+    for _ in range(10):
+        s.updateTree(Points.from_positions(pos), mn, mx)
+        for a, b in zip(counted, lists(s, depth)):
+            np.testing.assert_array_equal(a, b)
