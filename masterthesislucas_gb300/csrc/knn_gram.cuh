@@ -230,22 +230,25 @@ __global__ void __launch_bounds__(kGramThreads, 1)
             for (int c = 0; c < kGramCols / 32; c++) {
                 float g[32];
                 tmem_ld32(trow + 32 * c, g);
-                if (row >= n) continue;
-                float mn[8];
+                if (row < n) {
+                    float mn[8];
 #pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const float4 v = sj[8 * c + j];
-                    const float4 a = make_float4(fmaf(-2.f, g[4 * j], si + v.x), fmaf(-2.f, g[4 * j + 1], si + v.y),
-                                                 fmaf(-2.f, g[4 * j + 2], si + v.z), fmaf(-2.f, g[4 * j + 3], si + v.w));
-                    float* oc = o + (32 * c + 4 * j) * kGramRows;
-                    oc[0] = a.x;
-                    oc[kGramRows] = a.y;
-                    oc[2 * kGramRows] = a.z;
-                    oc[3 * kGramRows] = a.w;
-                    mn[j] = fminf(fminf(a.x, a.y), fminf(a.z, a.w));
+                    for (int j = 0; j < 8; j++) {
+                        const float4 v = sj[8 * c + j];
+                        const float4 a =
+                            make_float4(fmaf(-2.f, g[4 * j], si + v.x), fmaf(-2.f, g[4 * j + 1], si + v.y),
+                                        fmaf(-2.f, g[4 * j + 2], si + v.z), fmaf(-2.f, g[4 * j + 3], si + v.w));
+                        float* oc = o + (32 * c + 4 * j) * kGramRows;
+                        oc[0] = a.x;
+                        oc[kGramRows] = a.y;
+                        oc[2 * kGramRows] = a.z;
+                        oc[3 * kGramRows] = a.w;
+                        mn[j] = fminf(fminf(a.x, a.y), fminf(a.z, a.w));
+                    }
+                    om[2 * c] = make_float4(mn[0], mn[1], mn[2], mn[3]);
+                    om[2 * c + 1] = make_float4(mn[4], mn[5], mn[6], mn[7]);
                 }
-                om[2 * c] = make_float4(mn[0], mn[1], mn[2], mn[3]);
-                om[2 * c + 1] = make_float4(mn[4], mn[5], mn[6], mn[7]);
+                __syncwarp();  // the next load takes the warp as a whole, also where its rows end
             }
             tc_fence_before();
             __syncwarp();

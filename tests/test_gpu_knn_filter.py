@@ -35,6 +35,13 @@ def test_sizes(n, dim, k, values):
     check(x.astype(np.float32), k)
 
 
+@pytest.mark.parametrize("n", [1024 + 1, 1024 + 31, 1024 + 33, 1024 + 97, 2048 + 127])
+def test_last_rows_within_a_warp(n):
+    """The last row block ends inside a warp's 32 rows, several column tiles each."""
+    rng = np.random.default_rng(n)
+    check(rng.normal(size=(n, 40)).astype(np.float32), 30)
+
+
 @pytest.mark.parametrize("kind", ["equal", "some_equal", "offset", "tiny", "huge", "outlier", "infinite"])
 def test_rows_that_the_filter_gives_up_on(kind):
     rng = np.random.default_rng(5)
