@@ -153,9 +153,9 @@ struct KGrav {
     }
 };
 
-// Padding source: far enough that its force factor underflows to zero and its
-// pair term (~1e-18 gravity, ~1e-36 t-SNE) is absorbed by any real sum.
-constexpr float kFarAway = 1.0e18f;
+// Padding source: its squared distance is infinite to any sink, so that its pair
+// term and its force factor are zero whatever the units of the positions.
+constexpr float kFarAway = 1.0e38f;
 
 // One sink (px, py) against its share of the staged sources: g lanes share a
 // sink, lane r of the group takes 16-byte slots r, r + g, r + 2g, ... (two

@@ -81,3 +81,21 @@ def test_reference_order_dense_leaves(kernel, theta, precision, symmetric):
     else:
         assert np.median(err) <= 2e-6 and err.max() <= 1e-3
         assert total == pytest.approx(ref["total"], rel=2e-6)
+
+
+@pytest.mark.parametrize("order", [None, 8])
+@pytest.mark.parametrize("scale", [1.0, 1e12])
+@pytest.mark.parametrize("sizes", [(1, 1, 1, 1), (3, 33, 0, 1)])
+def test_pair_sum_in_any_units(order, scale, sizes):
+    """Sources that fill up a group's share add nothing to the pair sum, also where every term is 1e-12."""
+    pos, mn, mx = cells(sizes, 1)
+    pos *= scale
+    s = NBodySolverFMM_SYM_MORTON("gravity", tree_depth=1, theta=0.1, softening=0.1 * scale,
+                                  **({} if order is None else {"order": order}))  # all pairs direct
+    pts = Points.from_positions(pos)
+    s.updateTree(pts, mn, mx * scale)
+    total = s.solveNbody(0.0, pts)
+    _, ref_total = oracle.naive(pts.position, kernel=oracle.KERNEL_GRAVITY, eps=0.1 * scale)
+    # up to 38 terms a sink, each to 3 2^-23 (coordinates, square, reciprocal root), the sum to 38 2^-24; the order-p
+    # path adds and takes out the sink's own term, up to ten times the others'
+    assert total == pytest.approx(ref_total, rel=(3 * 2 + 38) * 10 * 2.0 ** -24, abs=0.0)
