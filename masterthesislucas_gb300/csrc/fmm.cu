@@ -178,13 +178,14 @@ __device__ inline bool pn_pass(double2 x, double2 com, double len, double inv_th
 // only where the FP32 squared distance is too close to the threshold: at the
 // threshold R is off by at most a few 2^-24 (thr + 3 h), which moves |R|^2 by
 // less than an eighth of the band.  FP64 runs at 1/64 of the FP32 rate, and
-// the test is made for every particle and partner leaf.
+// the test is made for every particle and partner leaf.  (Squares below 1e-30
+// are left to FP64: near the end of the normal range the band says nothing.)
 template <typename real, typename F>
 __device__ __forceinline__ bool pn_pass_fast(real Rx, real Ry, real thr, real h, F&& exact)
 {
     if (sizeof(real) == 4) {
-        const real diff = (Rx * Rx + Ry * Ry) - thr * thr;
-        if (fabs(diff) > real(3.2e-6) * thr * (thr + real(3) * h)) return diff > real(0);
+        const real thr2 = thr * thr, diff = (Rx * Rx + Ry * Ry) - thr2;
+        if (thr2 > real(1e-30) && fabs(diff) > real(3.2e-6) * thr * (thr + real(3) * h)) return diff > real(0);
     }
     return exact();
 }

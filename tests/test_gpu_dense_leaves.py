@@ -99,3 +99,20 @@ def test_pair_sum_in_any_units(order, scale, sizes):
     # up to 38 terms a sink, each to 3 2^-23 (coordinates, square, reciprocal root), the sum to 38 2^-24; the order-p
     # path adds and takes out the sink's own term, up to ten times the others'
     assert total == pytest.approx(ref_total, rel=(3 * 2 + 38) * 10 * 2.0 ** -24, abs=0.0)
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("theta", [0.4, 0.5, 0.7])
+@pytest.mark.parametrize("scale", [1.0, 2.0 ** -61, 2.0 ** -62, 2.0 ** -63, 2.0 ** -75, 2.0 ** 61])
+def test_point_criteria_at_any_scale(symmetric, theta, scale):
+    """The points' criteria decide as in FP64 where their FP32 squares leave the normal range."""
+    pos, mn, mx = cells(REF_SIZES, 2)
+    cls = NBodySolverFMM_SYM_MORTON if symmetric else NBodySolverFMM_MORTON
+    counts = []
+    for p, c in (("fp64", 1.0), ("fp32", scale)):
+        s = cls("tsne", tree_depth=2, theta=theta, precision=p)
+        pts = Points.from_positions(pos * c)
+        s.updateTree(pts, mn * c, mx * c)
+        s.solveNbody(0.0, pts)
+        counts.append(s.counters())
+    assert counts[0] == counts[1]
