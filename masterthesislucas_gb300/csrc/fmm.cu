@@ -180,15 +180,21 @@ __device__ inline bool pn_pass(double2 x, double2 com, double len, double inv_th
 // less than an eighth of the band.  FP64 runs at 1/64 of the FP32 rate, and
 // the test is made for every particle and partner leaf.  (Squares below 1e-30
 // are left to FP64: near the end of the normal range the band says nothing.)
-template <typename real, typename F>
-__device__ __forceinline__ bool pn_pass_fast(real Rx, real Ry, real thr, real h, F&& exact)
-{
-    if (sizeof(real) == 4) {
-        const real thr2 = thr * thr, diff = (Rx * Rx + Ry * Ry) - thr2;
-        if (thr2 > real(1e-30) && fabs(diff) > real(3.2e-6) * thr * (thr + real(3) * h)) return diff > real(0);
+template <typename real>
+struct PointMac {
+    real thr2, band;
+    __device__ PointMac(real thr, real h)
+        : thr2(thr * thr), band(thr2 > real(1e-30) ? real(3.2e-6) * thr * (thr + real(3) * h) : real(INFINITY)) {}
+    template <typename F>
+    __device__ __forceinline__ bool pass(real Rx, real Ry, F&& exact) const
+    {
+        if (sizeof(real) == 4) {
+            const real diff = (Rx * Rx + Ry * Ry) - thr2;
+            if (fabs(diff) > band) return diff > real(0);
+        }
+        return exact();
     }
-    return exact();
-}
+};
 
 constexpr int kLeafWarps = 4;
 
@@ -249,7 +255,8 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
     const int dep = geo.depth;
     const uint32_t li = level_index(dep);
     const int64_t nl = (int64_t)1 << (2 * dep);
-    const real h = (real)geo.h_leaf, thr = (real)(geo.h_leaf * geo.inv_theta);
+    const real h = (real)geo.h_leaf;
+    const PointMac<real> mac((real)(geo.h_leaf * geo.inv_theta), h);
     const double inv_theta = geo.inv_theta;
     // leaf si by nv warps, this one taking runs v, v + nv, ... of its partners' points; C and z are the warp's sums
     auto leaf = [&](int64_t si, int v, int nv, real (&C)[L_NCOEF], double& z) {
@@ -303,7 +310,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
                 // R' = com_S - x_t
                 const real Rx = T.ox + (csx - prel[2 * t]);
                 const real Ry = T.oy + (csy - prel[2 * t + 1]);
-                if (!pn_pass_fast(Rx, Ry, thr, h, [&] { return pn_pass(pos64[t], com64[S], bblen[S], inv_theta); }))
+                if (!mac.pass(Rx, Ry, [&] { return pn_pass(pos64[t], com64[S], bblen[S], inv_theta); }))
                     continue;
                 real D1, D2, D3, tt;
                 ker.far(Rx * Rx + Ry * Ry, D1, D2, D3, tt);
@@ -447,7 +454,8 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
     const int dep = geo.depth;
     const uint32_t li = level_index(dep);
     const int64_t nl = (int64_t)1 << (2 * dep);
-    const real h = (real)geo.h_leaf, thr = (real)(geo.h_leaf * geo.inv_theta);
+    const real h = (real)geo.h_leaf;
+    const PointMac<real> mac((real)(geo.h_leaf * geo.inv_theta), h);
     const double inv_theta = geo.inv_theta;
     const uint32_t nwork = chunk_ptr[nl];
     for (uint32_t wi = blockIdx.x; wi < nwork; wi += gridDim.x) {
@@ -509,7 +517,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
                     // symmetric: S is the first node of the pair and each sink is tested against T; non-symmetric:
                     // every sink tests every partner T, S itself included (traverseBHMP, :199-232)
                     const real Rx = (T.ox + px) - comrel[2 * nT], Ry = (T.oy + py) - comrel[2 * nT + 1];
-                    const bool pass = act && pn_pass_fast(Rx, Ry, thr, h, [&] {
+                    const bool pass = act && mac.pass(Rx, Ry, [&] {
                         return geo.variant ? pn_pass_m(pos64[s], com64[nT], bblen[nT], geo.theta)
                                            : pn_pass(pos64[s], com64[nT], bblen[nT], inv_theta);
                     });
@@ -539,7 +547,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
                         const real tx = prel[2 * t], ty = prel[2 * t + 1];
                         // only the points of T that fail the MAC against S interact with the sinks directly
                         if (tested)
-                            take = !pn_pass_fast(T.ox + (csx - tx), T.oy + (csy - ty), thr, h, [&] {
+                            take = !mac.pass(T.ox + (csx - tx), T.oy + (csy - ty), [&] {
                                 return pn_pass(pos64[t], com64[S], bblen[S], inv_theta);
                             });
                         x = tx - T.ox;
