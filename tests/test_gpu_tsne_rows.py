@@ -28,3 +28,27 @@ def test_rows_of_every_length(n, precision):
     tol = 5e-5 if precision == "fp32" else 1e-10
     assert np.abs(grad - gref).max() <= tol * np.abs(gref).max()
     assert np.abs(got - yn).max() <= tol * (np.abs(gref).max() * n / 15.0 + np.abs(y).max())
+
+
+@pytest.mark.parametrize("offset", [0.0] + [2.0 ** e + 0.4 * 2.0 ** (e - 23) for e in (20, 30, 40)])
+def test_attraction_far_from_the_origin(offset):
+    """FP32 products of differences that are as good as the FP64 positions', wherever the embedding lies."""
+    rng = np.random.default_rng(7)
+    n = 300
+    y = offset + rng.normal(0, 1, (n, 2))
+    lengths = np.resize([0, 1, 2, 90, 200], n)
+    row_ptr = np.concatenate([[0], np.cumsum(lengths)]).astype(np.uint32)
+    rows, col = np.repeat(np.arange(n), lengths), rng.integers(0, n, row_ptr[-1]).astype(np.uint32)
+    val = 1e6 * rng.random(len(col)) / len(col)  # an attraction far above the repulsion
+    t = TSNE(row_ptr, col, val, y, min_theta=0.5, max_theta=0.5, max_children=16)
+    t.time_step()
+    _, _, grad = t.embedding()
+    _, gref, _ = oracle.tsne_step(y, y, row_ptr, col, val, theta=0.5)
+    d = y[col] - y[rows]
+    w = 16.0 * val / (1.0 + (d * d).sum(1))
+    attr, size = np.zeros((n, 2)), np.zeros((n, 2))
+    np.add.at(attr, rows, w[:, None] * d)
+    np.add.at(size, rows, w[:, None] * np.abs(d).max(1)[:, None])
+    # a term is off by at most 12 roundings of 2^-24 (differences, square, reciprocal to two ulps, products), a sum of
+    # 200 terms by 7 in a lane and 5 across; the repulsion (positions and cells rounded at the offset) by a tenth
+    assert np.all(np.abs(grad - gref) <= 24 * 2.0 ** -24 * size + 0.1 * np.abs(gref - attr).max())
