@@ -25,7 +25,7 @@
 // points being neighbours in key order.  65,536 points of a Gaussian mixture,
 // leaves of 16, theta 0.5: 190 launches and 10 host round trips before,
 // 32 and one now; traversal 3,546 us with a thread per point in input order and
-// the MAC in FP64, 206 us now.  Deeper trees take the level-synchronous
+// the MAC in FP64, 234 us now.  Deeper trees take the level-synchronous
 // build and the per-point traversal, which know no depth limit.
 //
 // The multipole variant (NBodySolverBHMP + QuadTreeMultiPole,
@@ -371,7 +371,7 @@ struct PathNodes {
     double2* com;
     double* m64;        // multipole variant
     Quad* quad;
-    float4* rec;        // [2 i]: COM relative to the root corner, high and low parts (x, y, x, y);
+    float4* rec;        // [2 i]: COM relative to the root corner, high and low parts (x, y, x, y; path_split);
                         // [2 i + 1]: l / theta, mass, leaf flag, unused
     float4* mom;        // multipole variant, FP32: quadrupole / mass
 };
@@ -384,6 +384,47 @@ __device__ __forceinline__ void root_box(const double* keys, double2& lo, double
     const double ld = (ax < ay) ? ay : ax;  // std::max(a, b)
     lo = make_double2(lx, ly);
     hix = lx + ld + 0.0001;
+}
+
+// the points' extent is at most 2^E
+__device__ __forceinline__ int root_exponent(const double* keys)
+{
+    const unsigned long long* k = reinterpret_cast<const unsigned long long*>(keys);
+    return ilogb(fmax(fmax(bbox_unkey(k[2]) - bbox_unkey(k[0]), bbox_unkey(k[3]) - bbox_unkey(k[1])), 1e-300)) + 1;
+}
+
+// Coordinates relative to the root corner as FP32 pairs: highs on the grid 2^(E - 24), so that the difference of two is
+// exact, and the rest.
+struct PathSplit {
+    double snap;  // adding and subtracting it rounds to the grid
+    __device__ explicit PathSplit(const double* keys) : snap(ldexp(1.5, root_exponent(keys) + 28)) {}
+    __device__ __forceinline__ float4 operator()(double x, double y) const
+    {
+        const double hx = (x + snap) - snap, hy = (y + snap) - snap;
+        return make_float4((float)hx, (float)hy, (float)(x - hx), (float)(y - hy));
+    }
+};
+
+// a - b of two such pairs, rounded once, and the square of its length with the roundings' share (10 of the traversal's
+// 234 us)
+struct PathDiff {
+    float2 d;
+    float d2;
+    __device__ __forceinline__ PathDiff(float4 a, float4 b)
+    {
+        const float sx = a.x - b.x, sy = a.y - b.y;  // exact
+        const float tx = a.z - b.z, ty = a.w - b.w;  // at most the grid's step, as a non-zero s is at least
+        d = make_float2(sx + tx, sy + ty);
+        const float rx = tx - (d.x - sx), ry = ty - (d.y - sy);
+        const float c = d.x * rx + d.y * ry;
+        d2 = d.x * d.x + (d.y * d.y + (c + c));
+    }
+};
+
+// squared distances below this are taken in FP64: the pairs' own error, 2^(E - 48), could exceed 2^-28 of the distance
+__device__ __forceinline__ float path_close2(const double* keys)
+{
+    return fmaxf((float)ldexp(1.0, 2 * (root_exponent(keys) - 20)), 1e-30f);
 }
 
 // one level down: the box of quadrant qd (quadtree.h:104-134; the upper y edge is never read)
@@ -447,6 +488,7 @@ __global__ void k_path_leaves(const uint32_t* __restrict__ keys, const uint32_t*
     double2 rlo;
     double rhi;
     root_box(bbox, rlo, rhi);
+    const PathSplit split(bbox);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t key = keys[i];
         uint32_t a = 0, b = n;
@@ -470,9 +512,7 @@ __global__ void k_path_leaves(const uint32_t* __restrict__ keys, const uint32_t*
         const double2 p = pos[o];
         order[r] = o;
         psort[r] = p;
-        const double rx = p.x - rlo.x, ry = p.y - rlo.y;
-        const float hx = (float)rx, hy = (float)ry;
-        prel[r] = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
+        prel[r] = split(p.x - rlo.x, p.y - rlo.y);
     }
 }
 
@@ -525,6 +565,7 @@ __global__ void k_path_moments(uint32_t total, PathNodes t, const double2* __res
     double2 rlo;
     double rhi;
     root_box(bbox, rlo, rhi);
+    const PathSplit split(bbox);
     for (uint32_t leaf = blockIdx.x * blockDim.x + threadIdx.x; leaf < total; leaf += gridDim.x * blockDim.x) {
         if (t.nchild[leaf] != 0) continue;
         uint32_t nd = leaf;
@@ -605,9 +646,7 @@ __global__ void k_path_moments(uint32_t total, PathNodes t, const double2* __res
                 t.comf[nd] = make_float2((float)cx, (float)cy);
                 m = (double)tm;
             }
-            const double rx = cx - rlo.x, ry = cy - rlo.y;
-            const float hx = (float)rx, hy = (float)ry;
-            t.rec[2 * (size_t)nd] = make_float4(hx, hy, (float)(rx - (double)hx), (float)(ry - (double)hy));
+            t.rec[2 * (size_t)nd] = split(cx - rlo.x, cy - rlo.y);
             t.rec[2 * (size_t)nd + 1] = make_float4((float)(t.len[nd] / theta), (float)m, nch <= 1 ? 1.0f : 0.0f, 0.0f);
             if (nd == 0) break;
             const uint32_t par = t.parent[nd];
@@ -619,26 +658,23 @@ __global__ void k_path_moments(uint32_t total, PathNodes t, const double2* __res
     }
 }
 
-// a - b of two (high, low) pairs of coordinates relative to the root corner, to FP32 accuracy whatever they cancel
-__device__ __forceinline__ float2 split_sub(float4 a, float4 b)
-{
-    return make_float2((a.x - b.x) + (a.z - b.z), (a.y - b.y) + (a.w - b.w));
-}
-
 constexpr int kPathThreads = 64;  // few points leave few warps: small blocks spread them evenly
 
 // traverseBH, a warp per 32 points neighbouring in tree order: the warp walks the nodes depth first, going into a
 // node while any of its points opens it; a point that has accepted a node sits out the subtree.  Each point meets
 // its nodes in the order it would alone.  The MAC is decided in FP32 and, within 1e-5 of its threshold (the FP32
-// square is good to 3e-7), as the reference decides it.
+// square is good to 2e-7), as the reference decides it.  FP32 forces take offset and square as good as the FP64 ones
+// rounded (path_close2: the FP64 ones where the pairs are too few bits).
 template <typename real, typename K, bool MP>
 __global__ void __launch_bounds__(kPathThreads) k_path_traverse(K ker, uint32_t n, uint32_t total, PathNodes t,
                                                        const double2* __restrict__ psort,
                                                        const float4* __restrict__ prel,
-                                                       const uint32_t* __restrict__ order, double theta,
+                                                       const uint32_t* __restrict__ order,
+                                                       const double* __restrict__ bbox, double theta,
                                                        double* __restrict__ grad, double* __restrict__ zrow)
 {
     constexpr bool kF32 = sizeof(real) == 4;
+    const float close2 = path_close2(bbox);
     for (uint32_t p0 = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; p0 < n; p0 += gridDim.x * blockDim.x) {
         const uint32_t i = p0 + (threadIdx.x & 31);
         const bool valid = i < n;
@@ -650,17 +686,19 @@ __global__ void __launch_bounds__(kPathThreads) k_path_traverse(K ker, uint32_t 
             const float4 c = t.rec[2 * (size_t)nd], r = t.rec[2 * (size_t)nd + 1];
             const uint32_t skip = t.skip[nd];
             const bool on = nd >= resume;
-            const float2 d = split_sub(xs, c);
-            const float d2 = d.x * d.x + d.y * d.y, thr2 = r.x * r.x;
+            const PathDiff diff(xs, c);
+            const float2 d = diff.d;
+            const float d2 = diff.d2, thr2 = r.x * r.x;
+            const bool apart = d2 >= close2;  // false for NaN (highs that overflow)
             bool pass = d2 > thr2;
-            if (on && !(fabsf(d2 - thr2) > 1e-5f * thr2 && thr2 > 1e-30f)) {
+            if (on && !(fabsf(d2 - thr2) > 1e-5f * thr2 && thr2 > 1e-30f && apart)) {
                 const double2 com = t.com[nd];
                 const double ex = x.x - com.x, ey = x.y - com.y;
                 pass = t.len[nd] / sqrt(ex * ex + ey * ey) < theta;
             }
             if (on && pass) {
                 resume = skip;
-                if constexpr (kF32) {
+                if (kF32 && apart) {
                     if constexpr (MP) {
                         const float4 q = t.mom[nd];
                         real D1, D2, D3, tt;
@@ -710,15 +748,29 @@ __global__ void __launch_bounds__(kPathThreads) k_path_traverse(K ker, uint32_t 
                 if constexpr (kF32) {
                     // summed by themselves first: fewer roundings against the running sums
                     real lx = 0, ly = 0, lz = 0;
+                    bool near = false;
 #pragma unroll 4
                     for (uint32_t j = t.start[nd]; j < e; j++) {
-                        const float2 f = split_sub(xs, prel[j]);
+                        const PathDiff f(xs, prel[j]);
                         real D1, tt;
-                        ker.near(f.x * f.x + f.y * f.y, D1, tt);
-                        const bool use = open && j != i;
+                        ker.near(f.d2, D1, tt);
+                        const bool ok = f.d2 >= close2, use = open && ok;
+                        near |= open && !ok && j != i;
                         lz += use ? tt : real(0);
-                        lx += use ? D1 * f.x : real(0);
-                        ly += use ? D1 * f.y : real(0);
+                        lx += use ? D1 * f.d.x : real(0);
+                        ly += use ? D1 * f.d.y : real(0);
+                    }
+                    if (near) {
+                        for (uint32_t j = t.start[nd]; j < e; j++) {
+                            if (PathDiff(xs, prel[j]).d2 >= close2 || j == i) continue;
+                            const double2 q = psort[j];
+                            const double ex = x.x - q.x, ey = x.y - q.y;
+                            real D1, tt;
+                            ker.near((real)(ex * ex + ey * ey), D1, tt);
+                            lz += tt;
+                            lx += D1 * (real)ex;
+                            ly += D1 * (real)ey;
+                        }
                     }
                     gx += lx;
                     gy += ly;
@@ -893,8 +945,8 @@ int bh_path_solve(int kernel, double softening, int max_children, double theta, 
         k_path_moments<false><<<grid_for(total, 128), 128, 0, s>>>(total, t, psort, bbox, theta);
     bh_dispatch(kernel, softening, precision, mp, [&](auto ker, auto zero, auto m) {
         k_path_traverse<decltype(zero), decltype(ker), decltype(m)::value>
-            <<<grid_for(n, kPathThreads, 1 << 20), kPathThreads, 0, s>>>(ker, n, total, t, psort, prel, order, theta,
-                                                                        d_grad_xy, zrow);
+            <<<grid_for(n, kPathThreads, 1 << 20), kPathThreads, 0, s>>>(ker, n, total, t, psort, prel, order, bbox,
+                                                                        theta, d_grad_xy, zrow);
     });
     TC_CUDA_TRY(cudaGetLastError());
     return TC_OK;

@@ -54,3 +54,24 @@ def test_tree_shapes(kernel, shape, n, leaf, multipole):
     err = rel_err(g32, ref)
     assert np.median(err) < 1e-5 and err.max() < 1e-3
     assert total32 == pytest.approx(ref_total, rel=1e-5)
+
+
+@pytest.mark.parametrize("multipole", [False, True])
+@pytest.mark.parametrize("kernel", ["gravity", "tsne"])
+@pytest.mark.parametrize("shift", [10, 20, 30, 40])
+def test_close_pairs_in_fp32(shift, kernel, multipole):
+    """Points with a partner 2^-shift away: the FP32 forces of the FP64 offsets."""
+    rng = np.random.default_rng(shift)
+    a = rng.random((64, 2))
+    pos = np.concatenate([a, a + 2.0 ** -shift * (1.0 + rng.random((64, 2)))])
+    kw = dict(kernel=kernel, softening=0.0 if kernel == "gravity" else EPS, max_children=16, theta=0.5,
+              multipole=multipole)
+    ref, ref_total = barnes_hut(pos, precision="fp64", **kw)
+    g, total = barnes_hut(pos, **kw)
+    # sums of up to 128 terms; a term takes some 16 roundings of 2^-24 (offset, square, reciprocal root to two ulps and
+    # its cube), an accepted node's quadrupole twice that
+    d = pos[:, None, :] - pos[None, :, :]
+    r2 = (d * d).sum(-1) + np.eye(len(pos)) * 1e300
+    size = (np.sqrt(r2) * ((1.0 + r2) ** -2 if kernel == "tsne" else r2 ** -1.5)).sum(1)
+    assert np.all(np.linalg.norm(g - ref, axis=1) <= (32 + 40) * 2.0 ** -24 * size)
+    assert total == pytest.approx(ref_total, rel=2e-6)
