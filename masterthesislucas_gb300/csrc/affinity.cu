@@ -143,6 +143,7 @@ constexpr int kStageFloats = 2 * kKC * (kQ + kC);
 constexpr int kTileFloats = kQ * (kC + kTilePad);
 // the distance tile takes the staging buffers' place once its last chunk is used
 constexpr size_t kKnnStatic = 4 * (size_t)(kStageFloats > kTileFloats ? kStageFloats : kTileFloats);
+constexpr size_t kKnnMaxDyn = kKnnStatic + (size_t)kQ * kMaxK * 8;
 typedef unsigned long long u64;
 
 // packed FP32 operations that keep subnormals, as fmaf does
@@ -340,6 +341,7 @@ __global__ void __launch_bounds__(kKnnT, 2)
 // its query block's units): an entry's place is its own index plus, for every
 // other list, the number of that list's smaller entries.
 constexpr int kMergeWarps = 4;
+constexpr size_t kMergeMaxDyn = (size_t)kMergeWarps * (kListRuns + 2) * kMaxK * 8;
 __global__ void __launch_bounds__(32 * kMergeWarps)
     k_knn_merge(const u64* __restrict__ part, int64_t n, int k, int64_t ctiles, int64_t qblocks, int64_t max_runs,
                 const uint32_t* __restrict__ list, const uint32_t* __restrict__ nlist, int maxseg,
@@ -679,11 +681,17 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
     int64_t maxseg = gram ? kListRuns + 2 : runs / qblocks + 2;
     if (maxseg > ctiles) maxseg = ctiles;
     const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
+    if (mdyn > kMergeMaxDyn) {  // up to 400 runs (200 multiprocessors) a row lies in at most 16
+        tc_set_error("tc_knn_device: more runs a query block than the merge holds");
+        cudaFreeAsync(buf_p, s);
+        return TC_ERR_STATE;
+    }
     u64* part = reinterpret_cast<u64*>(buf);
     uint32_t *list = nullptr, *nlist = nullptr;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
+    // the limits of every k, not this one's: calls of other threads set them too
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKnnMaxDyn);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mdyn);
+        e = cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMergeMaxDyn);
     if (gram && e == cudaSuccess) {
         uint8_t *hi = buf + b_part, *lo = hi + b_half;
         float* norm = reinterpret_cast<float*>(lo + b_half);

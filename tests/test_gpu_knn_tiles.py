@@ -28,3 +28,34 @@ def test_knn_matches_the_oracle(n, dim, k, offset, ties):
     rd, ri = oracle.knn(x, k)
     np.testing.assert_array_equal(d.cpu().numpy(), rd)
     np.testing.assert_array_equal(i.cpu().numpy(), ri)
+
+
+def test_threads_of_different_k():
+    """Calls of different list lengths from several threads at once, each on its own stream."""
+    import threading
+
+    import torch
+    rng = np.random.default_rng(11)
+    x = torch.from_numpy(rng.random((1500, 24)).astype(np.float32)).cuda()
+    refs = {k: oracle.knn(x.cpu().numpy(), k) for k in (1, 100, 128)}
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(k):
+        try:
+            st = torch.cuda.Stream()
+            for _ in range(60):
+                with torch.cuda.stream(st):
+                    d, i = affinity.knn(x, k, stream=st.cuda_stream)
+                st.synchronize()
+                np.testing.assert_array_equal(i.cpu().numpy(), refs[k][1])
+                np.testing.assert_array_equal(d.cpu().numpy(), refs[k][0])
+        except BaseException as e:  # reported by the main thread
+            errors.append((k, e))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in refs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
