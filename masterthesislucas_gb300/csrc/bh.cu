@@ -968,7 +968,7 @@ int bh_level_solve(int kernel, double softening, int max_children, double theta,
         (rc = dalloc<uint32_t>(b_nodeof2, n)) || (rc = dalloc<uint8_t>(b_q, n)) ||
         (rc = dalloc<uint32_t>(b_ind, (size_t)4 * n)) || (rc = dalloc<uint32_t>(b_pre, (size_t)4 * (n + 1))) ||
         (rc = dalloc<uint32_t>(b_nck, cap)) || (rc = dalloc<uint32_t>(b_coff, cap + 1)) ||
-        (rc = dalloc<uint32_t>(b_tmp, (size_t)scan_tmp_words((int64_t)cap + n) + 16)))
+        (rc = dalloc<uint32_t>(b_tmp, (size_t)(scan_tmp_words((int64_t)cap + n) + 2 * scan_tmp_words(n)))))
         return rc;
     DevBuf b_m64, b_quad;
     if (mp && ((rc = dalloc<double>(b_m64, cap)) || (rc = dalloc<Quad>(b_quad, cap)))) return rc;
@@ -991,8 +991,9 @@ int bh_level_solve(int kernel, double softening, int max_children, double theta,
         const uint32_t lb = level_begin.back(), le = level_end.back();
         k_bh_classify<<<grid, 256, 0, s>>>((const double2*)d_pos_xy, order, node_of, n, lb, le, t, max_children, ind,
                                            (uint8_t*)b_q.p);
-        for (int k = 0; k < 4; k++)
-            if ((rc = exclusive_scan_u32(ind + (size_t)k * n, pre + (size_t)k * (n + 1), n, (uint32_t*)b_tmp.p, s)))
+        for (int k = 0; k < 4; k += 2)
+            if ((rc = exclusive_scan2_u32(ind + (size_t)k * n, pre + (size_t)k * (n + 1), ind + (size_t)(k + 1) * n,
+                                          pre + (size_t)(k + 1) * (n + 1), n, (uint32_t*)b_tmp.p, s)))
                 return rc;
         k_bh_nchild<<<grid_for(le - lb, 256), 256, 0, s>>>(lb, le, t, max_children, pre, n, (uint32_t*)b_nck.p);
         if ((rc = exclusive_scan_u32((uint32_t*)b_nck.p, (uint32_t*)b_coff.p, le - lb, (uint32_t*)b_tmp.p, s))) return rc;
