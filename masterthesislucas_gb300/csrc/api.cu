@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <functional>
+#include <mutex>
 #include <new>
 #include <vector>
 
@@ -63,6 +64,51 @@ void release(Buf& b)
     if (b.p) cudaFree(b.p);
     b.p = nullptr;
     b.bytes = 0;
+}
+
+namespace {
+constexpr int kStageDevices = 64, kStageKept = 4;
+constexpr size_t kStageBytes = 64ull << 20;
+std::mutex g_stage_mu;
+HostStage::Slot g_stage[kStageDevices][kStageKept];
+int g_stage_n[kStageDevices];
+}  // namespace
+
+int HostStage::open(size_t in_bytes, size_t out_bytes)
+{
+    int dev = 0;
+    TC_CUDA_TRY(cudaGetDevice(&dev));
+    dev_ = dev;
+    if (dev < kStageDevices) {
+        std::lock_guard<std::mutex> g(g_stage_mu);
+        if (g_stage_n[dev] > 0) {
+            slot_ = g_stage[dev][--g_stage_n[dev]];
+            g_stage[dev][g_stage_n[dev]] = Slot();
+        }
+    }
+    if (!slot_.stream) TC_CUDA_TRY(cudaStreamCreateWithFlags(&slot_.stream, cudaStreamNonBlocking));
+    const int rc = ensure(slot_.in, in_bytes);
+    return rc ? rc : ensure(slot_.out, out_bytes);
+}
+
+HostStage::~HostStage()
+{
+    if (!slot_.stream) return;
+    cudaStreamSynchronize(slot_.stream);
+    if (slot_.in.bytes + slot_.out.bytes > kStageBytes) {
+        release(slot_.in);
+        release(slot_.out);
+    }
+    if (dev_ < kStageDevices) {
+        std::lock_guard<std::mutex> g(g_stage_mu);
+        if (g_stage_n[dev_] < kStageKept) {
+            g_stage[dev_][g_stage_n[dev_]++] = slot_;
+            return;
+        }
+    }
+    release(slot_.in);
+    release(slot_.out);
+    cudaStreamDestroy(slot_.stream);
 }
 
 int record_on(Handle& h, int i, cudaStream_t s)

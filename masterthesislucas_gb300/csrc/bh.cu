@@ -805,7 +805,6 @@ __global__ void __launch_bounds__(kPathThreads) k_path_traverse(K ker, uint32_t 
 struct BHWork {
     std::mutex mu;
     Buf slot[64];
-    cudaStream_t stream = nullptr;  // of the host entry points
     cudaEvent_t done = nullptr;  // recorded after each call's last use of the workspace
     bool recorded = false;
 };
@@ -1035,16 +1034,20 @@ int bh_level_solve(int kernel, double softening, int max_children, double theta,
     return TC_OK;
 }
 
-// host: the three arrays are host memory and pass through the workspace, on its stream
-int bh_solve_impl(int kernel, double softening, int max_children, double theta, int precision,
-                  const double* d_pos_xy, int64_t n64, double* d_grad_xy, double* d_total, void* stream, bool mp,
-                  bool host = false)
+int bh_check(int kernel, int max_children, double theta, const double* pos_xy, int64_t n, const double* grad_xy)
 {
-    if (!d_pos_xy || !d_grad_xy || n64 <= 0 || n64 > (1 << 30) || max_children <= 0 || !(theta > 0.0) ||
+    if (!pos_xy || !grad_xy || n <= 0 || n > (1 << 30) || max_children <= 0 || !(theta > 0.0) ||
         (kernel != TC_KERNEL_TSNE && kernel != TC_KERNEL_GRAVITY)) {
         tc_set_error("tc_bh_solve_device: invalid arguments");
         return TC_ERR_INVALID;
     }
+    return TC_OK;
+}
+
+int bh_solve_impl(int kernel, double softening, int max_children, double theta, int precision,
+                  const double* d_pos_xy, int64_t n64, double* d_grad_xy, double* d_total, void* stream, bool mp)
+{
+    if (const int bad = bh_check(kernel, max_children, theta, d_pos_xy, n64, d_grad_xy)) return bad;
     const uint32_t n = (uint32_t)n64;
     cudaStream_t s = (cudaStream_t)stream;
     int rc = TC_OK;
@@ -1053,8 +1056,6 @@ int bh_solve_impl(int kernel, double softening, int max_children, double theta, 
     BHWork& work = bh_work(dev);
     std::lock_guard<std::mutex> work_lock(work.mu);
     if (!work.done) TC_CUDA_TRY(cudaEventCreateWithFlags(&work.done, cudaEventDisableTiming));
-    if (host && !work.stream) TC_CUDA_TRY(cudaStreamCreateWithFlags(&work.stream, cudaStreamNonBlocking));
-    if (host) s = work.stream;
     // the previous call's kernels (possibly on another stream) finish first
     if (work.recorded) TC_CUDA_TRY(cudaStreamWaitEvent(s, work.done, 0));
     WorkRelease release_on_exit{work, s};
@@ -1069,18 +1070,6 @@ int bh_solve_impl(int kernel, double softening, int max_children, double theta, 
     const double* bbox = (const double*)b_bbox.p;
     double* zrow = (double*)b_zrow.p;
     uint32_t* err = (uint32_t*)b_err.p;
-    double *h_grad = nullptr, *h_total = nullptr;
-    if (host) {
-        DevBuf b_pos, b_grad, b_tot;
-        if ((rc = dalloc<double2>(b_pos, n)) || (rc = dalloc<double2>(b_grad, n)) || (rc = dalloc<double>(b_tot, 1)))
-            return rc;
-        TC_CUDA_TRY(cudaMemcpyAsync(b_pos.p, d_pos_xy, (size_t)n * 16, cudaMemcpyHostToDevice, s));
-        h_grad = d_grad_xy;
-        h_total = d_total;
-        d_pos_xy = (const double*)b_pos.p;
-        d_grad_xy = (double*)b_grad.p;
-        d_total = (double*)b_tot.p;
-    }
     TC_CUDA_TRY(cudaMemsetAsync(b_err.p, 0, 16, s));
     if ((rc = bbox_keys(d_pos_xy, n64, (double*)b_bbox.p, (uint32_t*)b_err.p, s))) return rc;
     const int first_slot = g_slot;
@@ -1097,12 +1086,6 @@ int bh_solve_impl(int kernel, double softening, int max_children, double theta, 
         return rc;
     uint32_t herr = 0;
     TC_CUDA_TRY(cudaMemcpyAsync(&herr, b_err.p, 4, cudaMemcpyDeviceToHost, s));
-    if (h_grad) {
-        // written only by a solve that succeeded
-        TC_CUDA_TRY(cudaStreamSynchronize(s));
-        if (!herr) TC_CUDA_TRY(cudaMemcpyAsync(h_grad, d_grad_xy, (size_t)n * 16, cudaMemcpyDeviceToHost, s));
-        if (!herr && h_total) TC_CUDA_TRY(cudaMemcpyAsync(h_total, d_total, 8, cudaMemcpyDeviceToHost, s));
-    }
     TC_CUDA_TRY(cudaStreamSynchronize(s));
     if (herr) {
         tc_set_error("tc_bh_solve_device: traversal stack exhausted");
@@ -1137,8 +1120,19 @@ static int bh_solve_host(int kernel, double softening, int max_children, double 
         tc_set_error("tc_bh_solve: invalid arguments");
         return TC_ERR_INVALID;
     }
-    return tc::bh_solve_impl(kernel, softening, max_children, theta, precision, pos_xy, n, grad_xy, total, nullptr, mp,
-                             true);
+    int rc = tc::bh_check(kernel, max_children, theta, pos_xy, n, grad_xy);
+    if (rc) return rc;
+    tc::HostStage st;
+    if ((rc = st.open((size_t)n * 16, (size_t)n * 16 + 64))) return rc;
+    double *d_total = static_cast<double*>(st.out()), *d_grad = d_total + 8;
+    TC_CUDA_TRY(cudaMemcpyAsync(st.in(), pos_xy, (size_t)n * 16, cudaMemcpyHostToDevice, st.stream()));
+    rc = tc::bh_solve_impl(kernel, softening, max_children, theta, precision, static_cast<const double*>(st.in()), n,
+                           d_grad, d_total, st.stream(), mp);
+    if (rc) return rc;
+    TC_CUDA_TRY(cudaMemcpyAsync(grad_xy, d_grad, (size_t)n * 16, cudaMemcpyDeviceToHost, st.stream()));
+    if (total) TC_CUDA_TRY(cudaMemcpyAsync(total, d_total, 8, cudaMemcpyDeviceToHost, st.stream()));
+    TC_CUDA_TRY(cudaStreamSynchronize(st.stream()));
+    return TC_OK;
 }
 
 extern "C" int tc_bh_solve(int kernel, double softening, int max_children, double theta, int precision,

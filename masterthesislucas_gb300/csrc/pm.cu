@@ -422,9 +422,8 @@ __global__ void k_pm_total(double* __restrict__ total, double n)
 struct PmWork {
     std::mutex mu;
     Buf vals_max, vals_min, mm, key, skey, perm, alt_k, alt_v, sort_tmp, wx, wy, bstart, bend, xt, kt, kf, fin, fw,
-        fout, zterm, sumtmp, host_pos, host_out;
+        fout, zterm, sumtmp;
     std::map<int, cufftHandle> d2z1, d2z4, z2d4;  // plans by FFT size
-    cudaStream_t stream = nullptr;  // of the host entry point
     cudaEvent_t done = nullptr;
     bool recorded = false;
 };
@@ -479,16 +478,22 @@ int pm_plan(CufftApi& api, std::map<int, cufftHandle>& cache, int nf, cufftType 
 
 }  // namespace
 
-// host: positions, gradient and total are host memory and pass through the workspace, on its stream
-static int pm_solve(int n_interp, double cell_size, int min_intervals, const double* d_pos, int64_t n, double* d_grad,
-                    double* d_total, cudaStream_t s, bool host)
+static int pm_check(int n_interp, double cell_size, int min_intervals, const double* pos, int64_t n, const double* grad,
+                    const double* total)
 {
-    if (n <= 0 || n > (int64_t)UINT32_MAX / 2 || !d_pos || !d_grad || !d_total || n_interp < 1 ||
+    if (n <= 0 || n > (int64_t)UINT32_MAX / 2 || !pos || !grad || !total || n_interp < 1 ||
         n_interp > kPmMaxInterp || !(cell_size > 0.0) || min_intervals < 1) {
         tc_set_error("particle mesh: invalid arguments (1 <= n_interp <= %d, cell_size > 0, min_intervals >= 1)",
                      kPmMaxInterp);
         return TC_ERR_INVALID;
     }
+    return TC_OK;
+}
+
+int pm_solve_device(int n_interp, double cell_size, int min_intervals, const double* d_pos, int64_t n, double* d_grad,
+                    double* d_total, cudaStream_t s)
+{
+    if (const int bad = pm_check(n_interp, cell_size, min_intervals, d_pos, n, d_grad, d_total)) return bad;
     CufftApi& api = cufft();
     if (!api.ok) {
         tc_set_error("particle mesh: libcufft could not be loaded");
@@ -499,19 +504,9 @@ static int pm_solve(int n_interp, double cell_size, int min_intervals, const dou
     PmWork& w = pm_work(dev);
     std::lock_guard<std::mutex> lock(w.mu);
     if (!w.done) TC_CUDA_TRY(cudaEventCreateWithFlags(&w.done, cudaEventDisableTiming));
-    if (host && !w.stream) TC_CUDA_TRY(cudaStreamCreateWithFlags(&w.stream, cudaStreamNonBlocking));
-    if (host) s = w.stream;
     if (w.recorded) TC_CUDA_TRY(cudaStreamWaitEvent(s, w.done, 0));
     PmRelease release_on_exit{w, s};
     int rc;
-    double *h_grad = d_grad, *h_total = d_total;
-    if (host) {
-        if ((rc = ensure(w.host_pos, n * 16)) || (rc = ensure(w.host_out, n * 16 + 64))) return rc;
-        TC_CUDA_TRY(cudaMemcpyAsync(w.host_pos.p, d_pos, n * 16, cudaMemcpyHostToDevice, s));
-        d_pos = P<double>(w.host_pos);
-        d_total = P<double>(w.host_out);
-        d_grad = d_total + 8;
-    }
     // 1. min / max over the interleaved coordinates
     const int64_t m = 2 * n, nc = (m + kPmChunk - 1) / kPmChunk;
     if ((rc = ensure(w.vals_max, nc * 16 + 64)) || (rc = ensure(w.vals_min, nc * 8 + 64)) ||
@@ -620,18 +615,7 @@ static int pm_solve(int n_interp, double cell_size, int min_intervals, const dou
     if ((rc = sum_f64(P<double>(w.zterm), n, nullptr, nullptr, d_total, 0, P<double>(w.sumtmp), s))) return rc;
     k_pm_total<<<1, 32, 0, s>>>(d_total, (double)n);
     TC_CUDA_TRY(cudaGetLastError());
-    if (host) {
-        TC_CUDA_TRY(cudaMemcpyAsync(h_grad, d_grad, n * 16, cudaMemcpyDeviceToHost, s));
-        TC_CUDA_TRY(cudaMemcpyAsync(h_total, d_total, 8, cudaMemcpyDeviceToHost, s));
-        TC_CUDA_TRY(cudaStreamSynchronize(s));
-    }
     return TC_OK;
-}
-
-int pm_solve_device(int n_interp, double cell_size, int min_intervals, const double* d_pos, int64_t n, double* d_grad,
-                    double* d_total, cudaStream_t s)
-{
-    return pm_solve(n_interp, cell_size, min_intervals, d_pos, n, d_grad, d_total, s, false);
 }
 
 }  // namespace tc
@@ -651,5 +635,17 @@ extern "C" int tc_pm_solve(int n_interp, double cell_size, int min_intervals, co
         tc_set_error("tc_pm_solve: invalid arguments");
         return TC_ERR_INVALID;
     }
-    return pm_solve(n_interp, cell_size, min_intervals, pos_xy, n, grad_xy, total, nullptr, true);
+    int rc = pm_check(n_interp, cell_size, min_intervals, pos_xy, n, grad_xy, total);
+    if (rc) return rc;
+    HostStage st;
+    if ((rc = st.open((size_t)n * 16, (size_t)n * 16 + 64))) return rc;
+    double *d_total = static_cast<double*>(st.out()), *d_grad = d_total + 8;
+    TC_CUDA_TRY(cudaMemcpyAsync(st.in(), pos_xy, (size_t)n * 16, cudaMemcpyHostToDevice, st.stream()));
+    rc = pm_solve_device(n_interp, cell_size, min_intervals, static_cast<const double*>(st.in()), n, d_grad, d_total,
+                         st.stream());
+    if (rc) return rc;
+    TC_CUDA_TRY(cudaMemcpyAsync(grad_xy, d_grad, (size_t)n * 16, cudaMemcpyDeviceToHost, st.stream()));
+    TC_CUDA_TRY(cudaMemcpyAsync(total, d_total, 8, cudaMemcpyDeviceToHost, st.stream()));
+    TC_CUDA_TRY(cudaStreamSynchronize(st.stream()));
+    return TC_OK;
 }

@@ -173,6 +173,32 @@ int record_on(Handle& h, int i, cudaStream_t s);
 // the order-p near and far fields' streams and fork/join events (created on first use, never inside a capture)
 int ensure_near_stream(Handle& h);
 
+// Device copies of a host call's arrays and the stream it runs on, for entries
+// without a handle.  Up to four idle ones a device are kept for later calls,
+// without their buffers where these hold more than 64 MB; each open call has
+// its own, so the copies of one overlap another's work.  Closing waits for the
+// stream: nothing of the caller's memory is in flight afterwards.
+class HostStage {
+public:
+    HostStage() = default;
+    HostStage(const HostStage&) = delete;
+    HostStage& operator=(const HostStage&) = delete;
+    ~HostStage();
+    int open(size_t in_bytes, size_t out_bytes);
+    cudaStream_t stream() const { return slot_.stream; }
+    void* in() const { return slot_.in.p; }
+    void* out() const { return slot_.out.p; }
+
+    struct Slot {
+        cudaStream_t stream = nullptr;
+        Buf in, out;
+    };
+
+private:
+    Slot slot_;
+    int dev_ = -1;
+};
+
 template <typename T>
 inline T* P(const Buf& b) { return reinterpret_cast<T*>(b.p); }
 
