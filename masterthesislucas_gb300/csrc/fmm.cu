@@ -25,6 +25,8 @@
 // above.  Geometry is in cell-relative coordinates: offsets between cells are
 // integer multiples of the cell size, so FP32 differences lose nothing to the
 // absolute position magnitude.
+#include <cmath>
+
 #include "kernels.cuh"
 #include "state.cuh"
 
@@ -91,6 +93,7 @@ struct Geo {
     double inv_theta;
     double theta;
     double h_leaf;     // leaf cell size
+    double far;        // largest coordinate of the box: cell centres are rounded by 2^-53 of it
     int variant;       // 1: the non-symmetric FMM_MORTON leaf stage
 };
 
@@ -177,14 +180,19 @@ __device__ inline bool pn_pass(double2 x, double2 com, double len, double inv_th
 // L_B / theta, the same for every non-empty leaf), decided in FP64 by exact()
 // only where the FP32 squared distance is too close to the threshold: at the
 // threshold R is off by at most a few 2^-24 (thr + 3 h), which moves |R|^2 by
-// less than an eighth of the band.  FP64 runs at 1/64 of the FP32 rate, and
+// less than an eighth of the band (and by the rounding of the cells' centres,
+// the band's second part).  FP64 runs at 1/64 of the FP32 rate, and
 // the test is made for every particle and partner leaf.  (Squares below 1e-30
 // are left to FP64: near the end of the normal range the band says nothing.)
 template <typename real>
 struct PointMac {
     real thr2, band;
-    __device__ PointMac(real thr, real h)
-        : thr2(thr * thr), band(thr2 > real(1e-30) ? real(3.2e-6) * thr * (thr + real(3) * h) : real(INFINITY)) {}
+    __device__ PointMac(real thr, real h, real far)
+        : thr2(thr * thr),
+          band(thr2 > real(1e-30) ? real(3.2e-6) * thr * (thr + real(3) * h) + real(0x1p-49) * thr * far
+                                  : real(INFINITY))
+    {
+    }
     template <typename F>
     __device__ __forceinline__ bool pass(real Rx, real Ry, F&& exact) const
     {
@@ -256,7 +264,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
     const uint32_t li = level_index(dep);
     const int64_t nl = (int64_t)1 << (2 * dep);
     const real h = (real)geo.h_leaf;
-    const PointMac<real> mac((real)(geo.h_leaf * geo.inv_theta), h);
+    const PointMac<real> mac((real)(geo.h_leaf * geo.inv_theta), h, (real)geo.far);
     const double inv_theta = geo.inv_theta;
     // leaf si by nv warps, this one taking runs v, v + nv, ... of its partners' points; C and z are the warp's sums
     auto leaf = [&](int64_t si, int v, int nv, real (&C)[L_NCOEF], double& z) {
@@ -455,7 +463,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps)
     const uint32_t li = level_index(dep);
     const int64_t nl = (int64_t)1 << (2 * dep);
     const real h = (real)geo.h_leaf;
-    const PointMac<real> mac((real)(geo.h_leaf * geo.inv_theta), h);
+    const PointMac<real> mac((real)(geo.h_leaf * geo.inv_theta), h, (real)geo.far);
     const double inv_theta = geo.inv_theta;
     const uint32_t nwork = chunk_ptr[nl];
     for (uint32_t wi = blockIdx.x; wi < nwork; wi += gridDim.x) {
@@ -716,6 +724,8 @@ int solve_t(Handle& h, K ker, double* d_grad, int accumulate, int scatter, doubl
     geo.inv_theta = 1.0 / h.cfg.theta;
     geo.theta = h.cfg.theta;
     geo.h_leaf = h.L / (double)(1u << dep);
+    geo.far = std::fmax(std::fmax(std::fabs(h.minx), std::fabs(h.minx + h.L)),
+                        std::fmax(std::fabs(h.miny), std::fabs(h.miny + h.L)));
     geo.variant = h.variant;
     // work items of the near field: 32-sink chunks of the non-empty leaves
     const int64_t wmax = h.n / 32 + (h.n < nleaf ? h.n : nleaf) + 1;

@@ -116,3 +116,20 @@ def test_point_criteria_at_any_scale(symmetric, theta, scale):
         s.solveNbody(0.0, pts)
         counts.append(s.counters())
     assert counts[0] == counts[1]
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+@pytest.mark.parametrize("offset", [0.0, 2.0 ** 30 / 3, 2.0 ** 38 / 3, 2.0 ** 46 / 3])
+def test_point_criteria_far_from_the_origin(symmetric, offset):
+    """The points' criteria decide as in FP64 where the cells' centres are rounded by much of a cell."""
+    pos, mn, mx = cells(REF_SIZES, 2)
+    pos, mn, mx = pos + offset, mn + offset, mx + offset
+    cls = NBodySolverFMM_SYM_MORTON if symmetric else NBodySolverFMM_MORTON
+    counts = []
+    for p in ("fp64", "fp32"):
+        s = cls("tsne", tree_depth=2, theta=0.4, precision=p)
+        pts = Points.from_positions(pos)
+        s.updateTree(pts, mn - 0.0137, mx + 0.0171)
+        s.solveNbody(0.0, pts)
+        counts.append(s.counters())
+    assert counts[0] == counts[1]
