@@ -13,12 +13,12 @@
 //   13 log10 of A's order-4 norm   14 log2(c/h^2) (kernel scale)   15 level/16
 // (spread = sqrt(2 (mu20 + mu02) / M0), the RMS particle distance.)
 #include <cmath>
+#include <new>
+#include <vector>
 
 #include "controller.cuh"
 #include "expansion.cuh"
 #include "kernels.cuh"
-#include <vector>
-
 #include "state.cuh"
 
 namespace tc {
@@ -177,21 +177,38 @@ extern "C" int tc_get_list(tc_handle* t, int level, int kind, uint32_t* ptr, uin
         return TC_OK;
     }
     // a level's lists may lie in any order, and the words of empty nodes are not set: CSR in node order from the
-    // starts, ends and particle counts
+    // starts, ends and particle counts.  After replays of a captured step the pointers are the last replay's and the
+    // total still the capture's: no more entries than that are written
     const uint32_t* dptr = P<uint32_t>(h.ptr_pool) + (kind ? L.near_ptr_off[level] : L.nn_ptr_off[level]);
     const uint32_t* didx = P<uint32_t>(h.idx_pool) + (kind ? L.near_idx_off[level] : L.nn_idx_off[level]);
-    std::vector<uint32_t> se(list_ptr_words(nl)), cnt(nl), raw(idx ? tot : 0);
-    TC_CUDA_TRY(cudaMemcpyAsync(se.data(), dptr, se.size() * 4, cudaMemcpyDeviceToHost, h.stream));
-    TC_CUDA_TRY(cudaMemcpyAsync(cnt.data(), P<uint32_t>(h.count) + level_index(level), nl * 4, cudaMemcpyDeviceToHost,
-                                h.stream));
-    if (!raw.empty()) TC_CUDA_TRY(cudaMemcpyAsync(raw.data(), didx, tot * 4, cudaMemcpyDeviceToHost, h.stream));
-    TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    std::vector<uint32_t> se, cnt, raw;
+    try {
+        se.resize(list_ptr_words(nl));
+        cnt.resize(nl);
+        TC_CUDA_TRY(cudaMemcpyAsync(se.data(), dptr, se.size() * 4, cudaMemcpyDeviceToHost, h.stream));
+        TC_CUDA_TRY(cudaMemcpyAsync(cnt.data(), P<uint32_t>(h.count) + level_index(level), nl * 4,
+                                    cudaMemcpyDeviceToHost, h.stream));
+        TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+        uint32_t end = 0;
+        for (int64_t a = 0; a < nl; a++)
+            if (cnt[a] && se[list_end(nl, a)] > end) end = se[list_end(nl, a)];
+        raw.resize(idx ? end : 0);
+    } catch (const std::bad_alloc&) {
+        cudaStreamSynchronize(h.stream);
+        tc_set_error("tc_get_list: no host memory for the level's lists");
+        return TC_ERR_NOMEM;
+    }
+    if (!raw.empty()) {
+        TC_CUDA_TRY(cudaMemcpyAsync(raw.data(), didx, raw.size() * 4, cudaMemcpyDeviceToHost, h.stream));
+        TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+    }
     int64_t at = 0;
     for (int64_t a = 0; a < nl; a++) {
         if (ptr) ptr[a] = (uint32_t)at;
-        const int64_t b0 = se[a], b1 = cnt[a] ? se[list_end(nl, a)] : b0;
-        for (int64_t e = b0; idx && e < b1 && e < tot; e++) idx[at + (e - b0)] = raw[e];
-        at += b1 - b0;
+        if (!cnt[a]) continue;
+        const uint32_t b1 = se[list_end(nl, a)];
+        for (uint32_t e = se[a]; e < b1; e++, at++)
+            if (idx && at < tot) idx[at] = raw[e];
     }
     if (ptr) ptr[nl] = (uint32_t)at;
     return TC_OK;

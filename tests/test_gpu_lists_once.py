@@ -57,3 +57,39 @@ def test_kept_outcomes_of_several_batches(depth):
         s.updateTree(Points.from_positions(pos), mn, mx)
         for a, b in zip(counted, lists(s, depth)):
             np.testing.assert_array_equal(a, b)
+
+
+def test_lists_after_replays_of_a_captured_step():
+    """The pointers of the last replay; entries only as far as the captured step's total, which the caller has room for."""
+    import torch
+    rng = np.random.default_rng(4)
+    pos = rng.random((20000, 2))
+    box, depth = np.array([0.0, 0.0, 1.0, 1.0]), 5
+    pd = torch.from_numpy(pos).cuda()
+    g, t = torch.zeros_like(pd), torch.zeros(1, dtype=torch.float64, device="cuda")
+    s, fresh = (NBodySolverFMM_SYM_MORTON("tsne", tree_depth=depth, theta=0.8, order=4, mac="bmax") for _ in range(2))
+    s.update_tree_device(pd, box[:2], box[2:])
+    s.capture_step(pd, g, t, box=box)
+    more = 0
+    for f in (0.99, 0.97, 0.95, 0.93):
+        pd.copy_(torch.from_numpy(pos * f))
+        s.launch_step()
+        torch.cuda.synchronize()
+        assert s.async_status() == 0
+        fresh.update_tree_device(pd, box[:2], box[2:])
+        for level in range(depth + 1):
+            for kind in (0, 1):
+                words, tots = [], []
+                for h in (s, fresh):
+                    p, tot = np.zeros((1 << (2 * level)) + 1, np.uint32), ctypes.c_int64(0)
+                    check(lib().tc_get_list(h._h, level, kind, ptr(p), None, ctypes.byref(tot)))
+                    idx = np.full(2 * tot.value + 100000, 0xFFFFFFFF, np.uint32)
+                    check(lib().tc_get_list(h._h, level, kind, ptr(p), ptr(idx), ctypes.byref(tot)))
+                    assert np.all(idx[tot.value:] == 0xFFFFFFFF)
+                    words.append((p, idx))
+                    tots.append(tot.value)
+                np.testing.assert_array_equal(words[0][0], words[1][0])
+                m = min(tots)
+                np.testing.assert_array_equal(words[0][1][:m], words[1][1][:m])
+                more += words[1][0][-1] > tots[0]
+    assert more > 0  # some lists had outgrown the captured total
