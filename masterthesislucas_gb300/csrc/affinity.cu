@@ -34,7 +34,7 @@ namespace {
 #define TC_KNN_GRAM_MIN_N 1024
 #endif
 constexpr int64_t kGramMinN = TC_KNN_GRAM_MIN_N;
-constexpr int kGramMinDim = 1, kGramMaxDim = 4096;
+constexpr int kGramMaxDim = 4096;
 constexpr int64_t kGramBytes = 256ll << 20;
 
 // ------------------------------------------------------------------ exp, log
@@ -656,7 +656,7 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
     // faster one over all of that range, k = 90, against k_knn alone: 1,024 x 4: 91 us, 295; 2,000 x 32: 111, 573;
     // 20,000 x 128: 1.28 ms, 6.70; 20,000 x 784: 3.0, 23.2 (4.6 when the inputs have low parts); 70,000 x 784: 22.2,
     // 254.9
-    bool gram = n >= kGramMinN && dim >= kGramMinDim && dim <= kGramMaxDim;
+    bool gram = n >= kGramMinN && dim <= kGramMaxDim;
     auto kernel = vec ? k_knn<true> : k_knn<false>;
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
     // scratch: partial lists; for the filter the split inputs, norms, status, flags and list of query blocks, and

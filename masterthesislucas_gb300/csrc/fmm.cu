@@ -242,9 +242,12 @@ struct NearBatch {
 // and the number of 32-sink chunks of S.  A block takes kLeafWarps leaves, a
 // warp each; a leaf of more than kLeafLocalBlock particles, which lies in a
 // dense region, takes a block of its own: a warp alone was a
-// serial chain of up to 10^5 points there (200,003 particles of two disks:
-// 947 us, 172 us now).  The points of 32 partners are one flat range
+// serial chain of up to 10^5 points there (one draw of 200,003 particles of
+// two disks: 947 us, 174 us now).  The points of 32 partners are one flat range
 // dealt 32 at a time, so that partners of a few points fill the lanes too.
+// Where the line lies, at 32, 64 and 256: 200,000 uniform particles, leaves of
+// 64: 38, 29 and 28 us; 100,000 of twenty clusters: 91, 97 and 115; the disks
+// with leaves of 256, whose outer leaves hold 32 to 64: 307, 642 and 905.
 constexpr uint32_t kLeafLocalBlock = 64;
 
 template <typename real, typename K>
@@ -442,8 +445,8 @@ __device__ __forceinline__ void leaf_eval(const K& ker, const double* buf, uint3
 // sources), and stage the points that interact directly, shifted into S's
 // frame, until kLeafBuf of them can be evaluated at once; runs that only some
 // of the sinks see are evaluated by themselves.  The warps' sums are added in
-// warp order.  200,003 particles of two disks, 4,096 leaves, theta 0.5: 2,805 us
-// with a warp per item and one source at a time, 1,547 us now.
+// warp order.  The same draw of 200,003 particles of two disks, theta 0.5:
+// 2,805 us with a warp per item and one source at a time, 1,546 us now.
 template <typename real, typename K>
 __global__ void __launch_bounds__(32 * kLeafWarps)
     k_leaf_near(K ker, Geo geo, const uint32_t* __restrict__ count, const uint32_t* __restrict__ first,

@@ -826,10 +826,14 @@ constexpr uint32_t kBlockSinks = 32u * kNearWarps;
 // near list is tens of thousands of particles long: items of 128 sinks are
 // then fewer than the resident blocks and up to three times their mean, and
 // the last of them run alone on their SMs.  Its items hold 32 sinks and the
-// block's warps split the sources instead (near_split_item).  200,001
-// particles of two disks in 4,096 leaves (largest 6,600, 3.2e9 pairs):
-// 1,630 us with items of 128 sinks, 1,273 us now.  Leaves below the line
-// keep the wider items, which stage every source once for 128 sinks.
+// block's warps split the sources instead (near_split_item).  One draw of
+// 200,001 particles of two disks in 4,096 leaves (largest 6,600, 3.2e9 pairs;
+// the largest leaf follows the draw's outermost particles): 1,630 us with items
+// of 128 sinks, 1,273 us now.  Leaves below the line keep the wider items,
+// which stage every source once for 128 sinks.  The line at 256, 512 and 2,048:
+// 200,003 particles of two disks 1.99, 1.98 and 2.36 ms; 1M 4.27, 4.28 and 4.50;
+// 100,000 of twenty clusters 0.33, 0.32 and 0.33, of six tight ones 0.74, 0.76
+// and 0.82.
 constexpr uint32_t kSplitLeaf = 512u;
 __device__ __forceinline__ uint32_t block_item_sinks(uint32_t c) { return c > kSplitLeaf ? 32u : kBlockSinks; }
 

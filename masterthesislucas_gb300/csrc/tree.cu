@@ -223,9 +223,9 @@ __device__ inline void write_compute(int64_t node, double comx, double comy, dou
 // (then of xx, xy, yy) over the staged terms, so that a particle costs one
 // FP64 warp instruction per loop and not eight (FP64 issues at 1/64 of the
 // FP32 rate, as much for one lane as for 32).  The next chunk is loaded while
-// the chains run.  What is left is the chain of the largest leaf: 200,003
-// particles of two disks in 4,096 leaves (largest 6,400): 2,386 us with a
-// thread per leaf, 730 us now.
+// the chains run.  What is left is the chain of the largest leaf: one draw of
+// 200,003 particles of two disks in 4,096 leaves (largest 6,400; it follows the
+// draw's outermost particles): 2,386 us with a thread per leaf, 736 us now.
 constexpr int kMomLanes = 8;
 constexpr int kMomChunk = 32;
 constexpr int kMomThreads = 128;
@@ -569,8 +569,9 @@ int build_tree(Handle& h, const double* d_pos, int64_t n, double minx, double mi
     const int w = 1 << depth;
     if (!f64 && (rc = ensure(h.celloff, (size_t)w * 8))) return rc;
     if (physics && (rc = ensure(h.bigleaf, (size_t)bigleaf_words(n) * 4))) return rc;
-    // (a tree of many more leaves than points is cleared faster by itself than by the points' few blocks)
-    const bool sparse = nleaf > 16 * n;
+    // a tree of many more leaves than points is cleared faster by itself than by the points' few blocks: 2,000 points,
+    // a whole update by the blocks and by clears: 33 leaves a point 202 and 209 us, 131: 257 and 258, 524: 332 and 318
+    const bool sparse = nleaf > 128 * n;
     if (sparse) {
         TC_CUDA_TRY(cudaMemsetAsync(P<uint32_t>(h.count) + li, 0, nleaf * 4, s));
         TC_CUDA_TRY(cudaMemsetAsync(P<uint32_t>(h.first) + li, 0, nleaf * 4, s));
