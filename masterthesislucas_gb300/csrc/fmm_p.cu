@@ -834,12 +834,12 @@ constexpr uint32_t kBlockSinks = 32u * kNearWarps;
 // 200,003 particles of two disks 1.99, 1.98 and 2.36 ms; 1M 4.27, 4.28 and 4.50;
 // 100,000 of twenty clusters 0.33, 0.32 and 0.33, of six tight ones 0.74, 0.76
 // and 0.82.
-constexpr uint32_t kSplitLeaf = 512u;
-__device__ __forceinline__ uint32_t block_item_sinks(uint32_t c) { return c > kSplitLeaf ? 32u : kBlockSinks; }
+// (kSplitLeaf is in state.cuh: a handle whose GPU is full of other systems' items has no such line.)
+__device__ __forceinline__ uint32_t block_item_sinks(uint32_t c, uint32_t split) { return c > split ? 32u : kBlockSinks; }
 
 // per leaf: warp items (a leaf of 1..32 particles) and block items (a larger
 // leaf, one per block_item_sinks of its particles)
-__global__ void k_chunks(int dep, const uint32_t* __restrict__ count, uint32_t* __restrict__ nwarp,
+__global__ void k_chunks(int dep, const uint32_t* __restrict__ count, uint32_t split, uint32_t* __restrict__ nwarp,
                          uint32_t* __restrict__ nblock)
 {
     const uint32_t li = level_index(dep);
@@ -847,7 +847,7 @@ __global__ void k_chunks(int dep, const uint32_t* __restrict__ count, uint32_t* 
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < nl; i += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t c = count[li + i];
         nwarp[i] = c >= 1u && c <= 32u ? 1u : 0u;
-        nblock[i] = c > 32u ? (c + block_item_sinks(c) - 1u) / block_item_sinks(c) : 0u;
+        nblock[i] = c > 32u ? (c + block_item_sinks(c, split) - 1u) / block_item_sinks(c, split) : 0u;
     }
 }
 
@@ -1180,7 +1180,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, TC_NEAR_MIN_WARPS / kNearWarp
     k_near_p(KN ker, int dep, float h, const uint32_t* __restrict__ count, const uint32_t* __restrict__ first,
              const uint32_t* __restrict__ near_ptr, const uint32_t* __restrict__ near_idx,
              const uint32_t* __restrict__ wptr, const uint32_t* __restrict__ witem,
-             const uint32_t* __restrict__ bptr, const uint32_t* __restrict__ bitem, uint32_t cap,
+             const uint32_t* __restrict__ bptr, const uint32_t* __restrict__ bitem, uint32_t cap, uint32_t split,
              const float* __restrict__ prel, uint32_t n, float2* __restrict__ nearf, double* __restrict__ zwork,
              unsigned long long* __restrict__ counters)
 {
@@ -1197,7 +1197,7 @@ __global__ void __launch_bounds__(32 * kNearWarps, TC_NEAR_MIN_WARPS / kNearWarp
     for (uint32_t bi = blockIdx.x; bi < nb; bi += gridDim.x) {
         const int64_t si = bitem[bi];
         const uint32_t cS = count[li + si];
-        if (cS > kSplitLeaf) {
+        if (cS > split) {
             const uint32_t c0 = (bi - bptr[si]) * 32u;
             uint32_t pairs = 0;
             const float z = near_split_item(ker, dep, h, count, first, near_ptr, near_idx, prel2, n, nearf, si, c0,
@@ -1446,7 +1446,7 @@ int solve_p(Handle& h, KN ker, const PotParams& pp, double* d_grad, int accumula
         k_near_p<KN><<<(unsigned)(wblk < sm_count() * 256 ? wblk : sm_count() * 256), 32 * kNearWarps, 0, sn>>>(
             ker, dep, (float)(h.L / (double)(1u << dep)), count_n, P<uint32_t>(h.first),
             ptr_n + h.lists.near_ptr_off[dep], idx_n + h.lists.near_idx_off[dep], wptr, witem, bptr, bitem,
-            (uint32_t)wmax, P<float>(h.prel), (uint32_t)h.n, P<float2>(h.nearf), P<double>(h.zwork),
+            (uint32_t)wmax, h.items_split, P<float>(h.prel), (uint32_t)h.n, P<float2>(h.nearf), P<double>(h.zwork),
             P<unsigned long long>(h.counters));
     }
     if ((rc = record_on(h, 9, sn))) return rc;
@@ -1778,7 +1778,8 @@ int near_items(Handle& h)
     uint32_t* bptr = wptr + (nleaf + 1);
     uint32_t* nz = bptr + (nleaf + 1);
     uint32_t* witem = P<uint32_t>(h.chunk_leaf);
-    k_chunks<<<grid_for(nleaf, 256), 256, 0, s>>>(dep, P<uint32_t>(h.count), nwarp, nblock);
+    h.items_split = h.split_leaf;
+    k_chunks<<<grid_for(nleaf, 256), 256, 0, s>>>(dep, P<uint32_t>(h.count), h.items_split, nwarp, nblock);
     if ((rc = exclusive_scan2_u32(nwarp, wptr, nblock, bptr, nleaf, P<uint32_t>(h.items_tmp), s))) return rc;
     k_chunk_leaf<<<grid_for(nleaf, 256), 256, 0, s>>>(dep, wptr, bptr, witem, witem + wmax, (uint32_t)wmax, nz);
     h.launches += 2 + (nleaf <= 2048 ? 1 : 3);

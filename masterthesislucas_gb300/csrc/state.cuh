@@ -60,6 +60,9 @@ struct LevelLists {
 // level of node i of the level-dense numbering (level_index(l) = (4^l - 1) / 3 nodes come before level l)
 __device__ inline int level_of(uint32_t i) { return (63 - __clzll((long long)(3ull * i + 1ull))) >> 1; }
 
+// near field: the line above which a leaf's items hold 32 sinks and split the sources (k_near_p)
+constexpr uint32_t kSplitLeaf = 512u;
+
 struct Handle {
     tc_config cfg;
     cudaStream_t stream = nullptr;
@@ -78,6 +81,8 @@ struct Handle {
 #define TC_NEAR_OVERLAP_DEFAULT 1
 #endif
     bool near_overlap = TC_NEAR_OVERLAP_DEFAULT;
+    // near field: leaves above this many particles are split into items of 32 sinks; the line the item tables were built by
+    uint32_t split_leaf = kSplitLeaf, items_split = kSplitLeaf;
     cudaStream_t near_stream = nullptr, far_stream = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_far = nullptr;
     // the update's multipoles on near_stream beside the list build (ev_mu marks them done); build_tree

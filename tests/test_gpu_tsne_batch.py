@@ -71,3 +71,28 @@ def test_batch_rejects_systems_out_of_step():
     s[0].time_step()  # out of step with s[1]
     with pytest.raises(TreecodeError):
         TSNEBatch(s)
+
+
+@pytest.mark.parametrize("sizes", [[2049, 2600], [513, 5000, 40]])
+def test_dense_leaves_in_a_batch(sizes):
+    """Leaves of more than 512 points, whose near-field items a batch does not split, against single systems, which do."""
+    rng = np.random.default_rng(8)
+    data = []
+    for n in sizes:
+        rp = (4 * np.arange(n + 1)).astype(np.uint32)
+        data.append((rp, rng.integers(0, n, 4 * n).astype(np.uint32), np.full(4 * n, 0.25 / n), rng.normal(0, 3, (n, 2))))
+
+    def systems():  # four leaves, all pairs direct whatever the box
+        return [TSNE(rp, col, val, y0, max_children=16, order=8, depth=1, min_theta=0.1, max_theta=0.1)
+                for rp, col, val, y0 in data]
+
+    a, b = systems(), systems()
+    batch = TSNEBatch(a, margin=0.5)
+    for _ in range(3):  # the first uncaptured, then replays
+        batch.time_step()
+        for sa, sb in zip(a, b):
+            sb.time_step()
+            ga, gb = sa.embedding()[2], sb.embedding()[2]
+            # FP32 sums of up to 5,000 terms on either side, runs of 2,048 with 64 lanes' partial sums a run
+            assert np.abs(ga - gb).max() <= 2e-5 * np.abs(gb).max()
+    batch.close()
