@@ -23,6 +23,8 @@
 //   (j, i); the (at most two) contributions to an entry are added.
 // This file is compiled without FMA contraction: the fused operations above
 // are the explicit fma / fmaf calls.
+#include <mutex>
+
 #include "common.cuh"
 #include "knn_gram.cuh"
 
@@ -215,7 +217,8 @@ __device__ __forceinline__ void knn_insert(u64* __restrict__ list, int k, u64 ke
 template <bool kVec>
 __global__ void __launch_bounds__(kKnnT, 2)
     k_knn(const float* __restrict__ x, int64_t n, int dim, int k, int64_t ctiles, int64_t qblocks,
-          const uint32_t* __restrict__ list, const uint32_t* __restrict__ nlist, u64* __restrict__ part)
+          const uint32_t* __restrict__ list, const uint32_t* __restrict__ nlist, u64* __restrict__ part,
+          float* __restrict__ out_d, int32_t* __restrict__ out_i)
 {
     extern __shared__ __align__(16) uint8_t dyn[];
     float* stage = reinterpret_cast<float*>(dyn);          // [2][kKC][kQ + kC]
@@ -329,9 +332,16 @@ __global__ void __launch_bounds__(kKnnT, 2)
         }
         __syncthreads();
         if (u + 1 == u1 || (u + 1) % ctiles == 0) {
-            // runs and query blocks both grow along the units: their sum numbers the partial lists
-            u64* dst = part + (run + o) * (int64_t)(kQ * k);
-            for (int e = tid; e < kQ * k; e += kKnnT) dst[e] = lists[e];
+            if (out_d) {  // a single candidate tile: the lists are whole
+                for (int e = tid; e < kQ * k && q0 + e / k < n; e += kKnnT) {
+                    out_d[q0 * k + e] = __uint_as_float((uint32_t)(lists[e] >> 32));
+                    out_i[q0 * k + e] = (int32_t)(uint32_t)lists[e];
+                }
+            } else {
+                // runs and query blocks both grow along the units: their sum numbers the partial lists
+                u64* dst = part + (run + o) * (int64_t)(kQ * k);
+                for (int e = tid; e < kQ * k; e += kKnnT) dst[e] = lists[e];
+            }
             __syncthreads();
         }
     }
@@ -638,6 +648,42 @@ __global__ void k_sym_write(const uint32_t* __restrict__ ord, const uint32_t* __
 
 using namespace tc;
 
+// The kNN's scratch comes from a memory pool of its own, which keeps up to 64 MB between calls: the device's default
+// pool gives everything back at each synchronisation, and allocating anew took more than a small call's kernels (1,024 x 2,
+// k = 1: 266 us a call, 60 with the pool; 150 before the kNN had scratch).  nullptr: the default pool.
+constexpr size_t kKnnPoolKeep = 64ull << 20;
+static cudaMemPool_t knn_pool()
+{
+    static std::mutex mu;
+    static cudaMemPool_t pools[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+    std::lock_guard<std::mutex> g(mu);
+    if (!pools[dev]) {
+        cudaMemPoolProps p = {};
+        p.allocType = cudaMemAllocationTypePinned;
+        p.location.type = cudaMemLocationTypeDevice;
+        p.location.id = dev;
+        uint64_t keep = kKnnPoolKeep;
+        // (no stream's work: allowed while this or another thread captures)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaMemPoolCreate(&pools[dev], &p) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pools[dev], cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            pools[dev] = nullptr;
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
+    return pools[dev];
+}
+
+static cudaError_t knn_alloc(void** p, size_t bytes, cudaStream_t s)
+{
+    const cudaMemPool_t pool = knn_pool();
+    return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
+}
+
 extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float* d_dist, int32_t* d_idx, void* stream)
 {
     if (!d_x || !d_dist || !d_idx || n < 2 || dim < 1 || k < 1 || k > kMaxK || k >= n || n > 0x7FFFFFFF) {
@@ -667,15 +713,20 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
     rb_chunk = rb_chunk < 1 ? 1 : rb_chunk > rblocks ? rblocks : rb_chunk;
     const size_t b_part = up((size_t)(runs + qblocks) * kQ * k * 8), b_half = up((size_t)npad * dimp * 2),
                  b_norm = up((size_t)npad * 4), b_flag = up(sizeof(GramStat) + (size_t)qblocks * 4),
-                 b_list = up((size_t)qblocks * 4), b_gram = up((size_t)rb_chunk * kGramRows * npad * 4),
-                 b_gmin = b_gram / 4;
+                 b_list = up((size_t)qblocks * 4);
+    const size_t b_fixed = b_part + 2 * b_half + b_norm + b_flag + b_list, rb_bytes = (size_t)kGramRows * npad * 5;
+    // up to 12,288 points, where allocating the scratch anew costs more than shorter launches do, no more than the pool
+    // keeps, as long as a launch has two tiles for nearly every multiprocessor (10,000 x 2, k = 1: 890 us -> 303)
+    const int64_t rb_pool = b_fixed + 512 < kKnnPoolKeep ? (int64_t)((kKnnPoolKeep - b_fixed - 512) / rb_bytes) : 0;
+    if (n <= 12288 && rb_pool < rb_chunk && rb_pool * (npad / kGramCols) >= 2 * sm_count() - 64) rb_chunk = rb_pool;
+    const size_t b_gram = up((size_t)rb_chunk * kGramRows * npad * 4), b_gmin = b_gram / 4;
     void* buf_p = nullptr;
-    if (gram && cudaMallocAsync(&buf_p, b_part + 2 * b_half + b_norm + b_flag + b_list + b_gram + b_gmin, s) !=
-                    cudaSuccess) {
+    if (gram && knn_alloc(&buf_p, b_fixed + b_gram + b_gmin, s) != cudaSuccess) {
         cudaGetLastError();  // no room for the filter's scratch: every query block by k_knn
         gram = false;
     }
-    if (!gram) TC_CUDA_TRY(cudaMallocAsync(&buf_p, b_part, s));
+    const bool whole = ctiles == 1;  // no partial lists, no scratch
+    if (!gram && !whole) TC_CUDA_TRY(knn_alloc(&buf_p, b_part, s));
     uint8_t* buf = static_cast<uint8_t*>(buf_p);
     // runs that share a query block: each holds at least units / runs of its ctiles units
     int64_t maxseg = gram ? kListRuns + 2 : runs / qblocks + 2;
@@ -683,14 +734,14 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
     const size_t dyn = kKnnStatic + (size_t)kQ * k * 8, mdyn = (size_t)kMergeWarps * maxseg * k * 8;
     if (mdyn > kMergeMaxDyn) {  // up to 400 runs (200 multiprocessors) a row lies in at most 16
         tc_set_error("tc_knn_device: more runs a query block than the merge holds");
-        cudaFreeAsync(buf_p, s);
+        if (buf_p) cudaFreeAsync(buf_p, s);
         return TC_ERR_STATE;
     }
     u64* part = reinterpret_cast<u64*>(buf);
     uint32_t *list = nullptr, *nlist = nullptr;
     // the limits of every k, not this one's: calls of other threads set them too
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kKnnMaxDyn);
-    if (e == cudaSuccess)
+    if (e == cudaSuccess && !whole)
         e = cudaFuncSetAttribute(k_knn_merge, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMergeMaxDyn);
     if (gram && e == cudaSuccess) {
         uint8_t *hi = buf + b_part, *lo = hi + b_half;
@@ -720,12 +771,13 @@ extern "C" int tc_knn_device(const float* d_x, int64_t n, int dim, int k, float*
         }
     }
     if (e == cudaSuccess) {
-        kernel<<<(unsigned)runs, kKnnT, dyn, s>>>(d_x, n, dim, k, ctiles, qblocks, list, nlist, part);
-        k_knn_merge<<<(unsigned)(qblocks * (kQ / kMergeWarps)), 32 * kMergeWarps, mdyn, s>>>(
+        kernel<<<(unsigned)runs, kKnnT, dyn, s>>>(d_x, n, dim, k, ctiles, qblocks, list, nlist, part,
+                                                  whole ? d_dist : nullptr, d_idx);
+        if (!whole) k_knn_merge<<<(unsigned)(qblocks * (kQ / kMergeWarps)), 32 * kMergeWarps, mdyn, s>>>(
             part, n, k, ctiles, qblocks, runs, list, nlist, (int)maxseg, d_dist, d_idx);
         e = cudaGetLastError();
     }
-    const cudaError_t ef = cudaFreeAsync(buf, s);
+    const cudaError_t ef = buf ? cudaFreeAsync(buf, s) : cudaSuccess;
     if (e != cudaSuccess) return tc_cuda_fail(e, "tc_knn_device");
     TC_CUDA_TRY(ef);
     return TC_OK;

@@ -59,3 +59,63 @@ def test_threads_of_different_k():
     for t in threads:
         t.join()
     assert not errors, errors[0]
+
+
+@pytest.mark.parametrize("n", [127, 128, 129])
+@pytest.mark.parametrize("k", [1, 126])
+def test_one_candidate_tile(n, k):
+    """Up to 128 points the lists are whole and written at once; above, they are joined."""
+    import torch
+    x = np.random.default_rng(n).normal(size=(n, 7)).astype(np.float32)
+    d, i = affinity.knn(torch.from_numpy(x).cuda(), k)
+    rd, ri = oracle.knn(x, k)
+    np.testing.assert_array_equal(d.cpu().numpy(), rd)
+    np.testing.assert_array_equal(i.cpu().numpy(), ri)
+
+
+def test_scratch_kept_between_calls():
+    """Calls at the ends of the range whose launches are sized to what is kept, and a large one, which is given back."""
+    import torch
+    rng = np.random.default_rng(13)
+    free = []
+    for n in (1500, 9000, 12288, 12289, 20000, 1500):
+        x = torch.from_numpy(rng.random((n, 3)).astype(np.float32)).cuda()
+        d, i = affinity.knn(x, 5)
+        torch.cuda.synchronize()
+        dist = ((x[:200, None, :] - x[None, :, :]) ** 2).sum(-1)
+        dist[torch.arange(200), torch.arange(200)] = np.inf
+        ref = torch.topk(dist, 5, largest=False).values.sort(1).values
+        np.testing.assert_allclose(d[:200].cpu().numpy(), ref.cpu().numpy(), rtol=1e-5, atol=1e-12)
+        del x, d, i, dist, ref
+        torch.cuda.empty_cache()
+        free.append(torch.cuda.mem_get_info()[0])
+    assert max(free) - min(free) <= 96 << 20
+
+
+CAPTURED_FIRST_CALL = """
+import sys
+import torch
+from masterthesislucas_gb300 import affinity
+x = torch.rand(int(sys.argv[1]), 8, device="cuda")
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph, stream=torch.cuda.Stream()):
+    d, i = affinity.knn(x, 5, stream=torch.cuda.current_stream().cuda_stream)
+for _ in range(3):
+    x.copy_(torch.rand_like(x))
+    graph.replay()
+    torch.cuda.synchronize()
+    d2, i2 = affinity.knn(x, 5)
+    torch.cuda.synchronize()
+    assert torch.equal(d, d2) and torch.equal(i, i2)
+"""
+
+
+@pytest.mark.parametrize("n", [100, 900, 3000])
+def test_first_call_inside_a_capture(n):
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", CAPTURED_FIRST_CALL, str(n)], capture_output=True, text=True, cwd=root)
+    assert r.returncode == 0, r.stderr
