@@ -176,11 +176,17 @@ extern "C" int tc_get_list(tc_handle* t, int level, int kind, uint32_t* ptr, uin
         TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
         return TC_OK;
     }
-    // a level's lists may lie in any order, and the words of empty nodes are not set: CSR in node order from the
-    // starts, ends and particle counts.  After replays of a captured step the pointers are the last replay's and the
-    // total still the capture's: no more entries than that are written
     const uint32_t* dptr = P<uint32_t>(h.ptr_pool) + (kind ? L.near_ptr_off[level] : L.nn_ptr_off[level]);
     const uint32_t* didx = P<uint32_t>(h.idx_pool) + (kind ? L.near_idx_off[level] : L.nn_idx_off[level]);
+    if (nl > kListsOnceNodes) {  // lists placed by a scan: CSR as they stand
+        if (ptr) TC_CUDA_TRY(cudaMemcpyAsync(ptr, dptr, (nl + 1) * 4, cudaMemcpyDeviceToHost, h.stream));
+        if (idx && tot) TC_CUDA_TRY(cudaMemcpyAsync(idx, didx, tot * 4, cudaMemcpyDeviceToHost, h.stream));
+        TC_CUDA_TRY(cudaStreamSynchronize(h.stream));
+        return TC_OK;
+    }
+    // a coarser level's lists may lie in any order, and the words of empty nodes are not set: CSR in node order from the
+    // starts, ends and particle counts.  After replays of a captured step the pointers are the last replay's and the
+    // total still the capture's: no more entries than that are written
     std::vector<uint32_t> se, cnt, raw;
     try {
         se.resize(list_ptr_words(nl));
