@@ -24,7 +24,7 @@
 // after the subtree.  It visits the nodes a warp at a time, the warp's 32
 // points being neighbours in key order.  65,536 points of a Gaussian mixture,
 // leaves of 16, theta 0.5: 190 launches and 10 host round trips before,
-// 32 and one now; traversal 3,546 us with a thread per point in input order and
+// 16 and one now; traversal 3,546 us with a thread per point in input order and
 // the MAC in FP64, 234 us now.  Deeper trees take the level-synchronous
 // build and the per-point traversal, which know no depth limit.
 //

@@ -551,7 +551,7 @@ __global__ void __launch_bounds__(128, L2L ? (P >= 8 ? TC_M2L_FUSED_MIN_BLOCKS :
 // accumulators, then a fixed butterfly sum over the lanes.
 // The levels do not depend on one another, so levels l0 .. l1 share a launch:
 // one by one, seven levels of a 70,000-point tree took 109 us at order 8, most
-// of it the latency of each level's longest lists, and take 64 us us together.
+// of it the latency of each level's longest lists, and take 64 us together.
 template <int P>
 __global__ void __launch_bounds__(128) k_m2l_warp(int l0, int l1, float box, PotParams pp, LevelLists lists,
                                                   const float* __restrict__ comrel, const float* __restrict__ mu,
@@ -834,7 +834,7 @@ constexpr uint32_t kBlockSinks = 32u * kNearWarps;
 // 200,003 particles of two disks 1.99, 1.98 and 2.36 ms; 1M 4.27, 4.28 and 4.50;
 // 100,000 of twenty clusters 0.33, 0.32 and 0.33, of six tight ones 0.74, 0.76
 // and 0.82.
-// (kSplitLeaf is in state.cuh: a handle whose GPU is full of other systems' items has no such line.)
+// (kSplitLeaf is in state.cuh: the systems of a batch, whose items fill the GPU together, have no such line.)
 __device__ __forceinline__ uint32_t block_item_sinks(uint32_t c, uint32_t split) { return c > split ? 32u : kBlockSinks; }
 
 // per leaf: warp items (a leaf of 1..32 particles) and block items (a larger

@@ -78,7 +78,7 @@ __device__ __noinline__ float2 exact_terms(uint32_t bits, uint32_t e, uint32_t i
 // (high, low) pairs, and the FP64 ones where a pair's 48 bits are few: points
 // nearer than 2^-17 of their distance from the origin; the errors against 64
 // bits are those of FP64 differences to three digits.  70,000 rows of 180: 186 us
-// with FP64 differences throughout, 64 us now, and 3 for the split.
+// with FP64 differences throughout, 64 us now, and 4 for the split.
 constexpr int kAttrRows = 32;
 constexpr int kAttrThreads = 256;
 
