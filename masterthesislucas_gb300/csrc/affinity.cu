@@ -680,7 +680,8 @@ static cudaMemPool_t knn_pool()
 
 static cudaError_t knn_alloc(void** p, size_t bytes, cudaStream_t s)
 {
-    const cudaMemPool_t pool = knn_pool();
+    // more than the pool keeps: the default pool, whose memory the symmetrisation after it takes over
+    const cudaMemPool_t pool = bytes > kKnnPoolKeep ? nullptr : knn_pool();
     return pool ? cudaMallocFromPoolAsync(p, bytes, pool, s) : cudaMallocAsync(p, bytes, s);
 }
 
