@@ -37,7 +37,10 @@ def test_threads_of_different_sizes():
 
 
 def test_a_large_call_keeps_no_copies():
+    import gc
+
     import torch
+    gc.collect()  # handles of tests before this one give their memory back now, not meanwhile
     n = 3_000_000  # 48 MB in, 48 MB out
     pos = np.random.default_rng(0).random((n, 2))
     d = torch.from_numpy(pos).cuda()

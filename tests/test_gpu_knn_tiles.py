@@ -75,7 +75,10 @@ def test_one_candidate_tile(n, k):
 
 def test_scratch_kept_between_calls():
     """Calls at the ends of the range whose launches are sized to what is kept, and a large one, which is given back."""
+    import gc
+
     import torch
+    gc.collect()  # handles of tests before this one give their memory back now, not meanwhile
     rng = np.random.default_rng(13)
     free = []
     for n in (1500, 9000, 12288, 12289, 20000, 1500):
